@@ -404,19 +404,27 @@ struct HaloW {
   static constexpr int value = (LIM == LIM_MP5 || LIM == LIM_WENO5) ? 3 : 2;
 };
 
-// Shared-memory tile of BN x BN cells (sizes in doubles), halo width HW.
+// Shared-memory tile of BN x BN cells (sizes in elements), halo width HW.
+// Every variable holds its ring planes and its halo strips of plane k in one
+// block of VS elements, so the distance between two variables is the same
+// constant for every stencil cell, inside or halo: a face needs one address
+// per stencil cell (and one per rotated component), the rest are immediate
+// offsets of the loads.  The kernel is bound by instruction issue, and 610 of
+// a 3-D MHD face's 2570 instructions were address arithmetic when the halo
+// strips had strides of their own: 128^3 FP64 0.89 -> 0.83 ms per stage, mixed
+// 0.48 -> 0.43, 2-D HD 2048^2 0.45 -> 0.42 (same results bit for bit).
 template <class TF, int NW, int NDIM, int HW = 2, int BN = BN16>
 struct Tile {
   static constexpr int H2 = 2 * HW;
   static constexpr int NSLOT = NDIM == 3 ? H2 : 1;      // z ring: planes k-HW+1 .. k+HW
-  static constexpr int PLANE = BN * BN;
-  static constexpr int RING = NSLOT * NW * PLANE;        // [slot][v][j][i]
-  static constexpr int HX = NW * BN * H2;                // [v][j][c] c: i=-HW..-1, BN..BN+HW-1
-  static constexpr int HY = NW * H2 * BN;                // [v][r][i] r: j likewise
-  static constexpr int HC = NW * H2 * H2;                // [v][r][c] corners
-  static constexpr int FB = NW * (BN + 1) * BN;          // [v][face]
-  static constexpr int YX = NW * BN;                     // [v][i] y-faces of the top row (j = BN)
-  static constexpr int TOTAL = RING + HX + HY + HC + FB + YX;
+  static constexpr int PLANE = BN * BN;                  // [slot][j][i]
+  static constexpr int OX = NSLOT * PLANE;               // x halo [j][c] c: i=-HW..-1, BN..BN+HW-1
+  static constexpr int OY = OX + BN * H2;                // y halo [r][i] r: j likewise
+  static constexpr int OC = OY + H2 * BN;                // corners [r][c]
+  static constexpr int VS = OC + H2 * H2;                // one variable
+  static constexpr int FB = (BN + 1) * BN;               // scaled face fluxes of a variable
+  static constexpr int YX = BN;                          // y-faces of the top row (j = BN)
+  static constexpr int TOTAL = NW * (VS + FB + YX);
   static constexpr size_t BYTES = sizeof(TF) * TOTAL;
 };
 
@@ -432,40 +440,28 @@ __device__ __forceinline__ int ring_slot(int k) {
 
 template <class TF, int NW, int NDIM, int HW = 2, int BN = BN16>
 struct TileView {
+  using T = Tile<TF, NW, NDIM, HW, BN>;
   static constexpr int H2 = 2 * HW;
-  TF *ring, *hx, *hy, *hc, *fb, *yx;
+  TF *w, *fb, *yx;  // [v][VS], [v][face], [v][i]
   __device__ TileView(TF *s) {
-    using T = Tile<TF, NW, NDIM, HW, BN>;
-    ring = s;
-    hx = ring + T::RING;
-    hy = hx + T::HX;
-    hc = hy + T::HY;
-    fb = hc + T::HC;
-    yx = fb + T::FB;
+    w = s;
+    fb = w + NW * T::VS;
+    yx = fb + NW * T::FB;
   }
   // primitive v at in-plane (i, j) in [-HW, BN+HW-1]^2 of the plane held in `slot`
-  __device__ __forceinline__ TF at(int slot, int v, int i, int j) const {
-    const bool ii = (unsigned)i < (unsigned)BN, jj = (unsigned)j < (unsigned)BN;
-    if (ii && jj) return ring[(slot * NW + v) * (BN * BN) + j * BN + i];
-    if (jj) return hx[(v * BN + j) * H2 + halo_slot_w<HW, BN>(i)];
-    if (ii) return hy[(v * H2 + halo_slot_w<HW, BN>(j)) * BN + i];
-    return hc[(v * H2 + halo_slot_w<HW, BN>(j)) * H2 + halo_slot_w<HW, BN>(i)];
-  }
-  // Offset (in doubles from the tile start) of variable 0 at in-plane (i, j)
-  // of the plane in `slot`, and the stride between variables there; branch-free.
-  __device__ __forceinline__ void addr(int slot, int i, int j, int &base, int &stride) const {
-    using T = Tile<TF, NW, NDIM, HW, BN>;
+  __device__ __forceinline__ TF at(int slot, int v, int i, int j) const { return w[v * T::VS + off(slot, i, j)]; }
+  // element of variable 0 at in-plane (i, j) of the plane in `slot`; branch-free
+  __device__ __forceinline__ int off(int slot, int i, int j) const {
     const bool ii = (unsigned)i < (unsigned)BN, jj = (unsigned)j < (unsigned)BN;
     const int hi = halo_slot_w<HW, BN>(i), hj = halo_slot_w<HW, BN>(j);
-    const int oc = slot * NW * (BN * BN) + j * BN + i;
-    const int ox = T::RING + j * H2 + hi;
-    const int oy = T::RING + T::HX + hj * BN + i;
-    const int oz = T::RING + T::HX + T::HY + hj * H2 + hi;
-    base = ii ? (jj ? oc : oy) : (jj ? ox : oz);
-    stride = ii ? (jj ? BN * BN : H2 * BN) : (jj ? H2 * BN : H2 * H2);
+    const int oc = slot * T::PLANE + j * BN + i;
+    const int ox = T::OX + j * H2 + hi;
+    const int oy = T::OY + hj * BN + i;
+    const int oz = T::OC + hj * H2 + hi;
+    return ii ? (jj ? oc : oy) : (jj ? ox : oz);
   }
   __device__ __forceinline__ TF &center(int slot, int v, int i, int j) {
-    return ring[(slot * NW + v) * (BN * BN) + j * BN + i];
+    return w[v * T::VS + slot * T::PLANE + j * BN + i];
   }
 };
 
@@ -495,20 +491,20 @@ struct FaceFlux64 {
   uint32_t st;
 };
 
-template <class TF, bool MHD, int NDIR, bool GLM, int NDIM, int SOLVER, int LIM, int BS>
-__device__ __noinline__ FaceFlux64<Vars<MHD, NDIR, GLM>::NW> face_retry_fp64(
-    const TF *smem, int D, int b0, int b1, int b2, int b3, int s0, int s1, int s2, int s3, double rd, double cg,
-    const PhysParams P) {
+template <class TF, bool MHD, int NDIR, bool GLM, int NDIM, int SOLVER, int LIM, int BS, int VS>
+__device__ __noinline__ FaceFlux64<Vars<MHD, NDIR, GLM>::NW> face_retry_fp64(const TF *smem, int D, int b0, int b1,
+                                                                            int b2, int b3, double rd, double cg,
+                                                                            const PhysParams P) {
   using V = Vars<MHD, NDIR, GLM>;
   constexpr int NW = V::NW;
-  const int base[4] = {b0, b1, b2, b3}, strd[4] = {s0, s1, s2, s3};
+  const int base[4] = {b0, b1, b2, b3};
   double wLp[NW], wRp[NW];
 #pragma unroll
   for (int v = 0; v < NW; ++v) {
     const int ov = orig_index_rt<MHD, NDIR>(v, D);
     double q[4];
 #pragma unroll
-    for (int o = 0; o < 4; ++o) q[o] = double(smem[base[o] + ov * strd[o]]);
+    for (int o = 0; o < 4; ++o) q[o] = double(smem[base[o] + ov * VS]);
     const double d0 = q[1] - q[0], d1 = q[2] - q[1], d2 = q[3] - q[2];
     double ldw, rdw;
     face_slopes<double, LIM>(P.limiter, d0, d1, d2, rd, ldw, rdw);
@@ -569,24 +565,23 @@ __device__ __forceinline__ bool sv_near_floor(const float *wLp, const float *wRp
 
 // MUSCL-Hancock predictor, one direction D (hancock, src/mod_finite_volume.t:
 // 56-101; reconstruct_LR default branch 1171-1222): from the primitives of
-// cells c-1, c, c+1 along D (shared-memory offsets base[o], strides strd[o]),
+// cells c-1, c, c+1 along D (shared-memory offsets base[o], variables VS apart),
 // the cell's limited edge states — right edge wprim + ldw/2 (the left state of
 // the face above), left edge wprim - rdw/2 (the right state of the face
 // below) — the primitive small-value check on both, their conserved forms and
 // physical fluxes, and wnew += -qdt/dx (f(right edge) - f(left edge)).  No
 // Riemann solver and no GLM state modification.  D is a template parameter
 // so the accumulator index stays compile-time (registers, no local memory).
-template <bool MHD, int NDIR, bool GLM, int LIM, int D>
-__device__ __forceinline__ uint32_t hancock_dir(const double *smem, const int *base, const int *strd, double rd,
-                                                double sc, double cg, const PhysParams &P, double *acc) {
+template <bool MHD, int NDIR, bool GLM, int LIM, int D, int VS>
+__device__ __forceinline__ uint32_t hancock_dir(const double *smem, const int *base, double rd, double sc, double cg,
+                                                const PhysParams &P, double *acc) {
   using V = Vars<MHD, NDIR, GLM>;
   constexpr int NW = V::NW;
   double wl[NW], wr[NW];
 #pragma unroll
   for (int v = 0; v < NW; ++v) {
     const int ov = orig_index<MHD, NDIR, D>(v);
-    const double q0 = smem[base[0] + ov * strd[0]], q1 = smem[base[1] + ov * strd[1]],
-                 q2 = smem[base[2] + ov * strd[2]];
+    const double q0 = smem[base[0] + ov * VS], q1 = smem[base[1] + ov * VS], q2 = smem[base[2] + ov * VS];
     const double dm = q1 - q0, dp = q2 - q1;
     wr[v] = q1 + 0.5 * limited_slope<double, true, LIM>(P.limiter, dp, dm, rd);
     wl[v] = q1 - 0.5 * limited_slope<double, false, LIM>(P.limiter, dp, dm, rd);
@@ -711,6 +706,8 @@ __global__ void __launch_bounds__(StageOcc<TF, LIM, BN, VAR>::THREADS, StageOcc<
   constexpr bool RETRY = !FP64 || FASTF;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   TF *smem = reinterpret_cast<TF *>(smem_raw);
+  using TileT = Tile<TF, NW, NDIM, HW, TB>;
+  constexpr int VS = TileT::VS;
   TileView<TF, NW, NDIM, HW, TB> tv(smem);
   const int t = threadIdx.x;
   // Work: global tile-planes g = (block*NT + tile)*PL + k (PL = BN in 3-D,
@@ -809,7 +806,7 @@ __global__ void __launch_bounds__(StageOcc<TF, LIM, BN, VAR>::THREADS, StageOcc<
         pend = true;
         if (t == 0)
           plane_copy_async(smem_addr(&s_mbar), smem_addr(&tv.center(ring_slot<HW>(kk), 0, 0, 0)),
-                           (uint32_t)(sizeof(double) * TB * TB), A.uin + cell_offset<3>(src, NW, 0, 0, 0, sk, BN),
+                           (uint32_t)(sizeof(double) * VS), A.uin + cell_offset<3>(src, NW, 0, 0, 0, sk, BN),
                            (size_t)BN * BN * BN, NW, (uint32_t)(sizeof(double) * TB * TB));
       }
     }
@@ -851,31 +848,27 @@ __global__ void __launch_bounds__(StageOcc<TF, LIM, BN, VAR>::THREADS, StageOcc<
     // (small tiles have fewer threads than halo cells: a thread may take two)
 #pragma unroll 1
     for (int h = t; h < nhalo; h += THREADS) {
-      int i, j, stride;
-      TF *dst;
+      int i, j, dst;
       if (h < NHX) {
         j = h / H2;
         const int c = h - j * H2;
         i = c < HW ? c - HW : c + TB - HW;
-        dst = tv.hx + j * H2 + c;
-        stride = TB * H2;
+        dst = TileT::OX + h;
       } else if (h < NHX + NHY) {
         const int r = (h - NHX) / TB;
         i = (h - NHX) - r * TB;
         j = r < HW ? r - HW : r + TB - HW;
-        dst = tv.hy + r * TB + i;
-        stride = H2 * TB;
+        dst = TileT::OX + h;
       } else {
         const int r = (h - NHX - NHY) / H2, c = (h - NHX - NHY) - r * H2;
         i = c < HW ? c - HW : c + TB - HW;
         j = r < HW ? r - HW : r + TB - HW;
-        dst = tv.hc + r * H2 + c;
-        stride = H2 * H2;
+        dst = TileT::OX + h;
       }
       double w[NW];
       stb |= load_prim<MHD, NDIR, GLM, NDIM, BN>(A, b, i + ti0, j + tj0, k, w);
 #pragma unroll
-      for (int v = 0; v < NW; ++v) dst[v * stride] = TF(w[v]);
+      for (int v = 0; v < NW; ++v) smem[dst + v * VS] = TF(w[v]);
     }
     // ---- RK combination wnew0 = a*base + b*in (src/mod_advance.t:254-266)
     double acc[NW];
@@ -893,24 +886,21 @@ __global__ void __launch_bounds__(StageOcc<TF, LIM, BN, VAR>::THREADS, StageOcc<
       // staged primitives (cells c-1, c, c+1; z from ring slots k-1..k+1)
       static_assert(sizeof(TF) == 8, "the Hancock predictor is FP64 only");
       if (update && cell_thread) {
-        int base[3], strd[3];
+        int base[3];
         if (dsel < 0 || dsel == 0) {
 #pragma unroll
-          for (int o = 0; o < 3; ++o) tv.addr(slot, ci + o - 1, cj, base[o], strd[o]);
-          stb |= hancock_dir<MHD, NDIR, GLM, LIM, 0>(smem, base, strd, rdel[0], dxinv[0], cg, P, acc);
+          for (int o = 0; o < 3; ++o) base[o] = tv.off(slot, ci + o - 1, cj);
+          stb |= hancock_dir<MHD, NDIR, GLM, LIM, 0, VS>(smem, base, rdel[0], dxinv[0], cg, P, acc);
         }
         if (dsel < 0 || dsel == 1) {
 #pragma unroll
-          for (int o = 0; o < 3; ++o) tv.addr(slot, ci, cj + o - 1, base[o], strd[o]);
-          stb |= hancock_dir<MHD, NDIR, GLM, LIM, 1>(smem, base, strd, rdel[1], dxinv[1], cg, P, acc);
+          for (int o = 0; o < 3; ++o) base[o] = tv.off(slot, ci, cj + o - 1);
+          stb |= hancock_dir<MHD, NDIR, GLM, LIM, 1, VS>(smem, base, rdel[1], dxinv[1], cg, P, acc);
         }
         if (NDIM == 3 && (dsel < 0 || dsel == 2)) {
 #pragma unroll
-          for (int o = 0; o < 3; ++o) {
-            base[o] = ring_slot<HW>(k + o - 1) * NW * (TB * TB) + cj * TB + ci;
-            strd[o] = TB * TB;
-          }
-          stb |= hancock_dir<MHD, NDIR, GLM, LIM, 2>(smem, base, strd, rdel[2], dxinv[2], cg, P, acc);
+          for (int o = 0; o < 3; ++o) base[o] = ring_slot<HW>(k + o - 1) * (TB * TB) + cj * TB + ci;
+          stb |= hancock_dir<MHD, NDIR, GLM, LIM, 2, VS>(smem, base, rdel[2], dxinv[2], cg, P, acc);
         }
       }
     } else {
@@ -937,24 +927,40 @@ __global__ void __launch_bounds__(StageOcc<TF, LIM, BN, VAR>::THREADS, StageOcc<
         if (merge_yx && D == 0 && f >= FB) { FD = 1; fl = TB * TB + (f - FB); }
         else { FD = D; fl = f; }
       };
-      // where the flux of variable ov of face f lives
-      auto flux_ref = [&](int f, int FD, int fl, int ov) -> TF & {
-        return FD == D ? tv.fb[ov * FB + f] : tv.yx[ov * TB + (fl - TB * TB)];
+      // where the flux of (rotated) variable v of face f lives
+      auto flux_ref = [&](int f, int FD, int fl, int v) -> TF & {
+        return FD == D ? tv.fb[v * FB + f] : tv.yx[v * TB + (fl - TB * TB)];
       };
       // face coordinates and the shared-memory offsets of the 2 HW stencil
-      // cells (variable 0) with the per-variable strides
-      auto face_at = [&](int FD, int fl, int &fi, int &fj, int *base, int *strd) {
+      // cells (variable 0): inside the plane a step of 1 (x) or TB (y), in the
+      // halo strips their own
+      auto face_at = [&](int FD, int fl, int &fi, int &fj, int *base) {
         if (FD == 0) { fj = fl / (TB + 1); fi = fl - fj * (TB + 1); }
         else { fj = fl / TB; fi = fl - fj * TB; }
+        if (FD == 2) {
 #pragma unroll
-        for (int o = 0; o < H2; ++o) {
-          if (FD == 2) {
-            base[o] = ring_slot<HW>(k + o - HW + 1) * NW * (TB * TB) + fl;
-            strd[o] = TB * TB;
-          } else {
-            tv.addr(slot, FD == 0 ? fi + o - HW : fi, FD == 0 ? fj : fj + o - HW, base[o], strd[o]);
-          }
+          for (int o = 0; o < H2; ++o) base[o] = ring_slot<HW>(k + o - HW + 1) * TileT::PLANE + fl;
+        } else {
+          const int c0 = (FD == 0 ? fi : fj) - HW, step = FD == 0 ? 1 : TB;
+          const int cen = slot * TileT::PLANE + fj * TB + fi - HW * step;
+          const int hb = FD == 0 ? TileT::OX + fj * H2 : TileT::OY + fi;
+#pragma unroll
+          for (int o = 0; o < H2; ++o)
+            base[o] = (unsigned)(c0 + o) < (unsigned)TB ? cen + o * step : hb + halo_slot_w<HW, TB>(c0 + o) * step;
         }
+      };
+      // distance from variable 0 to (rotated) variable v: component c of the
+      // vectors is stored component (c + FD) mod NDIR, everything else is a
+      // constant
+      auto rot_of = [&](int FD, int *rot) {
+        rot[0] = FD * VS;
+        rot[1] = (FD == NDIR - 1 ? 0 : FD + 1) * VS;
+        if constexpr (NDIR == 3) rot[2] = (FD == 0 ? 2 : FD - 1) * VS;
+      };
+      auto var_off = [](int v, const int *rot) -> int {
+        if (v >= 1 && v <= NDIR) return VS + rot[v - 1];
+        if (MHD && v >= NDIR + 2 && v <= 2 * NDIR + 1) return (NDIR + 2) * VS + rot[v - NDIR - 2];
+        return v * VS;
       };
       // level jump across this block face: keep the boundary face flux
       // (store_flux, src/mod_fix_conserve.t:597-648) for the flux fix
@@ -975,8 +981,9 @@ __global__ void __launch_bounds__(StageOcc<TF, LIM, BN, VAR>::THREADS, StageOcc<
         face_dir(f, FD, fl);
         const TF rd = TF(FD == 0 ? rdel[0] : (FD == 1 ? rdel[1] : rdel[2]));
         TF wLp[NW], wRp[NW];
-        int base[H2], strd[H2];
-        face_at(FD, fl, fi, fj, base, strd);
+        int base[H2], rot[NDIR];
+        face_at(FD, fl, fi, fj, base);
+        rot_of(FD, rot);
         if constexpr (LIM == LIM_MP5) {
           static_assert(FP64, "MP5 is FP64 only");
           // MP5limiter, then fix_limiter1 (src/limiter/mod_weno.t:135-163):
@@ -985,21 +992,20 @@ __global__ void __launch_bounds__(StageOcc<TF, LIM, BN, VAR>::THREADS, StageOcc<
           // reconstructed state
 #pragma unroll
           for (int v = 0; v < NW; ++v) {
-            const int ov = orig_index_rt<MHD, NDIR>(v, FD);
             double q[6];
 #pragma unroll
-            for (int o = 0; o < 6; ++o) q[o] = smem[base[o] + ov * strd[o]];
+            for (int o = 0; o < 6; ++o) q[o] = smem[base[o] + var_off(v, rot)];
             wLp[v] = mp5_side(q[0], q[1], q[2], q[3], q[4]);
             wRp[v] = mp5_side(q[5], q[4], q[3], q[2], q[1]);
           }
           // density and energy are not rotated: variable index = tile index
           if (wLp[V::RHO] < P.small_density || wRp[V::RHO] < P.small_density) {
-            wLp[V::RHO] = smem[base[2] + V::RHO * strd[2]];
-            wRp[V::RHO] = smem[base[3] + V::RHO * strd[3]];
+            wLp[V::RHO] = smem[base[2] + V::RHO * VS];
+            wRp[V::RHO] = smem[base[3] + V::RHO * VS];
           }
           if (wLp[V::E] < P.small_pressure || wRp[V::E] < P.small_pressure) {
-            wLp[V::E] = smem[base[2] + V::E * strd[2]];
-            wRp[V::E] = smem[base[3] + V::E * strd[3]];
+            wLp[V::E] = smem[base[2] + V::E * VS];
+            wRp[V::E] = smem[base[3] + V::E * VS];
           }
         } else if constexpr (LIM == LIM_WENO5) {
           static_assert(FP64, "WENO5 is FP64 only");
@@ -1010,10 +1016,9 @@ __global__ void __launch_bounds__(StageOcc<TF, LIM, BN, VAR>::THREADS, StageOcc<
           const double lam = FD == 0 ? wlam[0] : (FD == 1 ? wlam[1] : wlam[2]);
 #pragma unroll
           for (int v = 0; v < NW; ++v) {
-            const int ov = orig_index_rt<MHD, NDIR>(v, FD);
             double q[6];
 #pragma unroll
-            for (int o = 0; o < 6; ++o) q[o] = smem[base[o] + ov * strd[o]];
+            for (int o = 0; o < 6; ++o) q[o] = smem[base[o] + var_off(v, rot)];
             wLp[v] = weno5_side(q[0], q[1], q[2], q[3], q[4], var, lam);
             wRp[v] = weno5_side(q[5], q[4], q[3], q[2], q[1], var, lam);
           }
@@ -1021,9 +1026,8 @@ __global__ void __launch_bounds__(StageOcc<TF, LIM, BN, VAR>::THREADS, StageOcc<
               wRp[V::E] < P.small_pressure) {
 #pragma unroll
             for (int v = 0; v < NW; ++v) {
-              const int ov = orig_index_rt<MHD, NDIR>(v, FD);
-              wLp[v] = smem[base[2] + ov * strd[2]];
-              wRp[v] = smem[base[3] + ov * strd[3]];
+              wLp[v] = smem[base[2] + var_off(v, rot)];
+              wRp[v] = smem[base[3] + var_off(v, rot)];
             }
           }
         } else if constexpr (LIM == LIM_WENO3) {
@@ -1035,10 +1039,9 @@ __global__ void __launch_bounds__(StageOcc<TF, LIM, BN, VAR>::THREADS, StageOcc<
           const double dx2 = dxd * dxd;
 #pragma unroll
           for (int v = 0; v < NW; ++v) {
-            const int ov = orig_index_rt<MHD, NDIR>(v, FD);
             double q[4];
 #pragma unroll
-            for (int o = 0; o < 4; ++o) q[o] = smem[base[o] + ov * strd[o]];
+            for (int o = 0; o < 4; ++o) q[o] = smem[base[o] + var_off(v, rot)];
             wLp[v] = weno3_side(q[0], q[1], q[2], var, dx2);
             wRp[v] = weno3_side(q[3], q[2], q[1], var, dx2);
           }
@@ -1046,9 +1049,8 @@ __global__ void __launch_bounds__(StageOcc<TF, LIM, BN, VAR>::THREADS, StageOcc<
               wRp[V::E] < P.small_pressure) {
 #pragma unroll
             for (int v = 0; v < NW; ++v) {
-              const int ov = orig_index_rt<MHD, NDIR>(v, FD);
-              wLp[v] = smem[base[1] + ov * strd[1]];
-              wRp[v] = smem[base[2] + ov * strd[2]];
+              wLp[v] = smem[base[1] + var_off(v, rot)];
+              wRp[v] = smem[base[2] + var_off(v, rot)];
             }
           }
         } else if constexpr (LIM == LIM_VENK) {
@@ -1058,20 +1060,18 @@ __global__ void __launch_bounds__(StageOcc<TF, LIM, BN, VAR>::THREADS, StageOcc<
           const double eps2 = kd * kd * kd;
 #pragma unroll
           for (int v = 0; v < NW; ++v) {
-            const int ov = orig_index_rt<MHD, NDIR>(v, FD);
             double q[4];
 #pragma unroll
-            for (int o = 0; o < 4; ++o) q[o] = smem[base[o] + ov * strd[o]];
+            for (int o = 0; o < 4; ++o) q[o] = smem[base[o] + var_off(v, rot)];
             wLp[v] = q[1] + 0.25 * (q[2] - q[0]) * venk_phi(q[0], q[1], q[2], eps2);
             wRp[v] = q[2] - 0.25 * (q[3] - q[1]) * venk_phi(q[1], q[2], q[3], eps2);
           }
         } else {
 #pragma unroll
           for (int v = 0; v < NW; ++v) {
-            const int ov = orig_index_rt<MHD, NDIR>(v, FD);
             TF q[4];
 #pragma unroll
-            for (int o = 0; o < 4; ++o) q[o] = smem[base[o] + ov * strd[o]];
+            for (int o = 0; o < 4; ++o) q[o] = smem[base[o] + var_off(v, rot)];
             const TF d0 = q[1] - q[0], d1 = q[2] - q[1], d2 = q[3] - q[2];
             TF ldw, rdw;
             face_slopes<TF, LIM, FASTF>(P.limiter, d0, d1, d2, rd, ldw, rdw);
@@ -1087,8 +1087,8 @@ __global__ void __launch_bounds__(StageOcc<TF, LIM, BN, VAR>::THREADS, StageOcc<
             TF srho = TF(0), sp = TF(0);
 #pragma unroll
             for (int o = 0; o < 4; ++o) {
-              srho = fmaxf(srho, fabsf(smem[base[o] + V::RHO * strd[o]]));
-              sp = fmaxf(sp, fabsf(smem[base[o] + V::E * strd[o]]));
+              srho = fmaxf(srho, fabsf(smem[base[o] + V::RHO * VS]));
+              sp = fmaxf(sp, fabsf(smem[base[o] + V::E * VS]));
             }
             near = sv_near_floor<MHD, NDIR, GLM>(wLp, wRp, srho, sp, P);
           }
@@ -1115,9 +1115,8 @@ __global__ void __launch_bounds__(StageOcc<TF, LIM, BN, VAR>::THREADS, StageOcc<
         const double sc = FD == 0 ? dxinv[0] : (FD == 1 ? dxinv[1] : dxinv[2]);
 #pragma unroll
         for (int v = 0; v < NW; ++v) {
-          const int ov = orig_index_rt<MHD, NDIR>(v, FD);
-          if constexpr (FP64) flux_ref(f, FD, fl, ov) = sc * Fr[v];
-          else flux_ref(f, FD, fl, ov) = Fr[v];
+          if constexpr (FP64) flux_ref(f, FD, fl, v) = sc * Fr[v];
+          else flux_ref(f, FD, fl, v) = Fr[v];
         }
         if (amr_mask) capture(FD, fi, fj, Fr, sc);
       }
@@ -1134,13 +1133,13 @@ __global__ void __launch_bounds__(StageOcc<TF, LIM, BN, VAR>::THREADS, StageOcc<
             for (int v = 0; v < NW; ++v) finite = finite && isfinite(flux_ref(f, FD, fl, v));
             if (finite) continue;
             const double sc = FD == 0 ? dxinv[0] : (FD == 1 ? dxinv[1] : dxinv[2]);
-            int fi, fj, base[H2], strd[H2];
-            face_at(FD, fl, fi, fj, base, strd);
+            int fi, fj, base[H2];
+            face_at(FD, fl, fi, fj, base);
             const double rdd = FD == 0 ? rdel[0] : (FD == 1 ? rdel[1] : rdel[2]);
             FaceFlux64<NW> r;
             if constexpr (FP64)
-              r = face_retry_fp64<TF, MHD, NDIR, GLM, NDIM, SOLVER, LIM, BS>(
-                  smem, FD, base[0], base[1], base[2], base[3], strd[0], strd[1], strd[2], strd[3], rdd, cg, P);
+              r = face_retry_fp64<TF, MHD, NDIR, GLM, NDIM, SOLVER, LIM, BS, VS>(smem, FD, base[0], base[1], base[2],
+                                                                                 base[3], rdd, cg, P);
             else  // the R cell of the face, block-local
               r = face_retry_state<MHD, NDIR, GLM, NDIM, SOLVER, LIM, BS, BN>(
                   &A, b, FD, ti0 + fi, tj0 + fj, FD == 2 ? k + 1 : k, rdd, cg);
@@ -1149,7 +1148,7 @@ __global__ void __launch_bounds__(StageOcc<TF, LIM, BN, VAR>::THREADS, StageOcc<
             for (int v = 0; v < NW; ++v) {
               Fr[v] = TF(r.F[v]);
               // FP64 keeps the scaled flux fC = -qdt/dx f, mixed the FP32 flux
-              flux_ref(f, FD, fl, orig_index_rt<MHD, NDIR>(v, FD)) = FP64 ? TF(sc * r.F[v]) : Fr[v];
+              flux_ref(f, FD, fl, v) = FP64 ? TF(sc * r.F[v]) : Fr[v];
             }
             if (amr_mask) capture(FD, fi, fj, Fr, sc);
           }
@@ -1159,27 +1158,31 @@ __global__ void __launch_bounds__(StageOcc<TF, LIM, BN, VAR>::THREADS, StageOcc<
       }
       if (cell_thread) {
         const double sc = FP64 ? 1.0 : (D == 0 ? dxinv[0] : (D == 1 ? dxinv[1] : dxinv[2]));
+        // the fluxes are stored rotated: entry v is variable orig_index<D>(v)
         if (D == 0) {
           const int f = cj * (TB + 1) + ci;
 #pragma unroll
           for (int v = 0; v < NW; ++v) {
-            if constexpr (FP64) acc[v] = acc[v] + tv.fb[v * FB + f + 1] - tv.fb[v * FB + f];
-            else acc[v] = acc[v] + sc * double(tv.fb[v * FB + f + 1]) - sc * double(tv.fb[v * FB + f]);
+            double &a = acc[orig_index<MHD, NDIR, 0>(v)];
+            if constexpr (FP64) a = a + tv.fb[v * FB + f + 1] - tv.fb[v * FB + f];
+            else a = a + sc * double(tv.fb[v * FB + f + 1]) - sc * double(tv.fb[v * FB + f]);
           }
         } else if (D == 1) {
           const int f = cj * TB + ci;
 #pragma unroll
           for (int v = 0; v < NW; ++v) {
+            double &a = acc[orig_index<MHD, NDIR, 1>(v)];
             // the face above the top row was computed in the x phase
             const TF up = (merge_yx && cj == TB - 1) ? tv.yx[v * TB + ci] : tv.fb[v * FB + f + TB];
-            if constexpr (FP64) acc[v] = acc[v] + up - tv.fb[v * FB + f];
-            else acc[v] = acc[v] + sc * double(up) - sc * double(tv.fb[v * FB + f]);
+            if constexpr (FP64) a = a + up - tv.fb[v * FB + f];
+            else a = a + sc * double(up) - sc * double(tv.fb[v * FB + f]);
           }
         } else if constexpr (NDIM == 3) {
 #pragma unroll
           for (int v = 0; v < NW; ++v) {
+            double &a = acc[orig_index<MHD, NDIR, 2>(v)];
             const double fz = FP64 ? double(tv.fb[v * FB + t]) : sc * double(tv.fb[v * FB + t]);
-            if (update) acc[v] = acc[v] + fz - fz_prev[v];
+            if (update) a = a + fz - fz_prev[v];
             fz_prev[v] = fz;
           }
         }
@@ -1220,7 +1223,7 @@ __global__ void __launch_bounds__(StageOcc<TF, LIM, BN, VAR>::THREADS, StageOcc<
               auto nbv = [&](int d, int s, int v) -> double {  // wCT at cell +/- e_d
                 if (d == 0) return double(tv.at(slot, v, ci + s, cj));
                 if (d == 1) return double(tv.at(slot, v, ci, cj + s));
-                return double(tv.ring[(ring_slot<HW>(k + s) * NW + v) * (TB * TB) + cj * TB + ci]);
+                return double(tv.center(ring_slot<HW>(k + s), v, ci, cj));
               };
 #pragma unroll
               for (int d = 0; d < NDIM; ++d) {

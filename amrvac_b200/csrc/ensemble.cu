@@ -179,11 +179,8 @@ __device__ __forceinline__ uint32_t ens_face_at(const TF *s, const EnsView<TF, N
     TF q[4];
 #pragma unroll
     for (int o = 0; o < 4; ++o) q[o] = s[base[o] + ov * strd[o]];
-    const TF d0 = q[1] - q[0], d1 = q[2] - q[1], d2 = q[3] - q[2];
-    TF ldw, rdw;
-    face_slopes<TF, 0, sizeof(TF) == 4>(lim, d0, d1, d2, rd, ldw, rdw);
-    wLp[v] = q[1] + TF(0.5) * ldw;
-    wRp[v] = q[2] - TF(0.5) * rdw;
+    bool special = false;
+    face_states<TF, 0, sizeof(TF) == 4>(lim, q[0], q[1], q[2], q[3], rd, wLp[v], wRp[v], special);
   }
   TF Fr[NW];
   uint32_t st;

@@ -297,9 +297,10 @@ __device__ __forceinline__ void phys_flux(const T *wc, const T *w, T cg,
   }
 }
 
-// mhd_get_csound_prim (mod_mhd_phys.t:3329-3379): fast magnetosonic speed.
+// mhd_get_csound_prim (mod_mhd_phys.t:3329-3379): the square of the fast
+// magnetosonic speed, and the speed.
 template <class T, int NDIR, int BN, bool FAST = false>
-__device__ __forceinline__ T fast_speed(const T *w, const PhysParams &P) {
+__device__ __forceinline__ T fast_speed2(const T *w, const PhysParams &P) {
   constexpr int RHO = 0, E = NDIR + 1, B0 = NDIR + 2;
   const T inv_rho = rcp_f<FAST>(w[RHO]);
   const T cs = T(P.gamma) * w[E] * inv_rho;
@@ -309,12 +310,19 @@ __device__ __forceinline__ T fast_speed(const T *w, const PhysParams &P) {
   const T cfast2 = b2 * inv_rho + cs;
   T av = cfast2 * cfast2 - T(4.0) * cs * (w[BN] * w[BN]) * inv_rho;
   if (av < T(0.0)) av = T(0.0);
-  return sqrt_f<FAST>(T(0.5) * (cfast2 + sqrt_f<FAST>(av)));
+  return T(0.5) * (cfast2 + sqrt_f<FAST>(av));
+}
+template <class T, int NDIR, int BN, bool FAST = false>
+__device__ __forceinline__ T fast_speed(const T *w, const PhysParams &P) {
+  return sqrt_f<FAST>(fast_speed2<T, NDIR, BN, FAST>(w, P));
 }
 
 // hd_get_cbounds (mod_hd_phys.t:891-1001) / mhd_get_cbounds (mod_mhd_phys.t:3037-3127).
 // WITH_MIN=false gives the tvdlf form (cmax only).  Returns a status bit.
-template <class T, bool MHD, int NDIR, bool GLM, int D, bool WITH_MIN, int BS = 0, bool FAST = false>
+// SQUARED: the Einfeldt mean takes the squares of the fast speeds directly;
+// the reference squares the speeds (two square roots more, rounding apart).
+template <class T, bool MHD, int NDIR, bool GLM, int D, bool WITH_MIN, int BS = 0, bool FAST = false,
+          bool SQUARED = false>
 __device__ __forceinline__ uint32_t cbounds(const T *wLC, const T *wRC, const T *wLp,
                                             const T *wRp, const PhysParams &P, T &cmax,
                                             T &cmin) {
@@ -330,9 +338,17 @@ __device__ __forceinline__ uint32_t cbounds(const T *wLC, const T *wRC, const T 
     const T dv = wRp[MN] - wLp[MN];
     T dmean;
     if constexpr (MHD) {
-      const T csL = fast_speed<T, NDIR, V::B0 + D, FAST>(wLp, P);
-      const T csR = fast_speed<T, NDIR, V::B0 + D, FAST>(wRp, P);
-      dmean = sqrt_f<FAST>((tmp1 * (csL * csL) + tmp2 * (csR * csR)) * tmp3 +
+      T csL2, csR2;
+      if constexpr (SQUARED) {
+        csL2 = fast_speed2<T, NDIR, V::B0 + D, FAST>(wLp, P);
+        csR2 = fast_speed2<T, NDIR, V::B0 + D, FAST>(wRp, P);
+      } else {
+        const T csL = fast_speed<T, NDIR, V::B0 + D, FAST>(wLp, P);
+        const T csR = fast_speed<T, NDIR, V::B0 + D, FAST>(wRp, P);
+        csL2 = csL * csL;
+        csR2 = csR * csR;
+      }
+      dmean = sqrt_f<FAST>((tmp1 * csL2 + tmp2 * csR2) * tmp3 +
                    T(0.5) * tmp1 * tmp2 * (tmp3 * tmp3) * (dv * dv));
     } else {
       const T csL = div_f<FAST>(T(P.gamma) * wLp[V::E], wLp[V::RHO]);
@@ -471,17 +487,43 @@ __device__ __forceinline__ T limited_slope(int lim_rt, T a, T b, T rdelinv) {
   return slope_impl<T, LEFT>(LIM ? LIM : lim_rt, a, b, rdelinv);
 }
 
-// phi of the cada3 / schmid limiters (dwlimiter2, src/limiter/mod_limiter.t:
-// 253-290, 291-333) from the slope ratio t and tmpeta: the asymptotic third-
-// order form below 1 - cadepsilon, the limited form above 1 + cadepsilon,
-// their blend in between.  alfa / gam: 0.5 / 1.6 (cada3), 1 / 1.5 (schmid).
-// The blend is formed only inside its 2e-14 wide band.
+// Minimum and maximum of finite numbers.  In FP64 one compare and a select:
+// fmin / fmax also order NaN operands, which takes two or three instructions
+// more (a NaN here reaches the flux through the state that held it).
+__device__ __forceinline__ double min_(double a, double b) { return a < b ? a : b; }
+__device__ __forceinline__ double max_(double a, double b) { return a > b ? a : b; }
+__device__ __forceinline__ float min_(float a, float b) { return fminf(a, b); }
+__device__ __forceinline__ float max_(float a, float b) { return fmaxf(a, b); }
+__device__ __forceinline__ bool is_negative(double x) { return __double2hiint(x) < 0; }
+__device__ __forceinline__ bool is_negative(float x) { return __float_as_int(x) < 0; }
+
+// Asymptotic and limited form of the cada3 / schmid limiters (dwlimiter2,
+// src/limiter/mod_limiter.t:253-290, 291-333) at the slope ratio t:
+//   A = (2 + t) / 3,
+//   max(0, min(A, max(-alfa t, min(2 t, A, gam)))).
+// For t >= 0 the inner maximum is min(2 t, A, gam) >= 0; for t < 0 it is
+// -alfa t, and A < gam.  So with u = 2 t or -alfa t the limited form is
+// max(0, min(A, u, gam)): three minima and maxima instead of five.
+template <class T>
+__device__ __forceinline__ T cada_asymptotic(T t) {
+  constexpr T third = T(1.0) / T(3.0);
+  return (T(2.0) + t) * third;
+}
+template <class T>
+__device__ __forceinline__ T cada_limited(T t, T A, T alfa, T gam) {
+  const T u = t * (is_negative(t) ? -alfa : T(2.0));
+  const T m = min_(min_(A, u), gam);
+  return is_negative(m) ? T(0.0) : m;
+}
+
+// phi of the cada3 / schmid limiters from the slope ratio t and tmpeta: the
+// asymptotic form below 1 - cadepsilon, the limited form above
+// 1 + cadepsilon, their blend in between.  alfa / gam: 0.5 / 1.6 (cada3),
+// 1 / 1.5 (schmid).  The blend is formed only inside its 2e-14 wide band.
 template <class T>
 __device__ __forceinline__ T cada_blend_phi(T t, T tmpeta, T alfa, T gam) {
-  constexpr T cadbeta = T(2.0), cadepsilon = T(1.0e-14), invcadepsilon = T(1.0e14);
-  constexpr T third = T(1.0) / T(3.0);
-  const T A = (T(2.0) + t) * third;
-  const T lim2 = fmax(T(0.0), fmin(A, fmax(-(alfa * t), fmin(fmin(cadbeta * t, A), gam))));
+  constexpr T cadepsilon = T(1.0e-14), invcadepsilon = T(1.0e14);
+  const T A = cada_asymptotic(t), lim2 = cada_limited(t, A, alfa, gam);
   const bool low = tmpeta <= T(1.0) - cadepsilon;
   T phi = low ? A : lim2;
   if (!low && !(tmpeta >= T(1.0) + cadepsilon)) {
@@ -491,37 +533,73 @@ __device__ __forceinline__ T cada_blend_phi(T t, T tmpeta, T alfa, T gam) {
   return phi;
 }
 
-// Both limited slopes of one face i+1/2 and one variable from the centred
-// differences d0 = w(i)-w(i-1), d1 = w(i+1)-w(i), d2 = w(i+2)-w(i+1):
-// ldw of cell i (dwlimiter2 with a = d1, b = d0) and rdw of cell i+1
-// (a = d2, b = d1).  The cada family divides both ratios by the same
-// d1 + sign(eps, d1), so one reciprocal serves the face; the other limiters
-// take slope_impl as it is.
-template <class T, int LIM, bool FAST = false>
-__device__ __forceinline__ void face_slopes(int lim_rt, T d0, T d1, T d2, T rdelinv, T &ldw, T &rdw) {
+// tmpeta = s / r2 close to 1, by the high words (within 2^-19, which holds
+// the 2e-14 wide blending band): the hot loop leaves such a face to the
+// recomputation instead of carrying the blend's code.  In FP32 the band is
+// empty.
+__device__ __forceinline__ bool near_one(double s, double r2) {
+  return (unsigned)(__double2hiint(s) - __double2hiint(r2) + 1) <= 2u;
+}
+__device__ __forceinline__ bool near_one(float, float) { return false; }
+
+// Left and right state of one face i+1/2 and one variable from the cells
+// i-1 .. i+2: w(i) + ldw(i) / 2 and w(i+1) - rdw(i+1) / 2 with the limited
+// slopes of dwlimiter2 from the centred differences (ldw of cell i: a = d1,
+// b = d0; rdw of cell i+1: a = d2, b = d1).  The cada family divides both
+// ratios by the same d1 + sign(eps, d1), so one reciprocal serves the face;
+// the other limiters take slope_impl as it is.  rdel is what rdelinv is in
+// slope_impl, except with R2 (limiter fixed to cada3): then it is
+// (cada3_radius dx)^2 and tmpeta <= 1 is tested as a^2 + b^2 <= rdel without
+// the product.  With the limiter fixed to cada3 and BLEND false the blending
+// band is left out: a face near it gets `special` and is recomputed.
+template <class T, int LIM, bool FAST = false, bool R2 = false, bool BLEND = true>
+__device__ __forceinline__ void face_states(int lim_rt, T q0, T q1, T q2, T q3, T rdel, T &wL, T &wR, bool &special) {
   constexpr T eps = T(1.4901161193847656e-08);  // sqrt(epsilon(1d0)) = 2**-26
   const int lim = LIM ? LIM : lim_rt;
-  if (lim == LIM_CADA3 || lim == LIM_CADA || lim == LIM_SCHMID) {
+  const T d0 = q1 - q0, d1 = q2 - q1, d2 = q3 - q2;
+  if constexpr (LIM == LIM_CADA3) {
     const T rinv = rcp_f<FAST>(d1 + fsign(eps, d1));
     const T tl = d0 * rinv, tr = d2 * rinv;
+    const T sl = d1 * d1 + d0 * d0, sr = d2 * d2 + d1 * d1;
     T pl, pr;
-    if (lim == LIM_CADA3) {
-      pl = cada_blend_phi<T>(tl, (d1 * d1 + d0 * d0) * rdelinv, T(0.5), T(1.6));
-      pr = cada_blend_phi<T>(tr, (d2 * d2 + d1 * d1) * rdelinv, T(0.5), T(1.6));
-    } else if (lim == LIM_SCHMID) {  // rdelinv carries (a2max + cadepsilon) dx^2
-      pl = cada_blend_phi<T>(tl, sqrt_f<FAST>(T(0.4) * (d1 * d1 + d0 * d0)) / rdelinv, T(1.0), T(1.5));
-      pr = cada_blend_phi<T>(tr, sqrt_f<FAST>(T(0.4) * (d2 * d2 + d1 * d1)) / rdelinv, T(1.0), T(1.5));
-    } else {  // cada
-      constexpr T third = T(1.0) / T(3.0);
-      const T al = (T(2.0) + tl) * third, ar = (T(2.0) + tr) * third;
-      pl = fmax(T(0.0), fmin(al, fmax(-(T(0.5) * tl), fmin(fmin(T(2.0) * tl, al), T(1.6)))));
-      pr = fmax(T(0.0), fmin(ar, fmax(-(T(0.5) * tr), fmin(fmin(T(2.0) * tr, ar), T(1.6)))));
+    if constexpr (BLEND) {
+      const T rdelinv = R2 ? T(1.0) / rdel : rdel;
+      pl = cada_blend_phi<T>(tl, sl * rdelinv, T(0.5), T(1.6));
+      pr = cada_blend_phi<T>(tr, sr * rdelinv, T(0.5), T(1.6));
+    } else {
+      const T Al = cada_asymptotic(tl), Ar = cada_asymptotic(tr);
+      const T el = R2 ? sl : sl * rdel, er = R2 ? sr : sr * rdel, one = R2 ? rdel : T(1.0);
+      pl = el <= one ? Al : cada_limited(tl, Al, T(0.5), T(1.6));
+      pr = er <= one ? Ar : cada_limited(tr, Ar, T(0.5), T(1.6));
+      special = special || near_one(el, one) || near_one(er, one);
     }
-    ldw = pl * d1;  // phi * a (left), phi * b (right): both d1
-    rdw = pr * d1;
+    const T ldw = pl * d1, rdw = pr * d1;  // phi * a (left), phi * b (right): both d1
+    wL = q1 + T(0.5) * ldw;
+    wR = q2 - T(0.5) * rdw;
   } else {
-    ldw = slope_impl<T, true, FAST>(lim, d1, d0, rdelinv);
-    rdw = slope_impl<T, false, FAST>(lim, d2, d1, rdelinv);
+    T ldw, rdw;
+    if (lim == LIM_CADA3 || lim == LIM_CADA || lim == LIM_SCHMID) {
+      const T rinv = rcp_f<FAST>(d1 + fsign(eps, d1));
+      const T tl = d0 * rinv, tr = d2 * rinv;
+      T pl, pr;
+      if (lim == LIM_CADA3) {
+        pl = cada_blend_phi<T>(tl, (d1 * d1 + d0 * d0) * rdel, T(0.5), T(1.6));
+        pr = cada_blend_phi<T>(tr, (d2 * d2 + d1 * d1) * rdel, T(0.5), T(1.6));
+      } else if (lim == LIM_SCHMID) {  // rdel carries (a2max + cadepsilon) dx^2
+        pl = cada_blend_phi<T>(tl, sqrt_f<FAST>(T(0.4) * (d1 * d1 + d0 * d0)) / rdel, T(1.0), T(1.5));
+        pr = cada_blend_phi<T>(tr, sqrt_f<FAST>(T(0.4) * (d2 * d2 + d1 * d1)) / rdel, T(1.0), T(1.5));
+      } else {  // cada
+        pl = cada_limited(tl, cada_asymptotic(tl), T(0.5), T(1.6));
+        pr = cada_limited(tr, cada_asymptotic(tr), T(0.5), T(1.6));
+      }
+      ldw = pl * d1;  // phi * a (left), phi * b (right): both d1
+      rdw = pr * d1;
+    } else {
+      ldw = slope_impl<T, true, FAST>(lim, d1, d0, rdel);
+      rdw = slope_impl<T, false, FAST>(lim, d2, d1, rdel);
+    }
+    wL = q1 + T(0.5) * ldw;
+    wR = q2 - T(0.5) * rdw;
   }
 }
 

@@ -297,11 +297,9 @@ __global__ void __launch_bounds__(256) sv_stage_kernel(const StageArgs A, const 
         if (!in) continue;
         for (int v = 0; v < NW; ++v) {
           const double *q = Pa + v * cs;
-          const double d0 = q[c] - q[c - o], d1 = q[c + o] - q[c], d2 = q[c + 2 * o] - q[c + o];
-          double ldw, rdw;
-          face_slopes<double, 0>(P.limiter, d0, d1, d2, rdel[D], ldw, rdw);
-          L[v * cs + c] = q[c] + 0.5 * ldw;
-          Rr[v * cs + c] = q[c + o] - 0.5 * rdw;
+          bool special = false;
+          face_states<double, 0>(P.limiter, q[c - o], q[c], q[c + o], q[c + 2 * o], rdel[D], L[v * cs + c],
+                                 Rr[v * cs + c], special);
         }
       }
       __syncthreads();

@@ -220,6 +220,8 @@ __device__ __forceinline__ uint32_t load_prim(const StageArgs &A, int b, int i, 
 // Interface flux from reconstructed primitive left/right states: small-value
 // fix, to_conserved, GLM modify_wLR, physical fluxes, cbounds, Riemann solver
 // (src/mod_finite_volume.t:1217-1222, 200-245).  wLp/wRp are modified.
+// HLLD and the HD HLLC form the physical flux themselves, of the side of the
+// contact that the face lies in.
 template <class T, bool MHD, int NDIR, bool GLM, int NDIM, int SOLVER, int BS, bool FAST = false>
 __device__ __forceinline__ uint32_t face_from_states(T *wLp, T *wRp, const PhysParams &P, T cg, T *F,
                                                      bool small_check = true) {
@@ -232,11 +234,14 @@ __device__ __forceinline__ uint32_t face_from_states(T *wLp, T *wRp, const PhysP
     bool fr = small_values<T, MHD, NDIR, GLM>(wRp, true, P);
     if ((fl || fr) && P.small_values_method != 1) st |= ST_SMALL_VALUE;
   }
+  constexpr bool PRIM = SOLVER == SOLVER_HLLD && hlld_from_primitives<T, NDIM>;
   T wLC[NW], wRC[NW];
+  if constexpr (!PRIM) {
 #pragma unroll
-  for (int v = 0; v < NW; ++v) { wLC[v] = wLp[v]; wRC[v] = wRp[v]; }
-  to_conserved<T, MHD, NDIR, GLM>(wLC, P);
-  to_conserved<T, MHD, NDIR, GLM>(wRC, P);
+    for (int v = 0; v < NW; ++v) { wLC[v] = wLp[v]; wRC[v] = wRp[v]; }
+    to_conserved<T, MHD, NDIR, GLM>(wLC, P);
+    to_conserved<T, MHD, NDIR, GLM>(wRC, P);
+  }
   if constexpr (MHD && GLM) {
     // mhd_modify_wLR (src/mhd/mod_mhd_phys.t:6352-6372)
     constexpr int BNI = V::B0 + D, PS = V::PSI, E = V::E;
@@ -245,37 +250,48 @@ __device__ __forceinline__ uint32_t face_from_states(T *wLp, T *wRp, const PhysP
     const T nb = T(0.5) * (wRp[BNI] + wLp[BNI] - div_f<FAST>(dPsi, cg));
     const T np = T(0.5) * (wRp[PS] + wLp[PS] - dB * cg);
     wLp[BNI] = nb; wLp[PS] = np; wRp[BNI] = nb; wRp[PS] = np;
-    wRC[E] = wRC[E] - T(0.5) * (wRC[BNI] * wRC[BNI]);
-    wLC[E] = wLC[E] - T(0.5) * (wLC[BNI] * wLC[BNI]);
-    wRC[BNI] = nb; wRC[PS] = np; wLC[BNI] = nb; wLC[PS] = np;
-    wRC[E] = wRC[E] + T(0.5) * (nb * nb);
-    wLC[E] = wLC[E] + T(0.5) * (nb * nb);
-  }
-  T fL[NW], fR[NW];
-  phys_flux<T, MHD, NDIR, GLM, D>(wLC, wLp, cg, fL);
-  phys_flux<T, MHD, NDIR, GLM, D>(wRC, wRp, cg, fR);
-  T cmax, cmin = T(0.0);
-  if constexpr (SOLVER == SOLVER_TVDMU) {
-    (void)cmax;
-    if constexpr (MHD) {
-      static_assert(!GLM, "TVD-MUSCL with GLM is not built");
-      riemann_tvdmu_mhd<T, NDIR>(wLC, wRC, fL, fR, P, F);
-    } else {
-      riemann_tvdmu_hd<T, NDIR>(wLC, wRC, fL, fR, P, F);
+    if constexpr (!PRIM) {
+      wRC[E] = wRC[E] - T(0.5) * (wRC[BNI] * wRC[BNI]);
+      wLC[E] = wLC[E] - T(0.5) * (wLC[BNI] * wLC[BNI]);
+      wRC[BNI] = nb; wRC[PS] = np; wLC[BNI] = nb; wLC[PS] = np;
+      wRC[E] = wRC[E] + T(0.5) * (nb * nb);
+      wLC[E] = wLC[E] + T(0.5) * (nb * nb);
     }
-  } else if constexpr (SOLVER == SOLVER_TVDLF) {
-    st |= cbounds<T, MHD, NDIR, GLM, D, false, BS, FAST>(wLC, wRC, wLp, wRp, P, cmax, cmin);
-    riemann_tvdlf<T, NW>(wLC, wRC, fL, fR, cmax, T(P.tvdlfeps), F);
-  } else {
-    st |= cbounds<T, MHD, NDIR, GLM, D, true, BS, FAST>(wLC, wRC, wLp, wRp, P, cmax, cmin);
-    if constexpr (SOLVER == SOLVER_HLL) {
-      riemann_hll<T, MHD, NDIR, GLM, NDIM, D, FAST>(wLC, wRC, fL, fR, cmax, cmin, T(P.tvdlfeps), F);
-    } else if constexpr (SOLVER == SOLVER_HLLC) {
-      if constexpr (MHD) riemann_hllc_mhd<T, NDIR, GLM, NDIM, D, FAST>(wLC, wRC, fL, fR, cmax, cmin, T(P.tvdlfeps), F);
-      else riemann_hllc_hd<T, NDIR, D, FAST>(wLC, wRC, fL, fR, cmax, cmin, F);
+  }
+  T cmax, cmin = T(0.0);
+  if constexpr (SOLVER == SOLVER_HLLD) {
+    static_assert(MHD, "HLLD needs MHD");
+    if constexpr (PRIM) {  // the MHD bounds read the primitive states
+      st |= cbounds<T, MHD, NDIR, GLM, D, true, BS, FAST, true>(wLp, wRp, wLp, wRp, P, cmax, cmin);
+      riemann_hlld_prim<T, NDIR, GLM, NDIM, FAST>(wLp, wRp, cmax, cmin, cg, T(P.inv_gamma_1), F);
     } else {
-      static_assert(MHD, "HLLD needs MHD");
-      riemann_hlld<T, NDIR, GLM, NDIM, D, FAST>(wLC, wRC, wLp, wRp, fL, fR, cmax, cmin, F);
+      st |= cbounds<T, MHD, NDIR, GLM, D, true, BS, FAST>(wLC, wRC, wLp, wRp, P, cmax, cmin);
+      riemann_hlld<T, NDIR, GLM, NDIM, FAST>(wLC, wRC, wLp, wRp, cmax, cmin, cg, F);
+    }
+  } else if constexpr (SOLVER == SOLVER_HLLC && !MHD) {
+    st |= cbounds<T, MHD, NDIR, GLM, D, true, BS, FAST>(wLC, wRC, wLp, wRp, P, cmax, cmin);
+    riemann_hllc_hd<T, NDIR, FAST>(wLC, wRC, wLp, wRp, cmax, cmin, F);
+  } else {
+    T fL[NW], fR[NW];
+    phys_flux<T, MHD, NDIR, GLM, D>(wLC, wLp, cg, fL);
+    phys_flux<T, MHD, NDIR, GLM, D>(wRC, wRp, cg, fR);
+    if constexpr (SOLVER == SOLVER_TVDMU) {
+      (void)cmax;
+      if constexpr (MHD) {
+        static_assert(!GLM, "TVD-MUSCL with GLM is not built");
+        riemann_tvdmu_mhd<T, NDIR>(wLC, wRC, fL, fR, P, F);
+      } else {
+        riemann_tvdmu_hd<T, NDIR>(wLC, wRC, fL, fR, P, F);
+      }
+    } else if constexpr (SOLVER == SOLVER_TVDLF) {
+      st |= cbounds<T, MHD, NDIR, GLM, D, false, BS, FAST>(wLC, wRC, wLp, wRp, P, cmax, cmin);
+      riemann_tvdlf<T, NW>(wLC, wRC, fL, fR, cmax, T(P.tvdlfeps), F);
+    } else {
+      st |= cbounds<T, MHD, NDIR, GLM, D, true, BS, FAST>(wLC, wRC, wLp, wRp, P, cmax, cmin);
+      if constexpr (SOLVER == SOLVER_HLL)
+        riemann_hll<T, MHD, NDIR, GLM, NDIM, D, FAST>(wLC, wRC, fL, fR, cmax, cmin, T(P.tvdlfeps), F);
+      else
+        riemann_hllc_mhd<T, NDIR, GLM, NDIM, D, FAST>(wLC, wRC, fL, fR, cmax, cmin, T(P.tvdlfeps), F);
     }
   }
   return st;
@@ -396,6 +412,11 @@ __device__ __forceinline__ double venk_phi(double wm, double w0, double wp, doub
   return fmin(phim, phip);
 }
 
+// Where cada3's short form (face_states with R2) is used: with the limiter
+// fixed to it, in 3-D and in FP32, as hlld_from_primitives (riemann.cuh).
+template <class TF, int NDIM, int LIM>
+constexpr bool cada3_short = LIM == LIM_CADA3 && (NDIM == 3 || sizeof(TF) == 4);
+
 // Halo width of the staged tile: two cells for the slope limiters, three for
 // the fifth-order reconstructions (face stencil i-2 .. i+3).  LIM_WENO5 as a
 // template argument stands for the whole WENO5 family (variant at run time).
@@ -491,7 +512,7 @@ struct FaceFlux64 {
   uint32_t st;
 };
 
-template <class TF, bool MHD, int NDIR, bool GLM, int NDIM, int SOLVER, int LIM, int BS, int VS>
+template <class TF, bool MHD, int NDIR, bool GLM, int NDIM, int SOLVER, int LIM, int BS, int VS, bool FAST>
 __device__ __noinline__ FaceFlux64<Vars<MHD, NDIR, GLM>::NW> face_retry_fp64(const TF *smem, int D, int b0, int b1,
                                                                             int b2, int b3, double rd, double cg,
                                                                             const PhysParams P) {
@@ -505,14 +526,12 @@ __device__ __noinline__ FaceFlux64<Vars<MHD, NDIR, GLM>::NW> face_retry_fp64(con
     double q[4];
 #pragma unroll
     for (int o = 0; o < 4; ++o) q[o] = double(smem[base[o] + ov * VS]);
-    const double d0 = q[1] - q[0], d1 = q[2] - q[1], d2 = q[3] - q[2];
-    double ldw, rdw;
-    face_slopes<double, LIM>(P.limiter, d0, d1, d2, rd, ldw, rdw);
-    wLp[v] = q[1] + 0.5 * ldw;
-    wRp[v] = q[2] - 0.5 * rdw;
+    bool special = false;
+    face_states<double, LIM, FAST, cada3_short<TF, NDIM, LIM>>(P.limiter, q[0], q[1], q[2], q[3], rd, wLp[v], wRp[v],
+                                                                special);
   }
   FaceFlux64<NW> r;
-  r.st = face_from_states<double, MHD, NDIR, GLM, NDIM, SOLVER, BS>(wLp, wRp, P, cg, r.F);
+  r.st = face_from_states<double, MHD, NDIR, GLM, NDIM, SOLVER, BS, FAST>(wLp, wRp, P, cg, r.F);
   return r;
 }
 
@@ -537,11 +556,9 @@ __device__ __noinline__ FaceFlux64<Vars<MHD, NDIR, GLM>::NW> face_retry_state(co
 #pragma unroll
   for (int v = 0; v < NW; ++v) {
     const int ov = orig_index_rt<MHD, NDIR>(v, D);
-    const double d0 = q[1][ov] - q[0][ov], d1 = q[2][ov] - q[1][ov], d2 = q[3][ov] - q[2][ov];
-    double ldw, rdw;
-    face_slopes<double, LIM>(A->P.limiter, d0, d1, d2, rd, ldw, rdw);
-    wLp[v] = q[1][ov] + 0.5 * ldw;
-    wRp[v] = q[2][ov] - 0.5 * rdw;
+    bool special = false;
+    face_states<double, LIM, false, cada3_short<float, NDIM, LIM>>(A->P.limiter, q[0][ov], q[1][ov], q[2][ov], q[3][ov], rd,
+                                                                   wLp[v], wRp[v], special);
   }
   FaceFlux64<NW> r;
   r.st = face_from_states<double, MHD, NDIR, GLM, NDIM, SOLVER, BS>(wLp, wRp, A->P, cg, r.F);
@@ -738,8 +755,6 @@ __global__ void __launch_bounds__(StageOcc<TF, LIM, BN, VAR>::THREADS, StageOcc<
   const int ci = t % TB, cj = t / TB;  // cell role (tile-relative) for t < TB*TB
   const bool cell_thread = t < TB * TB;
   const bool need_corners = MHD && !GLM && P.divb == DIVB_LINDE;
-  __shared__ int s_retry;  // some face of this phase needs the guarded FP64 recomputation
-  if (t == 0) s_retry = 0;
   // Asynchronous staging (variant; 3-D FP64, whole-plane tiles, slope
   // limiters): the conserved plane k+2 that iteration k stages is a
   // contiguous row of TB*TB doubles per variable, in this block or its
@@ -774,11 +789,11 @@ __global__ void __launch_bounds__(StageOcc<TF, LIM, BN, VAR>::THREADS, StageOcc<
     dx[d] = d < NDIM ? A.dxb[b * 3 + d] : 1.0;
     dxinv[d] = -qdt / dx[d];
     const double r = P.cada3_radius * dx[d];
-    // cada3: 1 / (cada3_radius dx)^2; schmid: (a2max + cadepsilon) dx^2 with
+    // cada3: 1 / (cada3_radius dx)^2, or its inverse for the short form; schmid: (a2max + cadepsilon) dx^2 with
     // a2max = schmid_rad (schmid2) or a2max_global of this step (schmid1)
     const double a2m = P.schmid_global ? A.dt_dev[10 + d] : P.schmid_rad[d];
     rdel[d] = (LIM == LIM_SCHMID || (LIM == 0 && P.limiter == LIM_SCHMID))
-                  ? (a2m + 1.0e-14) * (dx[d] * dx[d]) : 1.0 / (r * r);
+                  ? (a2m + 1.0e-14) * (dx[d] * dx[d]) : (cada3_short<TF, NDIM, LIM> ? r * r : 1.0 / (r * r));
     if constexpr (LIM == LIM_WENO5) wlam[d] = pow(dx[d], 2.0 / 3.0);
   }
   double fz_prev[NDIM == 3 ? NW : 1];
@@ -885,6 +900,7 @@ __global__ void __launch_bounds__(StageOcc<TF, LIM, BN, VAR>::THREADS, StageOcc<
       // ---- Hancock predictor: each cell thread, all directions, from the
       // staged primitives (cells c-1, c, c+1; z from ring slots k-1..k+1)
       static_assert(sizeof(TF) == 8, "the Hancock predictor is FP64 only");
+      static_assert(!cada3_short<TF, NDIM, LIM>, "limited_slope takes the inverse of the short form's rdel");
       if (update && cell_thread) {
         int base[3];
         if (dsel < 0 || dsel == 0) {
@@ -975,12 +991,14 @@ __global__ void __launch_bounds__(StageOcc<TF, LIM, BN, VAR>::THREADS, StageOcc<
             pf[orig_index_rt<MHD, NDIR>(v, FD) * (BN * BN) + ta + BN * (NDIM == 3 ? tb : 0)] = sc * double(Fr[v]);
         }
       };
+      bool retry = false;  // some face of this thread needs the recomputation
 #pragma unroll 1
       for (int f = t; f < nface; f += THREADS) {
         int fi, fj, FD, fl;
         face_dir(f, FD, fl);
         const TF rd = TF(FD == 0 ? rdel[0] : (FD == 1 ? rdel[1] : rdel[2]));
         TF wLp[NW], wRp[NW];
+        bool special = false;  // near a limiter's blending band: left to the recomputation
         int base[H2], rot[NDIR];
         face_at(FD, fl, fi, fj, base);
         rot_of(FD, rot);
@@ -1072,11 +1090,8 @@ __global__ void __launch_bounds__(StageOcc<TF, LIM, BN, VAR>::THREADS, StageOcc<
             TF q[4];
 #pragma unroll
             for (int o = 0; o < 4; ++o) q[o] = smem[base[o] + var_off(v, rot)];
-            const TF d0 = q[1] - q[0], d1 = q[2] - q[1], d2 = q[3] - q[2];
-            TF ldw, rdw;
-            face_slopes<TF, LIM, FASTF>(P.limiter, d0, d1, d2, rd, ldw, rdw);
-            wLp[v] = q[1] + TF(0.5) * ldw;
-            wRp[v] = q[2] - TF(0.5) * rdw;
+            face_states<TF, LIM, FASTF, cada3_short<TF, NDIM, LIM>, !FASTF>(P.limiter, q[0], q[1], q[2], q[3], rd, wLp[v], wRp[v],
+                                                                    special);
           }
         }
         // mixed form with fix_small_values: a state near a floor goes to the
@@ -1104,9 +1119,9 @@ __global__ void __launch_bounds__(StageOcc<TF, LIM, BN, VAR>::THREADS, StageOcc<
           TF fsum = Fr[0];
 #pragma unroll
           for (int v = 1; v < NW; ++v) fsum = fsum + Fr[v];
-          const bool finite = !near && isfinite(fsum);
+          const bool finite = !near && !special && isfinite(fsum);
           if (!finite) {
-            s_retry = 1;
+            retry = true;
             Fr[0] = TF(NAN);
           }
         }
@@ -1120,12 +1135,13 @@ __global__ void __launch_bounds__(StageOcc<TF, LIM, BN, VAR>::THREADS, StageOcc<
         }
         if (amr_mask) capture(FD, fi, fj, Fr, sc);
       }
-      __syncthreads();
       if constexpr (RETRY) {
-        // fix-up pass: the faces whose flux is not finite (an FP32 face of the
-        // mixed form, or an FP64 face that met a special operand in the
-        // unguarded arithmetic), recomputed in FP64 with the guarded forms
-        if (s_retry) {
+        // fix-up pass: the thread's own faces whose flux is not finite or
+        // whose limiter is near its blending band (an FP32 face of the mixed
+        // form, or an FP64 face that met a special operand in the unguarded
+        // arithmetic), recomputed in FP64: in the fast arithmetic with the
+        // blend first, then with the guarded forms
+        if (retry) {
           for (int f = t; f < nface; f += THREADS) {
             int FD, fl;
             face_dir(f, FD, fl);
@@ -1137,10 +1153,18 @@ __global__ void __launch_bounds__(StageOcc<TF, LIM, BN, VAR>::THREADS, StageOcc<
             face_at(FD, fl, fi, fj, base);
             const double rdd = FD == 0 ? rdel[0] : (FD == 1 ? rdel[1] : rdel[2]);
             FaceFlux64<NW> r;
-            if constexpr (FP64)
-              r = face_retry_fp64<TF, MHD, NDIR, GLM, NDIM, SOLVER, LIM, BS, VS>(smem, FD, base[0], base[1], base[2],
-                                                                                 base[3], rdd, cg, P);
-            else  // the R cell of the face, block-local
+            if constexpr (FP64) {
+              bool done = false;
+              if constexpr (LIM == LIM_CADA3) {
+                r = face_retry_fp64<TF, MHD, NDIR, GLM, NDIM, SOLVER, LIM, BS, VS, true>(smem, FD, base[0], base[1],
+                                                                                         base[2], base[3], rdd, cg, P);
+                done = true;
+                for (int v = 0; v < NW; ++v) done = done && isfinite(r.F[v]);
+              }
+              if (!done)
+                r = face_retry_fp64<TF, MHD, NDIR, GLM, NDIM, SOLVER, LIM, BS, VS, false>(smem, FD, base[0], base[1],
+                                                                                          base[2], base[3], rdd, cg, P);
+            } else  // the R cell of the face, block-local
               r = face_retry_state<MHD, NDIR, GLM, NDIM, SOLVER, LIM, BS, BN>(
                   &A, b, FD, ti0 + fi, tj0 + fj, FD == 2 ? k + 1 : k, rdd, cg);
             stb |= r.st;
@@ -1152,10 +1176,10 @@ __global__ void __launch_bounds__(StageOcc<TF, LIM, BN, VAR>::THREADS, StageOcc<
             }
             if (amr_mask) capture(FD, fi, fj, Fr, sc);
           }
-          __syncthreads();
-          if (t == 0) s_retry = 0;
         }
       }
+      // a z-face's flux is read by the thread that wrote it
+      if (NDIM < 3 || D < 2) __syncthreads();
       if (cell_thread) {
         const double sc = FP64 ? 1.0 : (D == 0 ? dxinv[0] : (D == 1 ? dxinv[1] : dxinv[2]));
         // the fluxes are stored rotated: entry v is variable orig_index<D>(v)

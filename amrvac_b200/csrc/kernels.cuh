@@ -318,7 +318,7 @@ struct KernelSet {
 template <bool MHD, int NDIR, bool GLM, int NDIM, int SOLVER, int LIM, int BS, class TF, int BN, int VAR>
 struct StageVar {
   using V = Vars<MHD, NDIR, GLM>;
-  using O = StageOcc<TF, LIM, BN, VAR>;
+  using O = StageOcc<TF, MHD, NDIM, LIM, BN, VAR>;
   static constexpr size_t SMEM = Tile<TF, V::NW, NDIM, HaloW<LIM>::value, tile_edge(BN)>::BYTES;
   static cudaError_t prepare() {
     return cudaFuncSetAttribute(fv_stage_kernel<TF, MHD, NDIR, GLM, NDIM, SOLVER, LIM, BS, BN, VAR>,
@@ -350,13 +350,27 @@ template <bool MHD, int NDIR, bool GLM, int NDIM, int SOLVER, int LIM = 0, int B
           int BN = BN16>
 struct Launch {
   using V = Vars<MHD, NDIR, GLM>;
-  static constexpr int THREADS = StageOcc<TF, LIM, BN>::THREADS;
+  static constexpr int THREADS = StageOcc<TF, MHD, NDIM, LIM, BN>::THREADS;
   static constexpr size_t SMEM = Tile<TF, V::NW, NDIM, HaloW<LIM>::value, tile_edge(BN)>::BYTES;
   // typepred1 = fs_hancock for tvdlf and tvdmu (src/io/mod_input_output.t:787-797)
+  // The 2-D hydrodynamics tile is small (30 KB) and its kernel waits for its
+  // block's loads and barriers: four CTAs per SM (64 registers) instead of two
+  // hide them, 2048^2 HLLC + vanleer FP64 0.37 -> 0.31 ms per stage.  A grid
+  // that the two-CTA kernel holds in one wave has no second CTA to hide
+  // behind, and runs the kernel without spills (64^2: 28 against 26 us a step).
+  static constexpr bool HAS_DENSE = !MHD && NDIM == 2 && sizeof(TF) == 8 && HaloW<LIM>::value == 2;
+  static constexpr int VMAIN = HAS_DENSE ? VAR_DENSE : 0;
+  static constexpr int SMALL_TILES = 2 * 148;
+  static constexpr int NTILE = (BN / tile_edge(BN)) * (BN / tile_edge(BN));
   static constexpr bool HAS_HANCOCK = (SOLVER == SOLVER_TVDLF || SOLVER == SOLVER_TVDMU) && sizeof(TF) == 8;
   static cudaError_t prepare() {
     cudaError_t e = cudaFuncSetAttribute(fv_stage_kernel<TF, MHD, NDIR, GLM, NDIM, SOLVER, LIM, BS, BN>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM);
+    if constexpr (HAS_DENSE) {
+      if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(fv_stage_kernel<TF, MHD, NDIR, GLM, NDIM, SOLVER, LIM, BS, BN, VAR_DENSE>,
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM);
+    }
     if constexpr (HAS_HANCOCK) {
       if (e == cudaSuccess)
         e = cudaFuncSetAttribute(fv_stage_kernel<TF, MHD, NDIR, GLM, NDIM, SOLVER_HANCOCK, LIM, BS, BN>,
@@ -365,6 +379,12 @@ struct Launch {
     return e;
   }
   static cudaError_t stage(const StageArgs &A, int nctas, cudaStream_t s) {
+    if constexpr (HAS_DENSE) {
+      if (A.nblocks * NTILE > SMALL_TILES) {
+        fv_stage_kernel<TF, MHD, NDIR, GLM, NDIM, SOLVER, LIM, BS, BN, VAR_DENSE><<<nctas, THREADS, SMEM, s>>>(A);
+        return cudaGetLastError();
+      }
+    }
     fv_stage_kernel<TF, MHD, NDIR, GLM, NDIM, SOLVER, LIM, BS, BN><<<nctas, THREADS, SMEM, s>>>(A);
     return cudaGetLastError();
   }
@@ -382,6 +402,8 @@ struct Launch {
   }
   static cudaError_t hancock(const StageArgs &A, int nctas, cudaStream_t s) {
     if constexpr (HAS_HANCOCK) {
+      // nctas is one wave of the main kernel, which is denser than this one
+      if (HAS_DENSE && A.zchunk == 0 && nctas > SMALL_TILES) nctas = SMALL_TILES;
       fv_stage_kernel<TF, MHD, NDIR, GLM, NDIM, SOLVER_HANCOCK, LIM, BS, BN><<<nctas, THREADS, SMEM, s>>>(A);
       return cudaGetLastError();
     } else {
@@ -391,7 +413,7 @@ struct Launch {
   static int ctas_per_sm() {
     int n = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-            &n, fv_stage_kernel<TF, MHD, NDIR, GLM, NDIM, SOLVER, LIM, BS, BN>, THREADS, SMEM) != cudaSuccess)
+            &n, fv_stage_kernel<TF, MHD, NDIR, GLM, NDIM, SOLVER, LIM, BS, BN, VMAIN>, THREADS, SMEM) != cudaSuccess)
       return 1;
     return n > 0 ? n : 1;
   }
@@ -447,6 +469,8 @@ struct Launch {
     k.stage_smem = SMEM;
     k.bn = BN;
     StageVar<MHD, NDIR, GLM, NDIM, SOLVER, LIM, BS, TF, BN, 0>::add(k, 0);
+    k.stage_v[0] = &stage;
+    k.ctas_v[0] = &ctas_per_sm;
     return k;
   }
 };

@@ -580,7 +580,9 @@ __device__ __forceinline__ void riemann_hlld_prim(const T *wLp, const T *wRp, T 
     if (FAST) return f + c1 * d1 + c2 * d2;
     return two ? f + c1 * d1 + c2 * d2 : (star ? f + c1 * d1 : f);
   };
-  auto put1 = [&](T f, T d1) -> T { return FAST || star ? f + c1 * d1 : f; };
+  // where w2 = w1; the product with zero carries an invalid Alfven speed into
+  // every variable, as the reference's does (with FAST the others do)
+  auto put1 = [&](T f, T d1) -> T { return FAST ? f + c1 * d1 : put(f, d1, T(0.0)); };
   const T m = rho * vn;
   T b2 = Bn * Bn, v2 = vn * vn, vb = vn * Bn, v1b = sm * Bx, v2b = sm * Bx;
 #pragma unroll

@@ -425,6 +425,12 @@ struct HaloW {
   static constexpr int value = (LIM == LIM_MP5 || LIM == LIM_WENO5) ? 3 : 2;
 };
 
+// The tiles that hold the faces of both directions of a 2-D plane at once:
+// hydrodynamics (nw 4: 30 KB).  Nine MHD variables would take 68 KB, and the
+// longer face phase measured no gain there (432x304 HLLD + cada3 994 -> 1006 us,
+// vanleer 1170 -> 1126).
+__host__ __device__ constexpr bool merged_faces(int nw, int ndim) { return ndim == 2 && nw <= 4; }
+
 // Shared-memory tile of BN x BN cells (sizes in elements), halo width HW.
 // Every variable holds its ring planes and its halo strips of plane k in one
 // block of VS elements, so the distance between two variables is the same
@@ -444,7 +450,8 @@ struct Tile {
   static constexpr int OC = OY + H2 * BN;                // corners [r][c]
   static constexpr int VS = OC + H2 * H2;                // one variable
   static constexpr int FB = (BN + 1) * BN;               // scaled face fluxes of a variable
-  static constexpr int YX = BN;                          // y-faces of the top row (j = BN)
+  // second flux buffer: the y-faces of the top row (j = BN), or all y-faces
+  static constexpr int YX = merged_faces(NW, NDIM) ? FB : BN;
   static constexpr int TOTAL = NW * (VS + FB + YX);
   static constexpr size_t BYTES = sizeof(TF) * TOTAL;
 };
@@ -636,6 +643,8 @@ __device__ __forceinline__ uint32_t hancock_dir(const double *smem, const int *b
 // benchmark schemes: threads per CTA, the CTAs per SM the registers are
 // capped for, and the staging mode (asynchronous bulk copies of the next
 // conserved plane, FP64 only).  stage_variant(VAR, fp64) gives them.
+// VAR_DENSE: the FP64 2-D hydrodynamics kernel at twice the CTAs per SM.
+constexpr int VAR_DENSE = 8;
 struct StageVariant {
   int threads, minb;
   bool async;
@@ -647,15 +656,26 @@ __host__ __device__ constexpr StageVariant stage_variant(int var, bool fp64) {
   }
   return var == 1 ? StageVariant{256, 2, false} : var == 2 ? StageVariant{256, 4, false} : StageVariant{288, 3, false};
 }
-template <class TF, int LIM, int BN, int VAR = 0>
+// CTAs per SM of 256 threads: two in FP64 MHD (104.8 KB of shared memory in
+// 3-D, and registers), three in mixed MHD; 3-D hydrodynamics has room for
+// three (58 KB; 80 registers, a few spilled: 96x80x112 HLLC FP64 0.155 ->
+// 0.143 ms per stage), mixed 2-D hydrodynamics for four (64 registers, 2048^2
+// 0.255 -> 0.228).  2.5-D MHD at three spills too much (432x304 0.033 -> 0.053).
+__host__ __device__ constexpr int stage_base(bool fp64, bool mhd, int ndim, int hw) {
+  if (hw == 3) return 1;
+  if (mhd) return fp64 ? AMRVAC_STAGE_MINB : AMRVAC_STAGE_MINB_MIXED;
+  if (ndim == 3) return 3;
+  return fp64 ? AMRVAC_STAGE_MINB : 4;
+}
+template <class TF, bool MHD, int NDIM, int LIM, int BN, int VAR = 0>
 struct StageOcc {
   static constexpr bool FP64 = sizeof(TF) == 8;
   static constexpr int THREADS =
-      VAR > 0 ? stage_variant(VAR, FP64).threads : (BN == BN16 ? STAGE_THREADS : stage_threads(BN));
-  static constexpr int BASE = FP64 ? (HaloW<LIM>::value == 3 ? 1 : AMRVAC_STAGE_MINB) : AMRVAC_STAGE_MINB_MIXED;
+      VAR > 0 && VAR != VAR_DENSE ? stage_variant(VAR, FP64).threads : (BN == BN16 ? STAGE_THREADS : stage_threads(BN));
+  static constexpr int BASE = stage_base(FP64, MHD, NDIM, HaloW<LIM>::value);
   static constexpr int MINB0 = BASE * 256 / THREADS < 1 ? 1 : (BASE * 256 / THREADS > 16 ? 16 : BASE * 256 / THREADS);
-  static constexpr int MINB = VAR > 0 ? stage_variant(VAR, FP64).minb : MINB0;
-  static constexpr bool ASYNC = VAR > 0 && stage_variant(VAR, FP64).async;
+  static constexpr int MINB = VAR == VAR_DENSE ? 2 * MINB0 : (VAR > 0 ? stage_variant(VAR, FP64).minb : MINB0);
+  static constexpr bool ASYNC = VAR > 0 && VAR != VAR_DENSE && stage_variant(VAR, FP64).async;
 };
 
 // Asynchronous plane staging: one thread copies a block's conserved plane
@@ -701,7 +721,7 @@ __device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t parity, int sp
 }
 
 template <class TF, bool MHD, int NDIR, bool GLM, int NDIM, int SOLVER, int LIM, int BS, int BN = BN16, int VAR = 0>
-__global__ void __launch_bounds__(StageOcc<TF, LIM, BN, VAR>::THREADS, StageOcc<TF, LIM, BN, VAR>::MINB)
+__global__ void __launch_bounds__(StageOcc<TF, MHD, NDIM, LIM, BN, VAR>::THREADS, StageOcc<TF, MHD, NDIM, LIM, BN, VAR>::MINB)
     fv_stage_kernel(const __grid_constant__ StageArgs A) {
   using V = Vars<MHD, NDIR, GLM>;
   constexpr int NW = V::NW;
@@ -710,7 +730,7 @@ __global__ void __launch_bounds__(StageOcc<TF, LIM, BN, VAR>::THREADS, StageOcc<
   constexpr int TB = tile_edge(BN);
   constexpr int NTX = BN / TB;                       // tiles per plane row
   constexpr int NT = NDIM >= 2 ? NTX * NTX : NTX;    // tiles per plane
-  constexpr int THREADS = StageOcc<TF, LIM, BN, VAR>::THREADS;
+  constexpr int THREADS = StageOcc<TF, MHD, NDIM, LIM, BN, VAR>::THREADS;
   constexpr int FB = (TB + 1) * TB;  // face-buffer stride per variable
   constexpr bool FP64 = sizeof(TF) == 8;
   constexpr int HW = HaloW<LIM>::value;  // halo width: 2, or 3 for MP5
@@ -763,7 +783,7 @@ __global__ void __launch_bounds__(StageOcc<TF, LIM, BN, VAR>::THREADS, StageOcc<
   // just before the z phase, the first phase that reads it, so the copy runs
   // behind the x and y phases.  Planes behind a physical boundary or a level
   // jump take the gather (load_prim).
-  constexpr bool ASYNC = StageOcc<TF, LIM, BN, VAR>::ASYNC && FP64 && NDIM == 3 && NT == 1 && HW == 2 &&
+  constexpr bool ASYNC = StageOcc<TF, MHD, NDIM, LIM, BN, VAR>::ASYNC && FP64 && NDIM == 3 && NT == 1 && HW == 2 &&
                          SOLVER != SOLVER_HANCOCK;
   __shared__ __align__(8) unsigned long long s_mbar;
   uint32_t mphase = 0;
@@ -927,25 +947,36 @@ __global__ void __launch_bounds__(StageOcc<TF, LIM, BN, VAR>::THREADS, StageOcc<
     // and the y phase one round of 256 (instead of two rounds of 256 + 16).
     // (With 272 or more threads a phase of 272 faces is one round already;
     // a split sweep has one phase only.)
-    const bool merge_yx = THREADS < FB && dsel < 0;
+    // 2-D hydrodynamics (merged_faces): one phase, the x-faces into tv.fb and
+    // the y-faces into tv.yx, so a block takes one barrier between its faces
+    // and their sums instead of three.
+    constexpr bool MERGED = merged_faces(NW, NDIM);
+    const bool merge_yx = !MERGED && THREADS < FB && dsel < 0;
     const int dlo = update ? 0 : (NDIM == 3 && k == k0 - 1 ? 2 : NDIM);
+    constexpr int NPHASE = MERGED ? 1 : NDIM;
 #pragma unroll 1
-    for (int D = dlo; D < NDIM; ++D) {
+    for (int D = dlo; D < NPHASE; ++D) {
       if (pend && D == 2) {  // the z phase reads plane k+2 (k+HW)
         finish_async();
         __syncthreads();
       }
-      if (dsel >= 0 && D != dsel) continue;  // not this sweep's direction (uniform)
-      const int nface = D == 0 ? (merge_yx ? FB + TB : FB) : (D == 1 && !merge_yx ? FB : TB * TB);
+      if (!MERGED && dsel >= 0 && D != dsel) continue;  // not this sweep's direction (uniform)
+      const int nface = MERGED ? (dsel < 0 ? 2 * FB : FB)
+                               : (D == 0 ? (merge_yx ? FB + TB : FB) : (D == 1 && !merge_yx ? FB : TB * TB));
       // direction FD and index fl (in that direction's face layout) of face f
       // of this phase
       auto face_dir = [&](int f, int &FD, int &fl) {
-        if (merge_yx && D == 0 && f >= FB) { FD = 1; fl = TB * TB + (f - FB); }
+        if constexpr (MERGED) {
+          const bool y = dsel < 0 ? f >= FB : dsel == 1;
+          FD = y ? 1 : 0;
+          fl = dsel < 0 && y ? f - FB : f;
+        } else if (merge_yx && D == 0 && f >= FB) { FD = 1; fl = TB * TB + (f - FB); }
         else { FD = D; fl = f; }
       };
       // where the flux of (rotated) variable v of face f lives
       auto flux_ref = [&](int f, int FD, int fl, int v) -> TF & {
-        return FD == D ? tv.fb[v * FB + f] : tv.yx[v * TB + (fl - TB * TB)];
+        if constexpr (MERGED) return tv.fb[(FD == 0 ? 0 : NW * FB) + v * FB + fl];
+        else return FD == D ? tv.fb[v * FB + f] : tv.yx[v * TB + (fl - TB * TB)];
       };
       // face coordinates and the shared-memory offsets of the 2 HW stencil
       // cells (variable 0): inside the plane a step of 1 (x) or TB (y), in the
@@ -1181,9 +1212,9 @@ __global__ void __launch_bounds__(StageOcc<TF, LIM, BN, VAR>::THREADS, StageOcc<
       // a z-face's flux is read by the thread that wrote it
       if (NDIM < 3 || D < 2) __syncthreads();
       if (cell_thread) {
-        const double sc = FP64 ? 1.0 : (D == 0 ? dxinv[0] : (D == 1 ? dxinv[1] : dxinv[2]));
         // the fluxes are stored rotated: entry v is variable orig_index<D>(v)
-        if (D == 0) {
+        if (MERGED ? dsel != 1 : D == 0) {
+          const double sc = FP64 ? 1.0 : dxinv[0];
           const int f = cj * (TB + 1) + ci;
 #pragma unroll
           for (int v = 0; v < NW; ++v) {
@@ -1191,17 +1222,22 @@ __global__ void __launch_bounds__(StageOcc<TF, LIM, BN, VAR>::THREADS, StageOcc<
             if constexpr (FP64) a = a + tv.fb[v * FB + f + 1] - tv.fb[v * FB + f];
             else a = a + sc * double(tv.fb[v * FB + f + 1]) - sc * double(tv.fb[v * FB + f]);
           }
-        } else if (D == 1) {
+        }
+        if (MERGED ? dsel != 0 : D == 1) {
+          const double sc = FP64 ? 1.0 : dxinv[1];
           const int f = cj * TB + ci;
+          const TF *fy = MERGED ? tv.yx : tv.fb;
 #pragma unroll
           for (int v = 0; v < NW; ++v) {
             double &a = acc[orig_index<MHD, NDIR, 1>(v)];
-            // the face above the top row was computed in the x phase
-            const TF up = (merge_yx && cj == TB - 1) ? tv.yx[v * TB + ci] : tv.fb[v * FB + f + TB];
-            if constexpr (FP64) a = a + up - tv.fb[v * FB + f];
-            else a = a + sc * double(up) - sc * double(tv.fb[v * FB + f]);
+            // not merged: the face above the top row was computed in the x phase
+            const TF up = (merge_yx && cj == TB - 1) ? tv.yx[v * TB + ci] : fy[v * FB + f + TB];
+            if constexpr (FP64) a = a + up - fy[v * FB + f];
+            else a = a + sc * double(up) - sc * double(fy[v * FB + f]);
           }
-        } else if constexpr (NDIM == 3) {
+        }
+        if constexpr (NDIM == 3) if (D == 2) {
+          const double sc = FP64 ? 1.0 : dxinv[2];
 #pragma unroll
           for (int v = 0; v < NW; ++v) {
             double &a = acc[orig_index<MHD, NDIR, 2>(v)];
@@ -1216,7 +1252,7 @@ __global__ void __launch_bounds__(StageOcc<TF, LIM, BN, VAR>::THREADS, StageOcc<
       // the next phase overwrites the face buffer; after the last phase the
       // barrier at the end of the plane orders the reads against the next
       // plane's writes
-      if (D < NDIM - 1) __syncthreads();
+      if (D < NPHASE - 1) __syncthreads();
     }
     // no z phase this iteration: the plane is needed by the next one (the
     // barrier at the end of the iteration orders it)

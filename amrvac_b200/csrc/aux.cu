@@ -3,7 +3,7 @@
 #include <cuda_runtime.h>
 
 #include "aux.cuh"
-#include "stage.cuh"
+#include "kernels.cuh"
 
 namespace amrvac {
 
@@ -107,36 +107,8 @@ __global__ void pack_kernel(const double *__restrict__ pool, double *__restrict_
 }
 
 // ---------------------------------------------------------------- setdt tail
-// After getdt_kernel: dt = courantpar / max (src/mod_dt.t:233-235), the
-// dtmin check (55-60), the slowsteps ramp (64-67), final_dt_reduction (69-79)
-// and the output-interval cap (88-99).  scal: [0]=dt [1]=cmax_global
-// [2]=global_time [3]=time_max [4]=dtsave [5]=dtmin [6]=courantpar
-// [7]=final_exit flag [8]=slowsteps [9]=steps since set_time (it - it_init).
 __global__ void setdt_finalize_kernel(unsigned long long *red, double *scal, uint32_t *status) {
-  const double smalldouble = 1.0e-12, bigdouble = 1.0e99;
-  const double x = __longlong_as_double((long long)red[0]);
-  const double cm = __longlong_as_double((long long)red[1]);
-  red[0] = 0ull;
-  red[1] = 0ull;
-  double dt = bigdouble;
-  if (x > smalldouble) dt = fmin(dt, scal[6] / x);
-  if (dt < scal[5]) atomicOr(status, ST_DT_TOO_SMALL);
-  if (scal[8] > scal[9] + 1.0) {
-    const double q = 1.0 - (scal[9] + 1.0) / scal[8];
-    dt = dt * (1.0 - q * q);
-  }
-  const double t = scal[2], tmax = scal[3], dtsave = scal[4];
-  if (tmax - t <= scal[5]) scal[7] = 1.0;
-  dt = fmin(dt, tmax - t);
-  if (dtsave > 0.0) {
-    double dtmax = ceil(t / dtsave) * dtsave;
-    const double other = t > 0.0 ? ceil(t / bigdouble) * bigdouble : 0.0;
-    dtmax = fmin(dtmax, other) - t;
-    if (dtmax > smalldouble) dt = fmin(dt, dtmax);
-    else dt = fmin(dt, dtsave);
-  }
-  scal[0] = dt;
-  scal[1] = cm;
+  setdt_finalize(red, scal, status);
 }
 
 __global__ void advance_time_kernel(double *scal) {

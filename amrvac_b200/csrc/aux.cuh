@@ -30,6 +30,7 @@ cudaError_t launch_unpack(const double *src, double *pool, int first, int n, int
                           cudaStream_t s);
 cudaError_t launch_pack(const double *pool, double *dst, int first, int n, int nw, int ndim, int ng, int bn,
                         const int *nbr, const SrlMaps &maps, const BcSpec &bc, const double *gbuf, cudaStream_t s);
+// setdt after the CFL reduction (setdt_finalize in kernels.cuh), as a kernel.
 cudaError_t launch_setdt_finalize(unsigned long long *red, double *scal, uint32_t *status, cudaStream_t s);
 cudaError_t launch_advance_time(double *scal, cudaStream_t s);
 cudaError_t launch_ssprk5_ps3(double *u3, const double *u2, const double *u1, double a53, double a54, size_t n,

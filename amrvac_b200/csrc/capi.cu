@@ -76,7 +76,7 @@ struct amrvac_ctx {
   int *d_nbr = nullptr;
   double *d_dx = nullptr;
   double *d_scal = nullptr;              // see setdt_finalize_kernel
-  unsigned long long *d_red = nullptr;   // getdt reduction accumulators
+  unsigned long long *d_red = nullptr;   // getdt reduction accumulators, then the getdt kernel's CTA ticket
   uint32_t *d_status = nullptr;
   uint32_t *d_block_status = nullptr;
   double *d_stage = nullptr;             // upload/download staging
@@ -84,6 +84,11 @@ struct amrvac_ctx {
   cudaGraphExec_t graph = nullptr;
   int64_t launches = 0;
   int64_t graph_nodes = 0;
+  // Dependent launches within one step (ChainScope): chained says that the
+  // last thing put on the stream is a kernel that begins with pdl_wait and
+  // pdl_trigger (stage, getdt), so the next one of them may be launched
+  // dependent on it.  Whatever else goes on the stream clears it.
+  bool chain_on = false, chained = false;
   int zchunk = 0;          // 0: persistent plane ranges; 16/8/4: one z-chunk per CTA
   int sweep = -1;          // dimensional splitting: the current sweep of the step (-1: unsplit)
   bool fixed_dir = false;  // sweep is a direction (amrvac_gpu_advect1_dim), not a sweep index
@@ -163,6 +168,12 @@ int check_ctx(amrvac_ctx *c, bool need_blocks) {
   return 0;
 }
 
+struct ChainScope {
+  amrvac_ctx *c;
+  explicit ChainScope(amrvac_ctx *ctx) : c(ctx) { c->chain_on = true; c->chained = false; }
+  ~ChainScope() { c->chain_on = c->chained = false; }
+};
+
 StageArgs stage_args(amrvac_ctx *c, int reg_ct, int reg_new, int reg_base, double a, double b,
                      double dtfactor) {
   StageArgs A;
@@ -204,6 +215,7 @@ int launch_amr_ghost_pass(amrvac_ctx *c, int reg) {
   AmrGhostArgs G = c->amr->G;
   G.u = c->pool[reg];
   CK(launch_amr_ghosts(G, c->amr->nslots, c->cfg.ndim, c->stream));
+  c->chained = false;
   ++c->launches;
   return 0;
 }
@@ -225,7 +237,10 @@ int launch_stage(amrvac_ctx *c, int reg_ct, int reg_new, int reg_base, double a,
   if (c->zchunk > 0) nctas = c->nblocks * ntile * (c->cfg.ndim == 3 ? bn / c->zchunk : 1);
   else nctas = (int)std::min<long>(planes, hancock ? c->wave_ctas : c->wave_v[c->var]);
   const bool restore = !hancock && c->P.fix_small_values && c->P.small_values_method == 0;
-  if (restore || c->sv_on) CK(cudaMemsetAsync(c->d_block_status, 0, sizeof(uint32_t) * c->nblocks, c->stream));
+  if (restore || c->sv_on) {
+    CK(cudaMemsetAsync(c->d_block_status, 0, sizeof(uint32_t) * c->nblocks, c->stream));
+    c->chained = false;
+  }
   // 'average': a register the stage overwrites in place is copied first (the
   // whole-block path reads its neighbours' values from before the stage)
   const double *snap_base = nullptr, *snap_in = nullptr;
@@ -241,8 +256,12 @@ int launch_stage(amrvac_ctx *c, int reg_ct, int reg_new, int reg_base, double a,
     CK(c->sv.detect(A, c->pool[reg_ct], c->stream));
     ++c->launches;
   }
+  A.dependent = c->chained;
   CK(hancock ? c->ks.hancock(A, nctas, c->stream) : c->ks.stage_v[c->var](A, nctas, c->stream));
   ++c->launches;
+  // (what this stage itself still launches behind its kernel breaks the chain)
+  c->chained = c->chain_on && !c->sv_on && !restore && !c->amr &&
+               !(c->cfg.ndim == 3 && c->cfg.physics == 1 && c->cfg.typedivbfix == AMRVAC_DIVB_LINDE);
   if (c->sv_on) {
     CK(c->sv.stage(A, snap_base, snap_in, SvScratch{c->sv_scratch, c->sv_per_cta}, c->sv_ctas, c->stream));
     ++c->launches;
@@ -273,8 +292,14 @@ int launch_stage(amrvac_ctx *c, int reg_ct, int reg_new, int reg_base, double a,
 // z-chunks of zchunk planes, zchunk >= 2 dividing the block edge.
 static bool valid_zchunk(int bn, int zchunk) { return zchunk == 0 || (zchunk >= 2 && bn % zchunk == 0); }
 
-int launch_getdt(amrvac_ctx *c, int reg) {
+// tail: 0 the reduction alone, 1 with setdt (dt, cmax_global) in the same
+// kernel, 2 also moving the time on; not with 'average', whose flagged blocks
+// are reduced by a second kernel.
+int launch_getdt(amrvac_ctx *c, int reg, int tail = 0) {
   GetdtArgs G;
+  G.scal = tail ? c->d_scal : nullptr;
+  G.ticket = reinterpret_cast<unsigned *>(c->d_red + 2);
+  G.advance = tail == 2;
   G.u = c->pool[reg];
   G.dxb = c->d_dx;
   G.nblocks = c->nblocks;
@@ -292,8 +317,10 @@ int launch_getdt(amrvac_ctx *c, int reg) {
     ++c->launches;
     G.skip = c->d_block_status;
   }
+  G.dependent = c->chained;
   CK(c->ks.getdt(G, c->stream));
   ++c->launches;
+  c->chained = c->chain_on && !c->sv_on && !c->cfg.schmid_global;
   if (c->sv_on) {
     CK(c->sv.getdt(SA, c->pool[reg], c->cfg.type_courant, c->d_red, SvScratch{c->sv_scratch, c->sv_per_cta},
                    c->sv_ctas, c->stream));
@@ -340,6 +367,7 @@ int launch_fourstep(amrvac_ctx *c, cudaEvent_t *ev) {
     CK(launch_rk4_combine(c->pool[0], c->pool[1], c->pool[2], c->pool[3], c->per_block * c->nw * c->nblocks,
                           c->stream));
     ++c->launches;
+    c->chained = false;
     mark(2);
     r = launch_stage(c, 3, 0, 0, 1.0, 0.0, 1.0 / 6.0);
     mark(3);
@@ -408,10 +436,12 @@ int launch_fivestep(amrvac_ctx *c, cudaEvent_t *ev) {
   mark(2);
   CK(launch_ssprk5_ps3(c->pool[3], c->pool[2], c->pool[1], K.a53, K.a54, n, c->stream));
   ++c->launches;
+  c->chained = false;
   if ((r = launch_stage(c, 1, 2, 0, K.a41, K.a44, K.b44))) return r;
   CK(launch_ssprk5_final(c->pool[0], c->pool[1], c->pool[2], c->pool[3], K.a55, K.b54 / K.b44, K.a41, K.a44, n,
                          c->stream));
   ++c->launches;
+  c->chained = false;
   mark(3);
   r = launch_stage(c, 2, 0, 0, 1.0, 0.0, K.b55);
   mark(4);
@@ -425,6 +455,7 @@ int launch_rk(amrvac_ctx *c) {
   if (k.time_stepper == AMRVAC_TS_ONESTEP) {
     CK(cudaMemcpyAsync(c->pool[1], c->pool[0], sizeof(double) * c->per_block * c->nw * c->nblocks,
                        cudaMemcpyDeviceToDevice, c->stream));
+    c->chained = false;
     r = launch_stage(c, 1, 0, 0, 0.0, 1.0, 1.0);
   } else if (k.time_stepper == AMRVAC_TS_TWOSTEP) {
     if (k.time_integrator == AMRVAC_TI_SSPRK2) {
@@ -452,9 +483,17 @@ int launch_rk(amrvac_ctx *c) {
 
 int launch_step(amrvac_ctx *c) {
   int r;
-  if ((r = launch_getdt(c, 0))) return r;
-  CK(launch_setdt_finalize(c->d_red, c->d_scal, c->d_status, c->stream));
-  ++c->launches;
+  ChainScope chain(c);
+  // setdt and the time update in the getdt kernel: two launches less of six.
+  // The direction of a dimensionally split sweep follows the step count, so
+  // there the count moves on at the end of the step.
+  const int tail = c->sv_on ? 0 : (c->cfg.dimsplit ? 1 : 2);
+  if ((r = launch_getdt(c, 0, tail))) return r;
+  if (tail == 0) {
+    CK(launch_setdt_finalize(c->d_red, c->d_scal, c->d_status, c->stream));
+    ++c->launches;
+    c->chained = false;
+  }
   if (c->cfg.dimsplit) {  // one full stepper per direction (src/mod_advance.t:23-45)
     for (int s = 0; s < c->cfg.ndim && !r; ++s) {
       c->sweep = s;
@@ -465,8 +504,10 @@ int launch_step(amrvac_ctx *c) {
   } else if ((r = launch_rk(c))) {
     return r;
   }
-  CK(launch_advance_time(c->d_scal, c->stream));
-  ++c->launches;
+  if (tail != 2) {
+    CK(launch_advance_time(c->d_scal, c->stream));
+    ++c->launches;
+  }
   return 0;
 }
 
@@ -714,8 +755,8 @@ int amrvac_gpu_create(const amrvac_cfg *cfg, amrvac_ctx **out) {
                          0.0, 0.0, 0.0};
   if ((e = cudaMalloc(&c->d_scal, sizeof(sc))) != cudaSuccess ||
       (e = cudaMemcpy(c->d_scal, sc, sizeof(sc), cudaMemcpyHostToDevice)) != cudaSuccess ||
-      (e = cudaMalloc(&c->d_red, 2 * sizeof(unsigned long long))) != cudaSuccess ||
-      (e = cudaMemset(c->d_red, 0, 2 * sizeof(unsigned long long))) != cudaSuccess ||
+      (e = cudaMalloc(&c->d_red, 3 * sizeof(unsigned long long))) != cudaSuccess ||
+      (e = cudaMemset(c->d_red, 0, 3 * sizeof(unsigned long long))) != cudaSuccess ||
       (e = cudaMalloc(&c->d_status, sizeof(uint32_t))) != cudaSuccess ||
       (e = cudaMemset(c->d_status, 0, sizeof(uint32_t))) != cudaSuccess) {
     amrvac_gpu_destroy(c);
@@ -1783,6 +1824,8 @@ int amrvac_gpu_step_dt(amrvac_ctx *c, double dt) {
   if (int r = check_a2max(c)) return r;
   CK(launch_set_scalar(c->d_scal + 0, dt, c->stream));
   ++c->launches;
+  ChainScope chain(c);
+  c->chained = true;  // the scalar's kernel begins as the stages do
   return launch_rk(c);
 }
 
@@ -1819,6 +1862,8 @@ int amrvac_gpu_step_dt_states(amrvac_ctx *c, double dt, const double *u0, double
   if (int r = check_a2max(c)) return r;
   CK(launch_set_scalar(c->d_scal + 0, dt, c->stream));
   ++c->launches;
+  ChainScope chain(c);
+  c->chained = true;  // the scalar's kernel begins as the stages do
   double *const saved[3] = {c->pool[0], c->pool[1], c->pool[2]};
   c->pool[0] = const_cast<double *>(u0);  // read only: every stage takes it as input or base
   c->pool[1] = u1;
@@ -1904,10 +1949,13 @@ static int adjoint_step_impl(amrvac_ctx *c, const double *u0, const double *u1, 
     A.b = b;
     for (int d = 0; d < 2; ++d) A.s[d] = dtf * dt / c->h_dx[d];
     A.gamma_part = gamma_part;
+    A.sa.dependent = c->chained;
     return A;
   };
   CK(launch_set_scalar(c->d_scal + 0, dt, c->stream));
   ++c->launches;
+  ChainScope chain(c);
+  c->chained = true;
   if (k.time_stepper == AMRVAC_TS_TWOSTEP) {
     // forward U1 = U0 + dt L(U0); U2 = (U0 + U1 + dt L(U1)) / 2
     if (!u0)

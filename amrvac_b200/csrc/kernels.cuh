@@ -7,6 +7,40 @@
 
 namespace amrvac {
 
+// ---------------------------------------------------------------- setdt tail
+// After the CFL reduction: dt = courantpar / max (src/mod_dt.t:233-235), the
+// dtmin check (55-60), the slowsteps ramp (64-67), final_dt_reduction (69-79)
+// and the output-interval cap (88-99).  scal: [0]=dt [1]=cmax_global
+// [2]=global_time [3]=time_max [4]=dtsave [5]=dtmin [6]=courantpar
+// [7]=final_exit flag [8]=slowsteps [9]=steps since set_time (it - it_init).
+__device__ __forceinline__ void setdt_finalize(volatile unsigned long long *red, volatile double *scal,
+                                               uint32_t *status) {
+  const double smalldouble = 1.0e-12, bigdouble = 1.0e99;
+  const double x = __longlong_as_double((long long)red[0]);
+  const double cm = __longlong_as_double((long long)red[1]);
+  red[0] = 0ull;
+  red[1] = 0ull;
+  double dt = bigdouble;
+  if (x > smalldouble) dt = fmin(dt, scal[6] / x);
+  if (dt < scal[5]) atomicOr(status, ST_DT_TOO_SMALL);
+  if (scal[8] > scal[9] + 1.0) {
+    const double q = 1.0 - (scal[9] + 1.0) / scal[8];
+    dt = dt * (1.0 - q * q);
+  }
+  const double t = scal[2], tmax = scal[3], dtsave = scal[4];
+  if (tmax - t <= scal[5]) scal[7] = 1.0;
+  dt = fmin(dt, tmax - t);
+  if (dtsave > 0.0) {
+    double dtmax = ceil(t / dtsave) * dtsave;
+    const double other = t > 0.0 ? ceil(t / bigdouble) * bigdouble : 0.0;
+    dtmax = fmin(dtmax, other) - t;
+    if (dtmax > smalldouble) dt = fmin(dt, dtmax);
+    else dt = fmin(dt, dtsave);
+  }
+  scal[0] = dt;
+  scal[1] = cm;
+}
+
 // ---------------------------------------------------------------- getdt
 // getdt_courant (src/mod_dt.t:160-287) per block, reduced over all blocks.
 // red[0] <- max over blocks of the block's courant sum (maxsum: max_cells
@@ -21,6 +55,14 @@ struct GetdtArgs {
   PhysParams P;
   uint32_t *status;  // the context's status word: the small-value check of getdt
   const uint32_t *skip;  // 'average': blocks flagged ST_SV_AVG are reduced by sv_getdt_kernel
+  // setdt in the same launch: the last CTA to finish (counted in *ticket)
+  // turns the maxima into dt (scal non-null), and with advance also moves
+  // global_time and the step count on (nothing between here and the end of
+  // an unsplit step reads them)
+  double *scal;
+  unsigned *ticket;
+  int advance;
+  bool dependent;  // launch: the predecessor on the stream allows a dependent launch
 };
 
 __device__ __forceinline__ double warp_max(double v) {
@@ -34,87 +76,113 @@ __device__ __forceinline__ void atomic_max_pos(unsigned long long *a, double v) 
   if (v > 0.0) atomicMax(a, (unsigned long long)__double_as_longlong(v));
 }
 
+// Work items: up to GETDT_CHUNK cells of one block, x fastest (coalesced), 256
+// threads at a time.  With 'maxsum' only two maxima leave a block, so the
+// CTAs (one wave of four per SM, 64 registers) stride over the items of all
+// blocks and reduce once at the end; 'summax' and 'minimum' combine the
+// directions' maxima of a block, so there an item is a whole block and each is
+// reduced on its own.  The kernel is bound by its loads' latency: one CTA per
+// block at two per SM measured 53 us at 128^3 MHD (151 MB).
+constexpr int GETDT_CHUNK = 1024;
 template <bool MHD, int NDIR, bool GLM, int NDIM>
-__global__ void __launch_bounds__(256) getdt_kernel(const GetdtArgs A) {
+__global__ void __launch_bounds__(256, 4) getdt_kernel(const GetdtArgs A) {
   using V = Vars<MHD, NDIR, GLM>;
   constexpr int NW = V::NW;
   const int bn = A.bn;
   const int ncell = bn * (NDIM >= 2 ? bn : 1) * (NDIM == 3 ? bn : 1);
-  const int b = blockIdx.x;
   const int t = threadIdx.x;
-  if (A.skip && (A.skip[b] & ST_SV_AVG)) return;
-  double dxinv[3];
-#pragma unroll
-  for (int d = 0; d < NDIM; ++d) dxinv[d] = 1.0 / A.dxb[b * 3 + d];
-  double mtot = 0.0, mcm = 0.0, mdim[3] = {0.0, 0.0, 0.0};
-  // the block's cells, x fastest (coalesced), 256 at a time; c is the
-  // cell's index within its block-variable row (cell_offset's layout)
-  const double *ub = A.u + (size_t)b * NW * ncell;
-#pragma unroll 2
-  for (int c = t; c < ncell; c += 256) {
-    double w[NW];
-#pragma unroll
-    for (int v = 0; v < NW; ++v) w[v] = __ldg(ub + (size_t)v * ncell + c);
-    // getdt_courant takes the primitives through phys_to_primitive, small-value
-    // fix included (src/mod_dt.t:189-191)
-    if (A.P.fix_small_values) {
-      if (small_values<double, MHD, NDIR, GLM>(w, false, A.P) && A.P.small_values_method != 1 && A.status)
-        atomicOr(A.status, ST_SMALL_VALUE);
-    }
-    to_primitive<MHD, NDIR, GLM>(w, A.P);
-    double tot = 0.0;
-#pragma unroll
-    for (int d = 0; d < NDIM; ++d) {
-      double cm;
-      if constexpr (MHD) {
-        double cf;
-        if (d == 0) cf = fast_speed<double, NDIR, V::B0 + 0>(w, A.P);
-        else if (d == 1) cf = fast_speed<double, NDIR, V::B0 + (NDIR > 1 ? 1 : 0)>(w, A.P);
-        else cf = fast_speed<double, NDIR, V::B0 + (NDIR > 2 ? 2 : 0)>(w, A.P);
-        cm = fabs(w[V::M0 + d]) + cf;
-      } else {
-        cm = fabs(w[V::M0 + d]) + sqrt(A.P.gamma * w[V::E] / w[V::RHO]);
-      }
-      const double c = cm * dxinv[d];
-      tot = d == 0 ? c : tot + c;
-      mdim[d] = fmax(mdim[d], c);
-      mcm = fmax(mcm, cm);
-    }
-    mtot = fmax(mtot, tot);
-  }
-  __shared__ double red[4][8];
+  const bool maxsum = A.type_courant == 1;
+  const int chunk = maxsum ? GETDT_CHUNK : ncell;
+  const int parts = (ncell + chunk - 1) / chunk, nitem = A.nblocks * parts;
+  __shared__ double red[5][8];
   const int lane = t & 31, wid = t >> 5;
-  double r0 = warp_max(mtot), r1 = warp_max(mcm);
-  double r2[3];
+  pdl_wait();
+  pdl_trigger();
+  double mtot = 0.0, mcm = 0.0, mdim[3] = {0.0, 0.0, 0.0};
+  // the maxima of all threads into red[0]; adds them to the global words
+  auto reduce = [&]() {
+    const double v[5] = {mtot, mcm, mdim[0], mdim[1], mdim[2]};
 #pragma unroll
-  for (int d = 0; d < 3; ++d) r2[d] = warp_max(mdim[d]);
-  if (lane == 0) {
-    red[0][wid] = r0; red[1][wid] = r1;
-    red[2][wid] = r2[0]; red[3][wid] = r2[1];
-  }
-  __shared__ double red3[8];
-  if (lane == 0) red3[wid] = r2[2];
-  __syncthreads();
-  if (t == 0) {
-    double a0 = 0, a1 = 0, d0 = 0, d1 = 0, d2 = 0;
-    for (int q = 0; q < 8; ++q) {
-      a0 = fmax(a0, red[0][q]); a1 = fmax(a1, red[1][q]);
-      d0 = fmax(d0, red[2][q]); d1 = fmax(d1, red[3][q]); d2 = fmax(d2, red3[q]);
+    for (int q = 0; q < 5; ++q) {
+      const double w = warp_max(v[q]);
+      if (lane == 0) red[q][wid] = w;
     }
-    double x;
-    if (A.type_courant == 1) {
-      x = a0;
-    } else {
-      double dd[3] = {d0, d1, d2};
-      double courantmax = 0.0, tot = 0.0;
-      for (int d = 0; d < NDIM; ++d) {
-        courantmax = fmax(courantmax, dd[d]);
-        tot = tot + courantmax;
+    __syncthreads();
+    if (t == 0) {
+      double m[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+      for (int q = 0; q < 5; ++q)
+        for (int w = 0; w < 8; ++w) m[q] = fmax(m[q], red[q][w]);
+      double x = m[0];
+      if (!maxsum) {
+        double courantmax = 0.0, tot = 0.0;
+        for (int d = 0; d < NDIM; ++d) {
+          courantmax = fmax(courantmax, m[2 + d]);
+          tot = tot + courantmax;
+        }
+        x = A.type_courant == 2 ? tot : courantmax;
       }
-      x = A.type_courant == 2 ? tot : courantmax;
+      atomic_max_pos(A.red + 0, x);
+      atomic_max_pos(A.red + 1, m[1]);
     }
-    atomic_max_pos(A.red + 0, x);
-    atomic_max_pos(A.red + 1, a1);
+    __syncthreads();
+  };
+  for (int it = blockIdx.x; it < nitem; it += gridDim.x) {
+    const int b = it / parts, c0 = (it - b * parts) * chunk, c1 = min(c0 + chunk, ncell);
+    if (A.skip && (A.skip[b] & ST_SV_AVG)) continue;
+    double dxinv[3];
+#pragma unroll
+    for (int d = 0; d < NDIM; ++d) dxinv[d] = 1.0 / A.dxb[b * 3 + d];
+    // c is the cell's index within its block-variable row (cell_offset's layout)
+    const double *ub = A.u + (size_t)b * NW * ncell;
+#pragma unroll 1
+    for (int c = c0 + t; c < c1; c += 256) {
+      double w[NW];
+#pragma unroll
+      for (int v = 0; v < NW; ++v) w[v] = ub[(size_t)v * ncell + c];
+      // getdt_courant takes the primitives through phys_to_primitive, small-value
+      // fix included (src/mod_dt.t:189-191)
+      if (A.P.fix_small_values) {
+        if (small_values<double, MHD, NDIR, GLM>(w, false, A.P) && A.P.small_values_method != 1 && A.status)
+          atomicOr(A.status, ST_SMALL_VALUE);
+      }
+      to_primitive<MHD, NDIR, GLM>(w, A.P);
+      double tot = 0.0;
+#pragma unroll
+      for (int d = 0; d < NDIM; ++d) {
+        double cm;
+        if constexpr (MHD) {
+          double cf;
+          if (d == 0) cf = fast_speed<double, NDIR, V::B0 + 0>(w, A.P);
+          else if (d == 1) cf = fast_speed<double, NDIR, V::B0 + (NDIR > 1 ? 1 : 0)>(w, A.P);
+          else cf = fast_speed<double, NDIR, V::B0 + (NDIR > 2 ? 2 : 0)>(w, A.P);
+          cm = fabs(w[V::M0 + d]) + cf;
+        } else {
+          cm = fabs(w[V::M0 + d]) + sqrt(A.P.gamma * w[V::E] / w[V::RHO]);
+        }
+        const double cd = cm * dxinv[d];
+        tot = d == 0 ? cd : tot + cd;
+        mdim[d] = fmax(mdim[d], cd);
+        mcm = fmax(mcm, cm);
+      }
+      mtot = fmax(mtot, tot);
+    }
+    if (!maxsum) {
+      reduce();
+      mtot = mcm = mdim[0] = mdim[1] = mdim[2] = 0.0;
+    }
+  }
+  if (maxsum) reduce();
+  if (t == 0 && A.scal) {
+    __threadfence();
+    if (atomicAdd(A.ticket, 1u) == gridDim.x - 1) {
+      __threadfence();
+      *A.ticket = 0u;
+      setdt_finalize(A.red, A.scal, A.status);
+      if (A.advance) {
+        A.scal[2] = A.scal[2] + A.scal[0];
+        A.scal[9] = A.scal[9] + 1.0;
+      }
+    }
   }
 }
 
@@ -325,8 +393,8 @@ struct StageVar {
                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM);
   }
   static cudaError_t stage(const StageArgs &A, int nctas, cudaStream_t s) {
-    fv_stage_kernel<TF, MHD, NDIR, GLM, NDIM, SOLVER, LIM, BS, BN, VAR><<<nctas, O::THREADS, SMEM, s>>>(A);
-    return cudaGetLastError();
+    return launch_dependent<StageArgs>(&fv_stage_kernel<TF, MHD, NDIR, GLM, NDIM, SOLVER, LIM, BS, BN, VAR>, nctas,
+                                       O::THREADS, SMEM, s, A.dependent, A);
   }
   static int ctas_per_sm() {
     int n = 0;
@@ -381,12 +449,12 @@ struct Launch {
   static cudaError_t stage(const StageArgs &A, int nctas, cudaStream_t s) {
     if constexpr (HAS_DENSE) {
       if (A.nblocks * NTILE > SMALL_TILES) {
-        fv_stage_kernel<TF, MHD, NDIR, GLM, NDIM, SOLVER, LIM, BS, BN, VAR_DENSE><<<nctas, THREADS, SMEM, s>>>(A);
-        return cudaGetLastError();
+        return launch_dependent<StageArgs>(&fv_stage_kernel<TF, MHD, NDIR, GLM, NDIM, SOLVER, LIM, BS, BN, VAR_DENSE>,
+                                           nctas, THREADS, SMEM, s, A.dependent, A);
       }
     }
-    fv_stage_kernel<TF, MHD, NDIR, GLM, NDIM, SOLVER, LIM, BS, BN><<<nctas, THREADS, SMEM, s>>>(A);
-    return cudaGetLastError();
+    return launch_dependent<StageArgs>(&fv_stage_kernel<TF, MHD, NDIR, GLM, NDIM, SOLVER, LIM, BS, BN>, nctas, THREADS,
+                                       SMEM, s, A.dependent, A);
   }
   static cudaError_t a2max(const StageArgs &A, double *out, cudaStream_t s) {
     a2max_kernel<V::NW, NDIM, BN><<<A.nblocks * (NDIM == 3 ? BN : 1), 256, 0, s>>>(A, out);
@@ -404,8 +472,8 @@ struct Launch {
     if constexpr (HAS_HANCOCK) {
       // nctas is one wave of the main kernel, which is denser than this one
       if (HAS_DENSE && A.zchunk == 0 && nctas > SMALL_TILES) nctas = SMALL_TILES;
-      fv_stage_kernel<TF, MHD, NDIR, GLM, NDIM, SOLVER_HANCOCK, LIM, BS, BN><<<nctas, THREADS, SMEM, s>>>(A);
-      return cudaGetLastError();
+      return launch_dependent<StageArgs>(&fv_stage_kernel<TF, MHD, NDIR, GLM, NDIM, SOLVER_HANCOCK, LIM, BS, BN>, nctas,
+                                         THREADS, SMEM, s, A.dependent, A);
     } else {
       return cudaErrorNotSupported;
     }
@@ -418,8 +486,11 @@ struct Launch {
     return n > 0 ? n : 1;
   }
   static cudaError_t getdt(const GetdtArgs &A, cudaStream_t s) {
-    getdt_kernel<MHD, NDIR, GLM, NDIM><<<A.nblocks, 256, 0, s>>>(A);
-    return cudaGetLastError();
+    int ncell = 1;
+    for (int d = 0; d < NDIM; ++d) ncell *= A.bn;
+    const long items = (long)A.nblocks * (A.type_courant == 1 ? (ncell + GETDT_CHUNK - 1) / GETDT_CHUNK : 1);
+    const int nctas = (int)(items < 4 * 148 ? items : 4 * 148);
+    return launch_dependent<GetdtArgs>(&getdt_kernel<MHD, NDIR, GLM, NDIM>, nctas, 256, 0, s, A.dependent, A);
   }
   template <int D>
   static void rp(const PointArgs &A, cudaStream_t s) {

@@ -145,14 +145,18 @@ __device__ __forceinline__ double sqrt_nr(double x) {
   h = fma(h, r, h);
   return fma(fma(-s, s, x), h, s);
 }
-template <bool FAST> __device__ __forceinline__ double rcp_f(double y) {
+// FAST of the face routines: the guarded forms, the unguarded ones, or the
+// unguarded reciprocal and quotient (which round as the guarded ones do) with
+// the IEEE square root (sqrt_nr differs from it about once in 2^27).
+enum : int { FAST_NONE = 0, FAST_ALL = 1, FAST_DIV = 2 };
+template <int FAST> __device__ __forceinline__ double rcp_f(double y) {
   if constexpr (FAST) return rcp_nr(y); else return rcp_(y);
 }
-template <bool FAST> __device__ __forceinline__ double div_f(double x, double y) {
+template <int FAST> __device__ __forceinline__ double div_f(double x, double y) {
   if constexpr (FAST) return div_nr(x, y); else return div_(x, y);
 }
-template <bool FAST> __device__ __forceinline__ double sqrt_f(double x) {
-  if constexpr (FAST) return sqrt_nr(x); else return sqrt(x);
+template <int FAST> __device__ __forceinline__ double sqrt_f(double x) {
+  if constexpr (FAST == FAST_ALL) return sqrt_nr(x); else return sqrt(x);
 }
 // Single precision (the mixed form's faces): IEEE, or with FAST the hardware
 // approximations of PTX (rcp.approx.ftz.f32, sqrt.approx.ftz.f32, about one
@@ -169,13 +173,13 @@ __device__ __forceinline__ float sqrt_approx(float x) {
   asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
   return r;
 }
-template <bool FAST> __device__ __forceinline__ float rcp_f(float y) {
+template <int FAST> __device__ __forceinline__ float rcp_f(float y) {
   if constexpr (FAST) return rcp_approx(y); else return rcp_(y);
 }
-template <bool FAST> __device__ __forceinline__ float div_f(float x, float y) {
+template <int FAST> __device__ __forceinline__ float div_f(float x, float y) {
   if constexpr (FAST) return x * rcp_approx(y); else return div_(x, y);
 }
-template <bool FAST> __device__ __forceinline__ float sqrt_f(float x) {
+template <int FAST> __device__ __forceinline__ float sqrt_f(float x) {
   if constexpr (FAST) return sqrt_approx(x); else return sqrtf(x);
 }
 
@@ -299,7 +303,7 @@ __device__ __forceinline__ void phys_flux(const T *wc, const T *w, T cg,
 
 // mhd_get_csound_prim (mod_mhd_phys.t:3329-3379): the square of the fast
 // magnetosonic speed, and the speed.
-template <class T, int NDIR, int BN, bool FAST = false>
+template <class T, int NDIR, int BN, int FAST = 0>
 __device__ __forceinline__ T fast_speed2(const T *w, const PhysParams &P) {
   constexpr int RHO = 0, E = NDIR + 1, B0 = NDIR + 2;
   const T inv_rho = rcp_f<FAST>(w[RHO]);
@@ -312,7 +316,7 @@ __device__ __forceinline__ T fast_speed2(const T *w, const PhysParams &P) {
   if (av < T(0.0)) av = T(0.0);
   return T(0.5) * (cfast2 + sqrt_f<FAST>(av));
 }
-template <class T, int NDIR, int BN, bool FAST = false>
+template <class T, int NDIR, int BN, int FAST = 0>
 __device__ __forceinline__ T fast_speed(const T *w, const PhysParams &P) {
   return sqrt_f<FAST>(fast_speed2<T, NDIR, BN, FAST>(w, P));
 }
@@ -321,7 +325,7 @@ __device__ __forceinline__ T fast_speed(const T *w, const PhysParams &P) {
 // WITH_MIN=false gives the tvdlf form (cmax only).  Returns a status bit.
 // SQUARED: the Einfeldt mean takes the squares of the fast speeds directly;
 // the reference squares the speeds (two square roots more, rounding apart).
-template <class T, bool MHD, int NDIR, bool GLM, int D, bool WITH_MIN, int BS = 0, bool FAST = false,
+template <class T, bool MHD, int NDIR, bool GLM, int D, bool WITH_MIN, int BS = 0, int FAST = 0,
           bool SQUARED = false>
 __device__ __forceinline__ uint32_t cbounds(const T *wLC, const T *wRC, const T *wLp,
                                             const T *wRp, const PhysParams &P, T &cmax,
@@ -402,7 +406,7 @@ __device__ __forceinline__ uint32_t cbounds(const T *wLC, const T *wRC, const T 
     } else {
       const T csL = div_f<FAST>(T(P.gamma) * wLp[V::E], wLp[V::RHO]);
       const T csR = div_f<FAST>(T(P.gamma) * wRp[V::E], wRp[V::RHO]);
-      cs = fmax(sqrt_f<FAST>(csL), sqrt_f<FAST>(csR));
+      cs = sqrt_f<FAST>(fmax(csL, csR));  // the root of the larger: both round the same way
     }
     if (WITH_MIN) cmin = fmin(wLp[MN], wRp[MN]) - cs;
     cmax = fmax(wLp[MN], wRp[MN]) + cs;
@@ -410,10 +414,20 @@ __device__ __forceinline__ uint32_t cbounds(const T *wLC, const T *wRC, const T 
   return st;
 }
 
+// Minimum and maximum of finite numbers.  In FP64 one compare and a select:
+// fmin / fmax also order NaN operands, which takes two or three instructions
+// more (a NaN here reaches the flux through the state that held it).
+__device__ __forceinline__ double min_(double a, double b) { return a < b ? a : b; }
+__device__ __forceinline__ double max_(double a, double b) { return a > b ? a : b; }
+__device__ __forceinline__ float min_(float a, float b) { return fminf(a, b); }
+__device__ __forceinline__ float max_(float a, float b) { return fmaxf(a, b); }
+__device__ __forceinline__ bool is_negative(double x) { return __double2hiint(x) < 0; }
+__device__ __forceinline__ bool is_negative(float x) { return __float_as_int(x) < 0; }
+
 // ------------------------------------------------------------------ limiters
 // dwlimiter2 (mod_limiter.t:128-334) for one cell: a = dwC(ix) (forward
 // difference), b = dwC(ix-1) (backward difference).  LEFT selects ldw, else rdw.
-template <class T, bool LEFT, bool FAST = false>
+template <class T, bool LEFT, int FAST = 0>
 __device__ __forceinline__ T slope_impl(int lim, T a, T b, T rdelinv) {
   constexpr T qsmall = T(1.0e-12), qsmall2 = T(2.0e-12);
   constexpr T eps = T(1.4901161193847656e-08);  // sqrt(epsilon(1d0)) = 2**-26
@@ -423,10 +437,10 @@ __device__ __forceinline__ T slope_impl(int lim, T a, T b, T rdelinv) {
   switch (lim) {
     case LIM_MINMOD: {
       const T t = fsign(T(1.0), a);
-      return t * fmax(T(0.0), fmin(fabs(a), t * b));
+      return t * max_(T(0.0), min_(fabs(a), t * b));
     }
     case LIM_VANLEER:
-      return div_f<FAST>(T(2.0) * fmax(b * a, T(0.0)), a + b + qsmall);
+      return div_f<FAST>(T(2.0) * max_(b * a, T(0.0)), a + b + qsmall);
     case LIM_CADA3: {
       // branch-free: both the asymptotic and the limited form are evaluated
       // and the reference's three-way choice is made with selects
@@ -487,16 +501,6 @@ __device__ __forceinline__ T limited_slope(int lim_rt, T a, T b, T rdelinv) {
   return slope_impl<T, LEFT>(LIM ? LIM : lim_rt, a, b, rdelinv);
 }
 
-// Minimum and maximum of finite numbers.  In FP64 one compare and a select:
-// fmin / fmax also order NaN operands, which takes two or three instructions
-// more (a NaN here reaches the flux through the state that held it).
-__device__ __forceinline__ double min_(double a, double b) { return a < b ? a : b; }
-__device__ __forceinline__ double max_(double a, double b) { return a > b ? a : b; }
-__device__ __forceinline__ float min_(float a, float b) { return fminf(a, b); }
-__device__ __forceinline__ float max_(float a, float b) { return fmaxf(a, b); }
-__device__ __forceinline__ bool is_negative(double x) { return __double2hiint(x) < 0; }
-__device__ __forceinline__ bool is_negative(float x) { return __float_as_int(x) < 0; }
-
 // Asymptotic and limited form of the cada3 / schmid limiters (dwlimiter2,
 // src/limiter/mod_limiter.t:253-290, 291-333) at the slope ratio t:
 //   A = (2 + t) / 3,
@@ -552,7 +556,7 @@ __device__ __forceinline__ bool near_one(float, float) { return false; }
 // (cada3_radius dx)^2 and tmpeta <= 1 is tested as a^2 + b^2 <= rdel without
 // the product.  With the limiter fixed to cada3 and BLEND false the blending
 // band is left out: a face near it gets `special` and is recomputed.
-template <class T, int LIM, bool FAST = false, bool R2 = false, bool BLEND = true>
+template <class T, int LIM, int FAST = 0, bool R2 = false, bool BLEND = true>
 __device__ __forceinline__ void face_states(int lim_rt, T q0, T q1, T q2, T q3, T rdel, T &wL, T &wR, bool &special) {
   constexpr T eps = T(1.4901161193847656e-08);  // sqrt(epsilon(1d0)) = 2**-26
   const int lim = LIM ? LIM : lim_rt;

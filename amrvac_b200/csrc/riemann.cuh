@@ -35,7 +35,7 @@ __device__ __forceinline__ void riemann_tvdlf(const T *wLC, const T *wRC, const 
 }
 
 // get_Riemann_flux_hll (mod_finite_volume.t:381-437)
-template <class T, bool MHD, int NDIR, bool GLM, int NDIM, int D, bool FAST = false>
+template <class T, bool MHD, int NDIR, bool GLM, int NDIM, int D, int FAST = 0>
 __device__ __forceinline__ void riemann_hll(const T *wLC, const T *wRC, const T *fL,
                                             const T *fR, T cmax, T cmin,
                                             T tvdlfeps, T *F) {
@@ -63,7 +63,7 @@ __device__ __forceinline__ void riemann_hll(const T *wLC, const T *wRC, const T 
 // state, every expression in the reference's order.  F = fS + c (wCD - wS)
 // behind the contact, fS in a supersonic state; the HLL flux (lambda_CD
 // outside the bounds) is a branch of its own.
-template <class T, int NDIR, bool FAST = false>
+template <class T, int NDIR, int FAST = 0>
 __device__ __forceinline__ void riemann_hllc_hd(const T *wLC, const T *wRC, const T *wLp, const T *wRp, T cmax, T cmin,
                                                 T *F) {
   using V = Vars<false, NDIR, false>;
@@ -121,7 +121,7 @@ __device__ __forceinline__ void riemann_hllc_hd(const T *wLC, const T *wRC, cons
 // has zero normal-B (and psi) entries, which the flux_type rules then
 // replace by the diffusive tvdlf form without GLM, and keep with GLM (the
 // reference's HLLC takes no flux_special branch).
-template <class T, int NDIR, bool GLM, int NDIM, int D, bool FAST = false>
+template <class T, int NDIR, bool GLM, int NDIM, int D, int FAST = 0>
 __device__ __forceinline__ void riemann_hllc_mhd(const T *wLC, const T *wRC, const T *fL, const T *fR, T cmax,
                                                  T cmin, T tvdlfeps, T *F) {
   using V = Vars<true, NDIR, GLM>;
@@ -431,7 +431,7 @@ __device__ __forceinline__ void riemann_tvdmu_mhd(const T *wLC, const T *wRC, co
 // everything behind it (physical flux, star energies, the outer Alfven
 // speed) is formed for the side of the contact that the face lies in alone,
 // every expression in the reference's order.
-template <class T, int NDIR, bool GLM, int NDIM, bool FAST = false>
+template <class T, int NDIR, bool GLM, int NDIM, int FAST = 0>
 __device__ __forceinline__ void riemann_hlld(const T *wLC, const T *wRC, const T *wLp, const T *wRp, T sR, T sL, T cg,
                                              T *F) {
   using V = Vars<true, NDIR, GLM>;
@@ -537,7 +537,7 @@ constexpr bool hlld_from_primitives = NDIM == 3 || sizeof(T) == 4;
 // common factors are taken out, a quarter fewer operations than riemann_hlld
 // (3-D MHD 128^3 FP64 0.64 -> 0.59 ms per stage, mixed 0.42 -> 0.39) at
 // rounding differences.  hlld_from_primitives says where it is used.
-template <class T, int NDIR, bool GLM, int NDIM, bool FAST = false>
+template <class T, int NDIR, bool GLM, int NDIM, int FAST = 0>
 __device__ __forceinline__ void riemann_hlld_prim(const T *wLp, const T *wRp, T sR, T sL, T cg, T inv_gamma_1, T *F) {
   using V = Vars<true, NDIR, GLM>;
   using FT = FluxTypes<true, NDIM, GLM>;

@@ -73,6 +73,33 @@ __host__ __device__ constexpr int stage_threads(int bn) {
 // thread, measured 17-25 % slower on 3-D MHD.)
 constexpr int STAGE_THREADS = AMRVAC_STAGE_THREADS;
 
+// ---------------------------------------------------------------- dependent launches
+// The kernels of a time step follow one another on one stream and each needs
+// all of its predecessor's results, but their launches need not wait for its
+// end: with programmatic dependent launch a kernel's CTAs are placed as the
+// predecessor's last CTAs leave, and wait there (pdl_wait) until it has
+// finished and its writes are visible.  Every kernel launched this way begins
+// with pdl_wait, before it reads anything, then lets its own successor come
+// (pdl_trigger: takes effect once every CTA has called it, so a successor
+// never holds the place of a CTA that has yet to start).
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+template <class Args>
+cudaError_t launch_dependent(void (*kernel)(Args), int nctas, int threads, size_t smem, cudaStream_t s, bool dependent,
+                             const Args &A) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)nctas);
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = dependent ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, A);
+}
+
 enum : int { BCK_PERIODIC = 0, BCK_CONT = 1, BCK_MIRROR = 2 };
 
 struct StageArgs {
@@ -106,6 +133,7 @@ struct StageArgs {
   int sweep;
   int split_xy;             // 1: typedimsplit 'xy' (same order every step)
   int bn;                   // block edge, for the kernels that take it at run time
+  int dependent;            // launch: the predecessor on the stream allows a dependent launch
 };
 
 // Direction of a dimensionally split sweep (src/mod_advance.t:23-45):
@@ -190,6 +218,8 @@ __device__ __forceinline__ size_t ghost_offset(int slot, int nw, int v, int i, i
 
 // Load the conserved state of a (possibly out-of-block) cell and return it
 // as primitives.  Returns a status bit if the small-value check fires.
+// (Plain loads: with a dependent launch the predecessor writes the state while
+// this kernel's CTAs already exist, which read-only loads do not allow for.)
 template <bool MHD, int NDIR, bool GLM, int NDIM, int BN = BN16>
 __device__ __forceinline__ uint32_t load_prim(const StageArgs &A, int b, int i, int j, int k,
                                               double *w) {
@@ -199,13 +229,13 @@ __device__ __forceinline__ uint32_t load_prim(const StageArgs &A, int b, int i, 
   if (blk >= 0) {
 #pragma unroll
     for (int v = 0; v < V::NW; ++v) {
-      double x = __ldg(A.uin + cell_offset<NDIM>(blk, V::NW, v, i, j, k, BN));
+      const double x = A.uin[cell_offset<NDIM>(blk, V::NW, v, i, j, k, BN)];
       w[v] = ((flip >> v) & 1u) ? -x : x;
     }
   } else {  // level jump: this block's ghost buffer
 #pragma unroll
     for (int v = 0; v < V::NW; ++v) {
-      const double x = __ldg(A.gbuf + ghost_offset<NDIM>(-2 - blk, V::NW, v, i, j, k, BN));
+      const double x = A.gbuf[ghost_offset<NDIM>(-2 - blk, V::NW, v, i, j, k, BN)];
       w[v] = ((flip >> v) & 1u) ? -x : x;
     }
   }
@@ -222,7 +252,7 @@ __device__ __forceinline__ uint32_t load_prim(const StageArgs &A, int b, int i, 
 // (src/mod_finite_volume.t:1217-1222, 200-245).  wLp/wRp are modified.
 // HLLD and the HD HLLC form the physical flux themselves, of the side of the
 // contact that the face lies in.
-template <class T, bool MHD, int NDIR, bool GLM, int NDIM, int SOLVER, int BS, bool FAST = false>
+template <class T, bool MHD, int NDIR, bool GLM, int NDIM, int SOLVER, int BS, int FAST = 0>
 __device__ __forceinline__ uint32_t face_from_states(T *wLp, T *wRp, const PhysParams &P, T cg, T *F,
                                                      bool small_check = true) {
   constexpr int D = 0;  // states arrive rotated: the face normal is component 0
@@ -519,7 +549,7 @@ struct FaceFlux64 {
   uint32_t st;
 };
 
-template <class TF, bool MHD, int NDIR, bool GLM, int NDIM, int SOLVER, int LIM, int BS, int VS, bool FAST>
+template <class TF, bool MHD, int NDIR, bool GLM, int NDIM, int SOLVER, int LIM, int BS, int VS, int FAST>
 __device__ __noinline__ FaceFlux64<Vars<MHD, NDIR, GLM>::NW> face_retry_fp64(const TF *smem, int D, int b0, int b1,
                                                                             int b2, int b3, double rd, double cg,
                                                                             const PhysParams P) {
@@ -739,7 +769,7 @@ __global__ void __launch_bounds__(StageOcc<TF, MHD, NDIM, LIM, BN, VAR>::THREADS
   // root (physics.cuh: unguarded Newton in FP64, the hardware approximations
   // in the mixed form's FP32); a face whose flux is not finite is recomputed
   // in FP64 with the guarded forms in the fix-up pass after its phase.
-  constexpr bool FASTF = !(LIM == LIM_MP5 || LIM == LIM_WENO5 || LIM == LIM_WENO3 || LIM == LIM_VENK);
+  constexpr int FASTF = !(LIM == LIM_MP5 || LIM == LIM_WENO5 || LIM == LIM_WENO3 || LIM == LIM_VENK);
   constexpr bool RETRY = !FP64 || FASTF;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   TF *smem = reinterpret_cast<TF *>(smem_raw);
@@ -747,6 +777,8 @@ __global__ void __launch_bounds__(StageOcc<TF, MHD, NDIM, LIM, BN, VAR>::THREADS
   constexpr int VS = TileT::VS;
   TileView<TF, NW, NDIM, HW, TB> tv(smem);
   const int t = threadIdx.x;
+  pdl_wait();
+  pdl_trigger();
   // Work: global tile-planes g = (block*NT + tile)*PL + k (PL = BN in 3-D,
   // 1 in 2-D).  zchunk > 0: one z-chunk of one tile column per CTA.
   // zchunk == 0: persistent plane ranges — the grid is one wave of CTAs,

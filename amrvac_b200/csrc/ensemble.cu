@@ -27,6 +27,7 @@
 #include <cstring>
 #include <numeric>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "../../include/amrvac_gpu.h"
@@ -60,6 +61,56 @@ struct EnsRow {
   double dxinv[2];
 };
 
+struct EnsTime {
+  int ninst;
+  unsigned long long *red;
+  double *dt, *time;
+  const double *time_max;
+  int *done, *steps;
+  uint32_t *inst_status, *status;
+  double courantpar, dtmin;
+  int advance;  // also move the instances' time and step count on
+};
+
+// setdt of instance i (src/mod_dt.t:30-79) and the exit test of the time loop
+// (src/amrvac.t:306: global_time >= time_max or final_dt_exit); with advance
+// the time update of the step that follows (nothing reads it in between).
+__device__ __forceinline__ void ens_finalize(const EnsTime &T, int i) {
+  const double x = __longlong_as_double((long long)__ldcg(T.red + i));
+  T.red[i] = 0ull;
+  if (T.done[i]) { T.dt[i] = 0.0; return; }
+  // An instance whose last step produced a non-finite density or energy (or
+  // a small-value error) stops here with that status; the others go on.
+  const uint32_t ist = __ldcg(T.inst_status + i);
+  if (ist & (ST_SMALL_VALUE | ST_NAN)) {
+    atomicOr(T.status, ist);
+    T.done[i] = 1;
+    T.dt[i] = 0.0;
+    return;
+  }
+  double d = 1.0e99;
+  if (x > 1.0e-12) d = fmin(d, T.courantpar / x);
+  const double t = T.time[i], tmax = T.time_max[i];
+  if (d < T.dtmin) {  // crash: this instance stops
+    T.inst_status[i] |= ST_DT_TOO_SMALL;
+    atomicOr(T.status, ST_DT_TOO_SMALL);
+    T.done[i] = 1;
+    T.dt[i] = 0.0;
+    return;
+  }
+  if (tmax - t <= T.dtmin || t >= tmax) {
+    T.done[i] = 1;
+    T.dt[i] = 0.0;
+    return;
+  }
+  const double dt = fmin(d, tmax - t);
+  T.dt[i] = dt;
+  if (T.advance) {
+    T.time[i] = t + dt;
+    T.steps[i] += 1;
+  }
+}
+
 // Fill the per-row table of a tile (threads 0..15); returns, for all
 // threads, whether any row of the tile is active.
 template <int ND>
@@ -91,13 +142,14 @@ __device__ __forceinline__ bool ens_rows(const EnsArgs &A, int tile, bool for_ge
   return __syncthreads_or(act) != 0;
 }
 
-// The mixed form's FP32 faces use the hardware approximations (rcp.approx /
-// sqrt.approx, about one FP32 ulp) as the stage kernel's do; FP64 faces keep
-// the guarded division (this kernel has no recomputation pass).
-template <class TF, int ND, int SOLVER>
-__device__ __forceinline__ uint32_t ens_face(TF *wLp, TF *wRp, const PhysParams &P, TF *F) {
-  return face_from_states<TF, false, ND, false, ND, SOLVER, 0, sizeof(TF) == 4>(wLp, wRp, P, TF(0), F);
-}
+// Face arithmetic: FP32 (mixed form) with the hardware approximations
+// (rcp.approx / sqrt.approx, about one FP32 ulp); FP64 with the unguarded
+// reciprocal and quotient and the IEEE square root, which on operands in range
+// give the guarded forms' results bit for bit (an instance's thousands of
+// steps must not depend on which form ran); an FP64 face whose flux comes out
+// non-finite is recomputed with the guarded forms (ens_face_guarded).
+template <class TF>
+constexpr int ENS_FAST = sizeof(TF) == 8 ? FAST_DIV : FAST_ALL;
 
 // Stage kernel organisation: 288 threads.  Threads 0..255 own the cells of
 // the tile (ci = t % 16, row cj = t / 16) and compute the x-face and the
@@ -109,32 +161,17 @@ __device__ __forceinline__ uint32_t ens_face(TF *wLp, TF *wRp, const PhysParams 
 //   | barrier | all faces of both directions | barrier | accumulate + store.
 constexpr int ENS_THREADS = 288;
 
-// Shared tile of one buffer, in TF elements, for up to 4 variables.
+// Shared tile of one buffer, in TF elements, for up to 4 variables: per
+// variable the cells and halos (VS apart, so a face needs one address per
+// stencil cell), then per variable the scaled face fluxes of both directions.
 template <class TF>
 struct EnsTile {
   static constexpr int NWM = 4;
-  static constexpr int TOTAL = NWM * (BN16 * BN16 + BN16 * 4 + 4 * BN16 + 2 * (BN16 + 1) * BN16);
-};
-
-template <class TF, int NW>
-struct EnsView {
-  TF *ring, *hx, *hy, *fbx, *fby;  // [v][j][i], [v][j][c], [v][r][i], [v][j][17], [v][17][i]
-  __device__ __forceinline__ explicit EnsView(TF *s) {
-    ring = s;
-    hx = ring + NW * BN16 * BN16;
-    hy = hx + NW * BN16 * 4;
-    fbx = hy + NW * 4 * BN16;
-    fby = fbx + NW * (BN16 + 1) * BN16;
-  }
-  // element offset of variable 0 at (i, j) in [-2, 17] x [0, 15] or [0, 15] x [-2, 17],
-  // and the stride between variables
-  __device__ __forceinline__ void addr(int i, int j, int &base, int &stride) const {
-    const bool ii = (unsigned)i < (unsigned)BN16;
-    const bool jj = (unsigned)j < (unsigned)BN16;
-    if (ii && jj) { base = j * BN16 + i; stride = BN16 * BN16; }
-    else if (jj) { base = NW * BN16 * BN16 + j * 4 + halo_slot_w<2>(i); stride = BN16 * 4; }
-    else { base = NW * BN16 * BN16 + NW * BN16 * 4 + halo_slot_w<2>(j) * BN16 + i; stride = 4 * BN16; }
-  }
+  static constexpr int OX = BN16 * BN16;         // x halo [j][c]
+  static constexpr int OY = OX + BN16 * 4;       // y halo [r][i]
+  static constexpr int VS = OY + 4 * BN16;       // one variable
+  static constexpr int FB = (BN16 + 1) * BN16;   // faces of one direction
+  static constexpr int TOTAL = NWM * (VS + 2 * FB);
 };
 
 // Row table entry of one row of a tile (2-D tile: the block, all rows alike).
@@ -158,43 +195,84 @@ __device__ __forceinline__ void ens_fill_row(const EnsArgs &A, int tile, bool tw
   }
 }
 
+// Riemann flux of one face from its four stencil cells (shared-memory offsets
+// base[o], component c of the vectors rot[c] further): limited reconstruction
+// and the row's solver.  The limiters of the usual schemes are compiled in,
+// chosen once per face; the others switch per slope.
+template <class TF, int ND, int FAST>
+__device__ __forceinline__ uint32_t ens_face_flux(const TF *s, const int *base, const int *rot, int lim, int solver,
+                                                  TF rd, const PhysParams &P, TF *F) {
+  constexpr int NW = ND + 2, VS = EnsTile<TF>::VS;
+  TF wL[NW], wR[NW];
+  bool special = false;
+  auto states = [&](auto limc) {
+    constexpr int LIM = decltype(limc)::value;
+#pragma unroll
+    for (int v = 0; v < NW; ++v) {
+      const int vo = v >= 1 && v <= ND ? VS + rot[v - 1] : v * VS;
+      face_states<TF, LIM, FAST>(lim, s[base[0] + vo], s[base[1] + vo], s[base[2] + vo], s[base[3] + vo], rd, wL[v],
+                                 wR[v], special);
+    }
+  };
+  if (lim == LIM_VANLEER) states(std::integral_constant<int, LIM_VANLEER>());
+  else if (lim == LIM_MINMOD) states(std::integral_constant<int, LIM_MINMOD>());
+  else states(std::integral_constant<int, 0>());
+  if (solver == SOLVER_HLLC)
+    return face_from_states<TF, false, ND, false, ND, SOLVER_HLLC, 0, FAST>(wL, wR, P, TF(0), F);
+  if (solver == SOLVER_HLL) return face_from_states<TF, false, ND, false, ND, SOLVER_HLL, 0, FAST>(wL, wR, P, TF(0), F);
+  return face_from_states<TF, false, ND, false, ND, SOLVER_TVDLF, 0, FAST>(wL, wR, P, TF(0), F);
+}
+
+// The same with the guarded forms, out of line (a face that met a special
+// operand: zero, subnormal, infinite or NaN).
+template <int ND>
+__device__ __noinline__ FaceFlux64<ND + 2> ens_face_guarded(const double *s, int b0, int b1, int b2, int b3, int D,
+                                                            int lim, int solver, double rd, const PhysParams *P) {
+  const int base[4] = {b0, b1, b2, b3};
+  const int rot[2] = {D * EnsTile<double>::VS, (1 - D) * EnsTile<double>::VS};
+  FaceFlux64<ND + 2> r;
+  r.st = ens_face_flux<double, ND, FAST_NONE>(s, base, rot, lim, solver, rd, *P, r.F);
+  return r;
+}
+
 // One face of direction D (run-time, so one copy of the face code serves
-// both directions and all call sites) at face coordinates (fi, fj): limited
-// reconstruction from the staged primitives, Riemann flux, store to fb.
+// both directions and all call sites) at face coordinates (fi, fj), stored
+// rotated (entry v is variable orig_index<D>(v)).
 template <class TF, int ND>
-__device__ __forceinline__ uint32_t ens_face_at(const TF *s, const EnsView<TF, ND + 2> &tv, const EnsRow &Rf,
-                                                const PhysParams &P, int D, int fi, int fj) {
+__device__ __forceinline__ uint32_t ens_face_at(TF *s, const EnsRow &Rf, const PhysParams &P, int D, int fi, int fj) {
+  using T = EnsTile<TF>;
   constexpr int NW = ND + 2;
-  constexpr int FB = (BN16 + 1) * BN16;
   constexpr bool FP64 = sizeof(TF) == 8;
   const TF rd = TF(D == 0 ? Rf.rd[0] : Rf.rd[ND - 1]);
-  const int lim = Rf.limiter;
-  TF wLp[NW], wRp[NW];
-  int base[4], strd[4];
+  int base[4];
+  {
+    const int c0 = (D == 0 ? fi : fj) - 2, step = D == 0 ? 1 : BN16;
+    const int cen = fj * BN16 + fi - 2 * step, hb = D == 0 ? T::OX + fj * 4 : T::OY + fi;
 #pragma unroll
-  for (int o = 0; o < 4; ++o) tv.addr(D == 0 ? fi + o - 2 : fi, D == 0 ? fj : fj + o - 2, base[o], strd[o]);
-#pragma unroll
-  for (int v = 0; v < NW; ++v) {
-    const int ov = orig_index_rt<false, ND>(v, D);
-    TF q[4];
-#pragma unroll
-    for (int o = 0; o < 4; ++o) q[o] = s[base[o] + ov * strd[o]];
-    bool special = false;
-    face_states<TF, 0, sizeof(TF) == 4>(lim, q[0], q[1], q[2], q[3], rd, wLp[v], wRp[v], special);
+    for (int o = 0; o < 4; ++o)
+      base[o] = (unsigned)(c0 + o) < (unsigned)BN16 ? cen + o * step : hb + halo_slot_w<2>(c0 + o) * step;
   }
+  const int rot[2] = {D * T::VS, (1 - D) * T::VS};
   TF Fr[NW];
-  uint32_t st;
-  if (Rf.solver == SOLVER_HLLC) st = ens_face<TF, ND, SOLVER_HLLC>(wLp, wRp, P, Fr);
-  else if (Rf.solver == SOLVER_HLL) st = ens_face<TF, ND, SOLVER_HLL>(wLp, wRp, P, Fr);
-  else st = ens_face<TF, ND, SOLVER_TVDLF>(wLp, wRp, P, Fr);
-  TF *fb = D == 0 ? tv.fbx : tv.fby;
-  const int f = D == 0 ? fj * (BN16 + 1) + fi : fj * BN16 + fi;
+  uint32_t st = ens_face_flux<TF, ND, ENS_FAST<TF>>(s, base, rot, Rf.limiter, Rf.solver, rd, P, Fr);
+  if constexpr (FP64) {
+    double sum = Fr[0];
+#pragma unroll
+    for (int v = 1; v < NW; ++v) sum = sum + Fr[v];
+    if (!isfinite(sum)) {
+      const FaceFlux64<NW> g =
+          ens_face_guarded<ND>(s, base[0], base[1], base[2], base[3], D, Rf.limiter, Rf.solver, rd, &P);
+      st |= g.st;
+#pragma unroll
+      for (int v = 0; v < NW; ++v) Fr[v] = g.F[v];
+    }
+  }
+  TF *fb = s + NW * T::VS + D * T::FB + (D == 0 ? fj * (BN16 + 1) + fi : fj * BN16 + fi);
   const double sc = D == 0 ? Rf.sc[0] : Rf.sc[ND - 1];
 #pragma unroll
   for (int v = 0; v < NW; ++v) {
-    const int ov = orig_index_rt<false, ND>(v, D);
-    if constexpr (FP64) fb[ov * FB + f] = sc * Fr[v];
-    else fb[ov * FB + f] = Fr[v];
+    if constexpr (FP64) fb[v * (2 * T::FB)] = sc * Fr[v];
+    else fb[v * (2 * T::FB)] = Fr[v];
   }
   return st;
 }
@@ -206,7 +284,8 @@ __device__ __forceinline__ uint32_t ens_stage_tile(const EnsArgs &A, TF *s, cons
                                                    int next, int nt, int n2) {
   using V = Vars<false, ND, false>;
   constexpr int NW = V::NW;
-  constexpr int FB = (BN16 + 1) * BN16;
+  using T = EnsTile<TF>;
+  constexpr int VS = T::VS;
   constexpr bool FP64 = sizeof(TF) == 8;
   const StageArgs &S = A.sa[ND - 1];
   const PhysParams &P = S.P;
@@ -215,7 +294,6 @@ __device__ __forceinline__ uint32_t ens_stage_tile(const EnsArgs &A, TF *s, cons
   const int ci = t & (BN16 - 1), cj = (t >> 4) & (BN16 - 1);
   const int lane = t - BN16 * BN16;  // ninth warp: 0..31
   uint32_t st = 0;
-  EnsView<TF, NW> tv(s);
   const EnsRow &R = cur[ND == 2 ? 0 : cj];
   const bool active = cell_thread && R.inst >= 0;
   const int cjj = ND == 2 ? cj : 0;
@@ -227,25 +305,22 @@ __device__ __forceinline__ uint32_t ens_stage_tile(const EnsArgs &A, TF *s, cons
     double w[NW];
     st |= load_prim<false, ND, false, ND>(S, R.blk, ci, cjj, 0, w);
 #pragma unroll
-    for (int v = 0; v < NW; ++v) tv.ring[v * BN16 * BN16 + cj * BN16 + ci] = TF(w[v]);
+    for (int v = 0; v < NW; ++v) s[v * VS + cj * BN16 + ci] = TF(w[v]);
   }
   if (t < (ND == 2 ? 128 : 64)) {
     int i, j, row;
     TF *dst;
-    int stride;
     if (t < 64) {
       j = t >> 2;
       const int c = t & 3;
       i = c < 2 ? c - 2 : c + BN16 - 2;
-      dst = tv.hx + j * 4 + c;
-      stride = BN16 * 4;
+      dst = s + T::OX + j * 4 + c;
       row = ND == 2 ? 0 : j;
     } else {
       const int r = (t - 64) >> 4;
       i = (t - 64) & (BN16 - 1);
       j = r < 2 ? r - 2 : r + BN16 - 2;
-      dst = tv.hy + r * BN16 + i;
-      stride = 4 * BN16;
+      dst = s + T::OY + r * BN16 + i;
       row = 0;
     }
     const EnsRow &H = cur[row];
@@ -253,7 +328,7 @@ __device__ __forceinline__ uint32_t ens_stage_tile(const EnsArgs &A, TF *s, cons
       double w[NW];
       st |= load_prim<false, ND, false, ND>(S, H.blk, i, ND == 2 ? j : 0, 0, w);
 #pragma unroll
-      for (int v = 0; v < NW; ++v) dst[v * stride] = TF(w[v]);
+      for (int v = 0; v < NW; ++v) dst[v * VS] = TF(w[v]);
     }
   }
   double acc[NW];
@@ -286,21 +361,22 @@ __device__ __forceinline__ uint32_t ens_stage_tile(const EnsArgs &A, TF *s, cons
     }
 #pragma unroll 1
     for (int q = 0; q < nf; ++q)
-      st |= ens_face_at<TF, ND>(s, tv, *rf, P, q == 0 ? fd0 : 1, q == 0 ? fi0 : fi1, q == 0 ? fj0 : fj1);
+      st |= ens_face_at<TF, ND>(s, *rf, P, q == 0 ? fd0 : 1, q == 0 ? fi0 : fi1, q == 0 ? fj0 : fj1);
   }
   __syncthreads();
   // ---- flux divergence in direction order, small values, store
   if (active) {
 #pragma unroll
     for (int D = 0; D < ND; ++D) {
-      const TF *fb = D == 0 ? tv.fbx : tv.fby;
-      const int f = D == 0 ? cj * (BN16 + 1) + ci : cj * BN16 + ci;
+      const TF *fb = s + NW * VS + D * T::FB + (D == 0 ? cj * (BN16 + 1) + ci : cj * BN16 + ci);
       const int step = D == 0 ? 1 : BN16;
       const double sc = FP64 ? 1.0 : R.sc[D];
 #pragma unroll
       for (int v = 0; v < NW; ++v) {
-        if constexpr (FP64) acc[v] = acc[v] + fb[v * FB + f + step] - fb[v * FB + f];
-        else acc[v] = acc[v] + sc * double(fb[v * FB + f + step]) - sc * double(fb[v * FB + f]);
+        double &a = acc[D == 0 ? orig_index<false, ND, 0>(v) : orig_index<false, ND, ND - 1>(v)];
+        const TF hi = fb[v * (2 * T::FB) + step], lo = fb[v * (2 * T::FB)];
+        if constexpr (FP64) a = a + hi - lo;
+        else a = a + sc * double(hi) - sc * double(lo);
       }
     }
     if (P.fix_small_values) {
@@ -321,6 +397,8 @@ __device__ __forceinline__ void ens_stage_body(const EnsArgs &A) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   TF *sm = reinterpret_cast<TF *>(smem_raw);
   __shared__ EnsRow rows[3][ENS_ROWS];
+  pdl_wait();
+  pdl_trigger();
   const int n2 = A.ntiles[0], nt = A.ntiles[1];
   int tile = blockIdx.x;
   if (tile >= nt) return;
@@ -351,12 +429,12 @@ __device__ __forceinline__ void ens_stage_body(const EnsArgs &A) {
 // Denser variants, which the autotuner times against the first kernel of a
 // form: FP64 at three CTAs per SM (72 registers, a few spilled) and four (56),
 // mixed at four (56 registers) and five (40).
-__global__ void __launch_bounds__(ENS_THREADS, 2) ens_stage_kernel_fp64(const EnsArgs A) { ens_stage_body<double>(A); }
-__global__ void __launch_bounds__(ENS_THREADS, 3) ens_stage_kernel_fp64_3(const EnsArgs A) { ens_stage_body<double>(A); }
-__global__ void __launch_bounds__(ENS_THREADS, 4) ens_stage_kernel_fp64_4(const EnsArgs A) { ens_stage_body<double>(A); }
-__global__ void __launch_bounds__(ENS_THREADS, 3) ens_stage_kernel_mixed(const EnsArgs A) { ens_stage_body<float>(A); }
-__global__ void __launch_bounds__(ENS_THREADS, 4) ens_stage_kernel_mixed_4(const EnsArgs A) { ens_stage_body<float>(A); }
-__global__ void __launch_bounds__(ENS_THREADS, 5) ens_stage_kernel_mixed_5(const EnsArgs A) { ens_stage_body<float>(A); }
+__global__ void __launch_bounds__(ENS_THREADS, 2) ens_stage_kernel_fp64(const __grid_constant__ EnsArgs A) { ens_stage_body<double>(A); }
+__global__ void __launch_bounds__(ENS_THREADS, 3) ens_stage_kernel_fp64_3(const __grid_constant__ EnsArgs A) { ens_stage_body<double>(A); }
+__global__ void __launch_bounds__(ENS_THREADS, 4) ens_stage_kernel_fp64_4(const __grid_constant__ EnsArgs A) { ens_stage_body<double>(A); }
+__global__ void __launch_bounds__(ENS_THREADS, 3) ens_stage_kernel_mixed(const __grid_constant__ EnsArgs A) { ens_stage_body<float>(A); }
+__global__ void __launch_bounds__(ENS_THREADS, 4) ens_stage_kernel_mixed_4(const __grid_constant__ EnsArgs A) { ens_stage_body<float>(A); }
+__global__ void __launch_bounds__(ENS_THREADS, 5) ens_stage_kernel_mixed_5(const __grid_constant__ EnsArgs A) { ens_stage_body<float>(A); }
 
 // the stage kernel of (precision, variant); variant v is capped for
 // ens_variant_ctas(mixed, v) CTAs per SM
@@ -385,7 +463,7 @@ __device__ __forceinline__ void ens_getdt_tile(const EnsArgs &A, int tile, EnsRo
   if (R.inst >= 0) {
     double w[NW];
 #pragma unroll
-    for (int v = 0; v < NW; ++v) w[v] = __ldg(S.uin + cell_offset<ND>(R.blk, NW, v, ci, ND == 2 ? cj : 0, 0));
+    for (int v = 0; v < NW; ++v) w[v] = S.uin[cell_offset<ND>(R.blk, NW, v, ci, ND == 2 ? cj : 0, 0)];
     // phys_to_primitive with its small-value fix (src/mod_dt.t:189-191)
     if (S.P.fix_small_values) {
       if (small_values<double, false, ND, false>(w, false, S.P) && S.P.small_values_method != 1)
@@ -416,66 +494,34 @@ __device__ __forceinline__ void ens_getdt_tile(const EnsArgs &A, int tile, EnsRo
   __syncthreads();
 }
 
-__global__ void __launch_bounds__(STAGE_THREADS) ens_getdt_kernel(const EnsArgs A) {
+// getdt of every active instance; the last CTA to finish (counted in *ticket)
+// then finalizes all instances, one per thread.
+struct EnsGetdt {
+  EnsArgs A;
+  EnsTime T;
+  unsigned *ticket;
+};
+__global__ void __launch_bounds__(STAGE_THREADS) ens_getdt_kernel(const __grid_constant__ EnsGetdt G) {
   __shared__ EnsRow rows[ENS_ROWS];
   __shared__ double wred[ENS_ROWS];
+  __shared__ int s_last;
+  pdl_wait();
+  pdl_trigger();
+  const EnsArgs &A = G.A;
   const int n2 = A.ntiles[0], nt = A.ntiles[1];
 #pragma unroll 1
   for (int tile = blockIdx.x; tile < nt; tile += gridDim.x) {
     if (tile < n2) ens_getdt_tile<2>(A, tile, rows, wred);
     else ens_getdt_tile<1>(A, tile, rows, wred);
   }
-}
-
-struct EnsTime {
-  int ninst;
-  unsigned long long *red;
-  double *dt, *time;
-  const double *time_max;
-  int *done, *steps;
-  uint32_t *inst_status, *status;
-  double courantpar, dtmin;
-};
-
-// setdt per instance (src/mod_dt.t:30-79) and the exit test of the time loop
-// (src/amrvac.t:306: global_time >= time_max or final_dt_exit).
-__global__ void ens_finalize_kernel(const EnsTime T) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= T.ninst) return;
-  const double x = __longlong_as_double((long long)T.red[i]);
-  T.red[i] = 0ull;
-  if (T.done[i]) { T.dt[i] = 0.0; return; }
-  // An instance whose last step produced a non-finite density or energy (or
-  // a small-value error) stops here with that status; the others go on.
-  if (T.inst_status[i] & (ST_SMALL_VALUE | ST_NAN)) {
-    atomicOr(T.status, T.inst_status[i]);
-    T.done[i] = 1;
-    T.dt[i] = 0.0;
-    return;
-  }
-  double d = 1.0e99;
-  if (x > 1.0e-12) d = fmin(d, T.courantpar / x);
-  const double t = T.time[i], tmax = T.time_max[i];
-  if (d < T.dtmin) {  // crash: this instance stops
-    T.inst_status[i] |= ST_DT_TOO_SMALL;
-    atomicOr(T.status, ST_DT_TOO_SMALL);
-    T.done[i] = 1;
-    T.dt[i] = 0.0;
-    return;
-  }
-  if (tmax - t <= T.dtmin || t >= tmax) {
-    T.done[i] = 1;
-    T.dt[i] = 0.0;
-    return;
-  }
-  T.dt[i] = fmin(d, tmax - t);
-}
-
-__global__ void ens_advance_kernel(const EnsTime T) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= T.ninst || T.done[i]) return;
-  T.time[i] = T.time[i] + T.dt[i];
-  T.steps[i] += 1;
+  __threadfence();  // this thread's maxima before the ticket
+  __syncthreads();
+  if (threadIdx.x == 0) s_last = atomicAdd(G.ticket, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  if (threadIdx.x == 0) *G.ticket = 0u;
+  for (int i = threadIdx.x; i < G.T.ninst; i += blockDim.x) ens_finalize(G.T, i);
 }
 
 }  // namespace amrvac
@@ -502,6 +548,8 @@ struct amrvac_ens {
   double *d_dt = nullptr, *d_time = nullptr, *d_tmax = nullptr, *d_dx = nullptr;
   int *d_solver = nullptr, *d_limiter = nullptr, *d_done = nullptr, *d_steps = nullptr;
   unsigned long long *d_red = nullptr;
+  unsigned *d_ticket = nullptr;              // CTAs of the getdt kernel that have finished
+  bool chained = false;                      // the last launch lets the next one be dependent on it
   uint32_t *d_status = nullptr, *d_inst_status = nullptr;
   double *d_stage = nullptr;
   size_t stage_doubles = 0;
@@ -578,26 +626,36 @@ EnsTime ens_time(amrvac_ens *e) {
   T.status = e->d_status;
   T.courantpar = e->cfg.courantpar;
   T.dtmin = e->cfg.dtmin;
+  T.advance = 0;
   return T;
 }
 
 int ens_launch_stage(amrvac_ens *e, int reg_ct, int reg_new, int reg_base, double a, double b, double dtf) {
   const EnsArgs A = ens_args(e, reg_ct, reg_new, reg_base, a, b, dtf);
-  ens_stage_fn(e->mixed, e->var)<<<e->grid, ENS_THREADS, ens_smem(e->mixed), e->stream>>>(A);
-  ECK(cudaGetLastError());
+  ECK(launch_dependent<EnsArgs>(ens_stage_fn(e->mixed, e->var), e->grid, ENS_THREADS, ens_smem(e->mixed), e->stream,
+                                e->chained, A));
   ++e->launches;
   return 0;
 }
 
-int ens_launch_step(amrvac_ens *e) {
-  const EnsArgs G = ens_args(e, 0, 0, 0, 0.0, 1.0, 1.0);
-  ens_getdt_kernel<<<e->grid, STAGE_THREADS, 0, e->stream>>>(G);
-  ECK(cudaGetLastError());
-  const EnsTime T = ens_time(e);
-  const int nb = (e->ninst + 127) / 128;
-  ens_finalize_kernel<<<nb, 128, 0, e->stream>>>(T);
-  ECK(cudaGetLastError());
-  e->launches += 2;
+int ens_launch_getdt(amrvac_ens *e, bool advance) {
+  EnsGetdt G;
+  G.A = ens_args(e, 0, 0, 0, 0.0, 1.0, 1.0);
+  G.T = ens_time(e);
+  G.T.advance = advance;
+  G.ticket = e->d_ticket;
+  ECK(launch_dependent<EnsGetdt>(&ens_getdt_kernel, e->grid, STAGE_THREADS, 0, e->stream, e->chained, G));
+  ++e->launches;
+  return 0;
+}
+
+// One step: getdt with setdt and the time update in one kernel, then the
+// stages, each launched dependent on the one before (first: the step's first
+// launch starts a chain, as nothing may be known of what is on the stream).
+int ens_launch_step(amrvac_ens *e, bool first) {
+  e->chained = !first;
+  if (int q = ens_launch_getdt(e, true)) return q;
+  e->chained = true;
   const amrvac_cfg &k = e->cfg;
   int r = 0;
   if (k.time_stepper == AMRVAC_TS_ONESTEP) {
@@ -605,6 +663,7 @@ int ens_launch_step(amrvac_ens *e) {
       if (e->nb[p])
         ECK(cudaMemcpyAsync(e->pool[p][1], e->pool[p][0], sizeof(double) * (size_t)e->nb[p] * (p ? 4 * 256 : 3 * 16),
                             cudaMemcpyDeviceToDevice, e->stream));
+    e->chained = false;
     r = ens_launch_stage(e, 1, 0, 0, 0.0, 1.0, 1.0);
   } else if (k.time_stepper == AMRVAC_TS_TWOSTEP) {
     if ((r = ens_launch_stage(e, 0, 1, 0, 0.0, 1.0, 1.0))) return r;
@@ -617,11 +676,8 @@ int ens_launch_step(amrvac_ens *e) {
     if ((r = ens_launch_stage(e, 1, 2, 0, a21, 1.0 - a21, b22))) return r;
     r = ens_launch_stage(e, 2, 0, 0, a31, 1.0 - a31, b33);
   }
-  if (r) return r;
-  ens_advance_kernel<<<nb, 128, 0, e->stream>>>(T);
-  ECK(cudaGetLastError());
-  ++e->launches;
-  return 0;
+  e->chained = false;
+  return r;
 }
 
 // Upload the tile list of the instances not yet done (done == nullptr: all).
@@ -688,7 +744,7 @@ void free_all(amrvac_ens *e) {
   cudaFree(e->d_tiles); cudaFree(e->d_ntiles);
   cudaFree(e->d_dt); cudaFree(e->d_time); cudaFree(e->d_tmax); cudaFree(e->d_dx);
   cudaFree(e->d_solver); cudaFree(e->d_limiter); cudaFree(e->d_done); cudaFree(e->d_steps);
-  cudaFree(e->d_red); cudaFree(e->d_status); cudaFree(e->d_inst_status); cudaFree(e->d_stage);
+  cudaFree(e->d_red); cudaFree(e->d_ticket); cudaFree(e->d_status); cudaFree(e->d_inst_status); cudaFree(e->d_stage);
   if (e->h_pin) cudaFreeHost(e->h_pin);
   if (e->stream) cudaStreamDestroy(e->stream);
 }
@@ -859,6 +915,7 @@ int amrvac_ens_create(const amrvac_cfg *cfg, int ninst, const amrvac_ens_instanc
   EALLOC(e->d_done, sizeof(int) * ninst);
   EALLOC(e->d_steps, sizeof(int) * ninst);
   EALLOC(e->d_red, sizeof(unsigned long long) * ninst);
+  EALLOC(e->d_ticket, sizeof(unsigned));
   EALLOC(e->d_status, sizeof(uint32_t));
   EALLOC(e->d_inst_status, sizeof(uint32_t) * ninst);
 #undef EALLOC
@@ -891,6 +948,7 @@ int amrvac_ens_create(const amrvac_cfg *cfg, int ninst, const amrvac_ens_instanc
       (ce = cudaMemcpy(e->d_solver, solver.data(), sizeof(int) * ninst, cudaMemcpyHostToDevice)) ||
       (ce = cudaMemcpy(e->d_limiter, lim.data(), sizeof(int) * ninst, cudaMemcpyHostToDevice)) ||
       (ce = cudaMemset(e->d_red, 0, sizeof(unsigned long long) * ninst)) ||
+      (ce = cudaMemset(e->d_ticket, 0, sizeof(unsigned))) ||
       (ce = cudaMemset(e->d_status, 0, sizeof(uint32_t))))
     return fail_free(ce, "cudaMemcpy(instances)");
   for (int p = 0; p < 2; ++p)
@@ -980,7 +1038,7 @@ int amrvac_ens_download(amrvac_ens *e, int inst, double *w) {
 
 int amrvac_ens_step(amrvac_ens *e) {
   if (int r = check_ens(e)) return r;
-  return ens_launch_step(e);
+  return ens_launch_step(e, true);
 }
 
 int amrvac_ens_run(amrvac_ens *e, int max_steps, int chunk, int *steps_taken, int *nactive) {
@@ -996,7 +1054,7 @@ int amrvac_ens_run(amrvac_ens *e, int max_steps, int chunk, int *steps_taken, in
     const int64_t before = e->launches;
     ECK(cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeThreadLocal));
     int r = 0;
-    for (int s = 0; s < chunk && !r; ++s) r = ens_launch_step(e);
+    for (int s = 0; s < chunk && !r; ++s) r = ens_launch_step(e, s == 0);
     cudaError_t ce = cudaStreamEndCapture(e->stream, &g);
     e->launches = before;
     if (r) { if (ce == cudaSuccess) cudaGraphDestroy(g); return r; }
@@ -1006,7 +1064,7 @@ int amrvac_ens_run(amrvac_ens *e, int max_steps, int chunk, int *steps_taken, in
     if (ce != cudaSuccess) { e->graph = nullptr; return ecuda(ce, "cudaGraphInstantiate"); }
     e->graph_steps = chunk;
   }
-  const int per_step = 3 + e->cfg.time_stepper;
+  const int per_step = 1 + e->cfg.time_stepper;
   int taken = 0, act = e->ninst;
   e->h_done.assign(e->ninst, 0);
   int ndone_prev = 0;
@@ -1095,13 +1153,9 @@ int amrvac_ens_autotune(amrvac_ens *e, int reps, int *best_ctas, double *best_ms
   if (int r = check_ens(e)) return r;
   if (reps <= 0) reps = 5;
   // dt of the current state, as the stages read it
-  const EnsArgs G = ens_args(e, 0, 0, 0, 0.0, 1.0, 1.0);
-  ens_getdt_kernel<<<e->grid, STAGE_THREADS, 0, e->stream>>>(G);
-  const EnsTime T = ens_time(e);
   std::vector<int> done_save(e->ninst);
   ECK(cudaMemcpyAsync(done_save.data(), e->d_done, sizeof(int) * e->ninst, cudaMemcpyDeviceToHost, e->stream));
-  ens_finalize_kernel<<<(e->ninst + 127) / 128, 128, 0, e->stream>>>(T);
-  ECK(cudaGetLastError());
+  if (int r = ens_launch_getdt(e, false)) return r;
   ECK(cudaStreamSynchronize(e->stream));
   cudaEvent_t a, b;
   ECK(cudaEventCreate(&a));

@@ -47,7 +47,7 @@ constexpr size_t ADJ_SMEM = sizeof(double) * (SM_WP + SM_LM + SM_G);
 
 // Partial derivatives of the limited slope (a: forward difference, b:
 // backward difference), on the branch of the forward value.
-template <int LIM>
+template <int LIM, int FAST>
 __device__ __forceinline__ void slope_partials(double a, double b, double &da, double &db) {
   if constexpr (LIM == LIM_MINMOD) {
     const double t = copysign(1.0, a);
@@ -61,8 +61,8 @@ __device__ __forceinline__ void slope_partials(double a, double b, double &da, d
     }
   } else {  // vanleer: 2*max(b*a, 0) / (a + b + qsmall)
     if (b * a >= 0.0) {
-      const double den = a + b + 1.0e-12, iden = rcp_(den);
-      const double s = div_(2.0 * fmax(b * a, 0.0), den);
+      const double den = a + b + 1.0e-12, iden = rcp_f<FAST>(den);
+      const double s = div_f<FAST>(2.0 * fmax(b * a, 0.0), den);
       da = (2.0 * b - s) * iden;
       db = (2.0 * a - s) * iden;
     } else {
@@ -73,6 +73,7 @@ __device__ __forceinline__ void slope_partials(double a, double b, double &da, d
 }
 
 // Reverse of the HLL flux (src/mod_finite_volume.t:381-437) for one face.
+template <int FAST>
 __device__ __forceinline__ void hll_reverse(const double *cL, const double *cR, const double *fL, const double *fR,
                                             double cmin, double cmax, const double *mu, double *fLb, double *fRb,
                                             double *cLb, double *cRb, double &cmaxb, double &cminb) {
@@ -86,7 +87,7 @@ __device__ __forceinline__ void hll_reverse(const double *cL, const double *cR, 
     for (int v = 0; v < 4; ++v) fRb[v] = mu[v];
     return;
   }
-  const double iD = rcp_(cmax - cmin);
+  const double iD = rcp_f<FAST>(cmax - cmin);
 #pragma unroll
   for (int v = 0; v < 4; ++v) {
     const double dW = cR[v] - cL[v];
@@ -105,18 +106,19 @@ __device__ __forceinline__ void hll_reverse(const double *cL, const double *cR, 
 // 439-504, with hd_get_lCD / hd_get_wCD, src/hd/mod_hd_hllc.t:56-257): the
 // region (patchf) of the forward, then the star state of the upwind side.
 // Rotated variables: 0 rho, 1 normal momentum, 2 tangential momentum, 3 e.
+template <int FAST>
 __device__ __forceinline__ void hllc_reverse(const double *cL, const double *cR, const double *fL, const double *fR,
                                              double cmin, double cmax, const double *mu, double *fLb, double *fRb,
                                              double *cLb, double *cRb, double &cmaxb, double &cminb) {
   if (cmin >= 0.0 || cmax <= 0.0) {
-    hll_reverse(cL, cR, fL, fR, cmin, cmax, mu, fLb, fRb, cLb, cRb, cmaxb, cminb);
+    hll_reverse<FAST>(cL, cR, fL, fR, cmin, cmax, mu, fLb, fRb, cLb, cRb, cmaxb, cminb);
     return;
   }
-  const double Dn = cmax - cmin, iDn = rcp_(Dn);
+  const double Dn = cmax - cmin, iDn = rcp_f<FAST>(Dn);
   double whll[2];
 #pragma unroll
   for (int v = 0; v < 2; ++v) whll[v] = (cmax * cR[v] - cmin * cL[v] + fL[v] - fR[v]) * iDn;
-  const double iwh0 = rcp_(whll[0]);
+  const double iwh0 = rcp_f<FAST>(whll[0]);
   double lam = whll[1] * iwh0;
   int patchf = 1;
   bool cond = true;
@@ -125,16 +127,19 @@ __device__ __forceinline__ void hllc_reverse(const double *cL, const double *cR,
   else if (lam >= cmax || lam <= cmin) { lam = 0.0; patchf = 3; cond = false; }
   if (cond && lam == 0.0) patchf = (-cmin >= cmax) ? 1 : -1;
   if (patchf == 3) {  // the HLL flux Fhll
-    hll_reverse(cL, cR, fL, fR, cmin, cmax, mu, fLb, fRb, cLb, cRb, cmaxb, cminb);
+    hll_reverse<FAST>(cL, cR, fL, fR, cmin, cmax, mu, fLb, fRb, cLb, cRb, cmaxb, cminb);
     return;
   }
   const bool right = patchf == 1;
-  const double *wS = right ? cR : cL, *fS = right ? fR : fL;
-  double *wSb = right ? cRb : cLb, *fSb = right ? fRb : fLb;
+  // the side's values and its adjoints by value: pointers to either side would
+  // put all eight arrays in local memory
+  double wS[4], fS[4], wSb[4] = {0.0, 0.0, 0.0, 0.0}, fSb[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+  for (int v = 0; v < 4; ++v) { wS[v] = right ? cR[v] : cL[v]; fS[v] = right ? fR[v] : fL[v]; }
   const double cs = right ? cmax : cmin;
-  const double iw0 = rcp_(wS[0]);
+  const double iw0 = rcp_f<FAST>(wS[0]);
   const double vS = wS[1] * iw0;
-  const double csmls = rcp_(cs - lam);
+  const double csmls = rcp_f<FAST>(cs - lam);
   double wCD[4];
   wCD[0] = wS[0] * (cs - vS) * csmls;
   wCD[2] = (cs * wS[2] - fS[2]) * csmls;
@@ -207,6 +212,13 @@ __device__ __forceinline__ void hllc_reverse(const double *cL, const double *cR,
     cmaxb += b * (cR[v] - whll[v]);
     cminb += b * (whll[v] - cL[v]);
   }
+#pragma unroll
+  for (int v = 0; v < 4; ++v) {
+    cRb[v] += right ? wSb[v] : 0.0;
+    cLb[v] += right ? 0.0 : wSb[v];
+    fRb[v] += right ? fSb[v] : 0.0;
+    fLb[v] += right ? 0.0 : fSb[v];
+  }
   if (right) cmaxb += csb;
   else cminb += csb;
 }
@@ -214,25 +226,30 @@ __device__ __forceinline__ void hllc_reverse(const double *cL, const double *cR,
 // Vector-Jacobian product of one face flux.  wp: staged primitives; D: face
 // direction; fi: face index along D (-1..17, face fi lies between cells fi-1
 // and fi); row: the other coordinate; mu: dL/dF in rotated variable order
-// (1 = normal, 2 = tangential velocity).  Adds dL/d(primitive) of the four
-// stencil cells fi-2..fi+1 to gq (rotated order); returns dL/dgamma.
-template <int LIM, int SOLVER>
+// (1 = normal, 2 = tangential velocity).  Writes dL/d(primitive) of the four
+// stencil cells fi-2..fi+1 to the face's column of G; returns dL/dgamma, and
+// in sum a value that is finite if they all are.
+// FAST: the unguarded reciprocal, quotient and square root; a face whose
+// result is not finite is done again with the guarded ones (face_vjp_guarded).
+template <int LIM, int SOLVER, int FAST>
 __device__ __forceinline__ double face_vjp(const double *wp, int D, int fi, int row, const double *mu,
-                                           const PhysParams &P, double (&gq)[4][4]) {
-  auto at = [&](int o, int ov) -> double {
-    const int pos = fi - 2 + o;
-    const int x = D == 0 ? pos : row, y = D == 0 ? row : pos;
-    return wp[ov * (WP * WP) + (y + 3) * WP + (x + 3)];
+                                           const PhysParams &P, double *G, double &sum) {
+  // stencil cell o of (rotated) variable v: a step along D per cell, and for
+  // the two velocities one address each
+  const int step = D == 0 ? 1 : WP;
+  const double *const w0 = wp + 3 * WP + 3 + row * (D == 0 ? WP : 1) + (fi - 2) * step;
+  const double *const w1 = w0 + (1 + D) * (WP * WP), *const w2 = w0 + (2 - D) * (WP * WP);
+  auto at = [&](int o, int v) -> double {
+    return v == 1 ? w1[o * step] : (v == 2 ? w2[o * step] : w0[v * (WP * WP) + o * step]);
   };
   // ---- forward replay: reconstruction (reconstruct_LR), as in the stage kernel
   double L[4], R[4];
 #pragma unroll
   for (int v = 0; v < 4; ++v) {
-    const int ov = orig_index_rt<false, 2>(v, D);
-    const double q0 = at(0, ov), q1 = at(1, ov), q2 = at(2, ov), q3 = at(3, ov);
+    const double q0 = at(0, v), q1 = at(1, v), q2 = at(2, v), q3 = at(3, v);
     const double d0 = q1 - q0, d1 = q2 - q1, d2 = q3 - q2;
-    L[v] = q1 + 0.5 * limited_slope<double, true, LIM>(LIM, d1, d0, 0.0);
-    R[v] = q2 - 0.5 * limited_slope<double, false, LIM>(LIM, d2, d1, 0.0);
+    L[v] = q1 + 0.5 * slope_impl<double, true, FAST>(LIM, d1, d0, 0.0);
+    R[v] = q2 - 0.5 * slope_impl<double, false, FAST>(LIM, d2, d1, 0.0);
   }
   const double g = P.gamma, ig = P.inv_gamma_1;
   // hd_to_conserved of the face states
@@ -243,23 +260,23 @@ __device__ __forceinline__ double face_vjp(const double *wp, int D, int fi, int 
   const double fL[4] = {L[1] * L[0], L[1] * cL[1] + L[3], L[1] * cL[2], L[1] * (cL[3] + L[3])};
   const double fR[4] = {R[1] * R[0], R[1] * cR[1] + R[3], R[1] * cR[2], R[1] * (cR[3] + R[3])};
   // Einfeldt bounds
-  const double t1 = sqrt(L[0]), t2 = sqrt(R[0]), t3 = rcp_(t1 + t2);
+  const double t1 = sqrt_f<FAST>(L[0]), t2 = sqrt_f<FAST>(R[0]), t3 = rcp_f<FAST>(t1 + t2);
   const double um = (L[1] * t1 + R[1] * t2) * t3, dv = R[1] - L[1];
-  const double iL0 = rcp_(L[0]), iR0 = rcp_(R[0]);
+  const double iL0 = rcp_f<FAST>(L[0]), iR0 = rcp_f<FAST>(R[0]);
   const double csL = g * L[3] * iL0, csR = g * R[3] * iR0;
-  const double dm = sqrt((t1 * csL + t2 * csR) * t3 + 0.5 * t1 * t2 * (t3 * t3) * (dv * dv));
+  const double dm = sqrt_f<FAST>((t1 * csL + t2 * csR) * t3 + 0.5 * t1 * t2 * (t3 * t3) * (dv * dv));
   const double cmin = um - dm, cmax = um + dm;
   // ---- reverse: Riemann solver
   double fLb[4] = {0.0, 0.0, 0.0, 0.0}, fRb[4] = {0.0, 0.0, 0.0, 0.0};
   double cLb[4] = {0.0, 0.0, 0.0, 0.0}, cRb[4] = {0.0, 0.0, 0.0, 0.0};
   double cmaxb = 0.0, cminb = 0.0;
-  if constexpr (SOLVER == SOLVER_HLLC) hllc_reverse(cL, cR, fL, fR, cmin, cmax, mu, fLb, fRb, cLb, cRb, cmaxb, cminb);
-  else hll_reverse(cL, cR, fL, fR, cmin, cmax, mu, fLb, fRb, cLb, cRb, cmaxb, cminb);
+  if constexpr (SOLVER == SOLVER_HLLC) hllc_reverse<FAST>(cL, cR, fL, fR, cmin, cmax, mu, fLb, fRb, cLb, cRb, cmaxb, cminb);
+  else hll_reverse<FAST>(cL, cR, fL, fR, cmin, cmax, mu, fLb, fRb, cLb, cRb, cmaxb, cminb);
   double Lb[4] = {0.0, 0.0, 0.0, 0.0}, Rb[4] = {0.0, 0.0, 0.0, 0.0}, gb = 0.0;
   // Einfeldt reverse
   {
     const double umb = cmaxb + cminb, dmb = cmaxb - cminb;
-    const double Xb = 0.5 * dmb * rcp_(dm);
+    const double Xb = 0.5 * dmb * rcp_f<FAST>(dm);
     const double dv2 = dv * dv, t33 = t3 * t3;
     double t1b = Xb * (csL * t3 + 0.5 * t2 * t33 * dv2) + umb * L[1] * t3;
     double t2b = Xb * (csR * t3 + 0.5 * t1 * t33 * dv2) + umb * R[1] * t3;
@@ -270,8 +287,8 @@ __device__ __forceinline__ double face_vjp(const double *wp, int D, int fi, int 
     Rb[1] += umb * t2 * t3 + dvb;
     t1b -= t3b * t33;
     t2b -= t3b * t33;
-    Lb[0] += 0.5 * t1b * rcp_(t1);
-    Rb[0] += 0.5 * t2b * rcp_(t2);
+    Lb[0] += 0.5 * t1b * rcp_f<FAST>(t1);
+    Rb[0] += 0.5 * t2b * rcp_f<FAST>(t2);
     Lb[3] += csLb * g * iL0;
     Lb[0] -= csLb * csL * iL0;
     gb += csLb * L[3] * iL0;
@@ -298,29 +315,44 @@ __device__ __forceinline__ double face_vjp(const double *wp, int D, int fi, int 
   // reconstruction reverse
 #pragma unroll
   for (int v = 0; v < 4; ++v) {
-    const int ov = orig_index_rt<false, 2>(v, D);
-    const double q0 = at(0, ov), q1 = at(1, ov), q2 = at(2, ov), q3 = at(3, ov);
+    const double q0 = at(0, v), q1 = at(1, v), q2 = at(2, v), q3 = at(3, v);
     const double d0 = q1 - q0, d1 = q2 - q1, d2 = q3 - q2;
     double dLa, dLb, dRa, dRb;
-    slope_partials<LIM>(d1, d0, dLa, dLb);
-    slope_partials<LIM>(d2, d1, dRa, dRb);
+    slope_partials<LIM, FAST>(d1, d0, dLa, dLb);
+    slope_partials<LIM, FAST>(d2, d1, dRa, dRb);
     const double sLb = 0.5 * Lb[v], sRb = -0.5 * Rb[v];
     const double d0b = sLb * dLb, d1b = sLb * dLa + sRb * dRb, d2b = sRb * dRa;
-    gq[0][v] -= d0b;
-    gq[1][v] += Lb[v] + d0b - d1b;
-    gq[2][v] += Rb[v] + d1b - d2b;
-    gq[3][v] += d2b;
+    // straight to the face's column of G (its entry o, variable ov is
+    // (o * 4 + ov) * NFACE further), so that the sixteen values are not held
+    double *const g = G + (v == 0 ? 0 : (v == 1 ? 1 + D : (v == 2 ? 2 - D : 3))) * NFACE;
+    const double g1 = Lb[v] + d0b - d1b, g2 = Rb[v] + d1b - d2b;
+    g[0 * 4 * NFACE] = -d0b;
+    g[1 * 4 * NFACE] = g1;
+    g[2 * 4 * NFACE] = g2;
+    g[3 * 4 * NFACE] = d2b;
+    sum += (d0b + d2b) + (g1 + g2);
   }
+  sum += gb;
   return gb;
 }
 
 template <int LIM, int SOLVER>
-__global__ void __launch_bounds__(ADJ_THREADS, AMRVAC_ADJ_MINB) adj_stage_kernel(const AdjArgs A) {
+__device__ __noinline__ double face_vjp_guarded(const double *wp, int D, int fi, int row, double m0, double m1,
+                                                double m2, double m3, const PhysParams *P, double *G) {
+  const double mu[4] = {m0, m1, m2, m3};
+  double sum = 0.0;
+  return face_vjp<LIM, SOLVER, FAST_NONE>(wp, D, fi, row, mu, *P, G, sum);
+}
+
+template <int LIM, int SOLVER>
+__global__ void __launch_bounds__(ADJ_THREADS, AMRVAC_ADJ_MINB) adj_stage_kernel(const __grid_constant__ AdjArgs A) {
   extern __shared__ __align__(16) double adj_sm[];
   double *wp = adj_sm;
   double *lm = wp + SM_WP;
   double *G = lm + SM_LM;
   __shared__ double gred[ADJ_THREADS / 32];
+  pdl_wait();
+  pdl_trigger();
   const int b = blockIdx.x;
   const int t = threadIdx.x;
   const StageArgs &S = A.sa;
@@ -375,7 +407,6 @@ __global__ void __launch_bounds__(ADJ_THREADS, AMRVAC_ADJ_MINB) adj_stage_kernel
     if (t < NFACE) {
       const int row = t / NF, fi = t - row * NF - 1;
       const bool valid = !((fi == -1 && phys_lo[D]) || (fi == BN16 + 1 && phys_hi[D]));
-      double gq[4][4] = {{0.0, 0.0, 0.0, 0.0}, {0.0, 0.0, 0.0, 0.0}, {0.0, 0.0, 0.0, 0.0}, {0.0, 0.0, 0.0, 0.0}};
       if (valid) {
         double mu[4];
         const int xr = D == 0 ? fi : row, yr = D == 0 ? row : fi;
@@ -386,16 +417,18 @@ __global__ void __launch_bounds__(ADJ_THREADS, AMRVAC_ADJ_MINB) adj_stage_kernel
           mu[v] = A.s[D] * (lm[ov * (LMW * LMW) + (yr + 2) * LMW + (xr + 2)] -
                             lm[ov * (LMW * LMW) + (yl + 2) * LMW + (xl + 2)]);
         }
-        const double gface = face_vjp<LIM, SOLVER>(wp, D, fi, row, mu, P, gq);
+        double sum = 0.0;
+        double gface = face_vjp<LIM, SOLVER, FAST_ALL>(wp, D, fi, row, mu, P, G + t, sum);
+        if (!isfinite(sum))  // a special operand
+          gface = face_vjp_guarded<LIM, SOLVER>(wp, D, fi, row, mu[0], mu[1], mu[2], mu[3], &P, G + t);
         // faces next to a block edge are computed by two or three blocks: the
         // gamma term counts once, in the block of the cell right of the face
         // (and face 16 at a physical high side)
         if ((fi >= 0 && fi < BN16) || (fi == BN16 && phys_hi[D])) gg += gface;
+      } else {
+#pragma unroll
+        for (int q = 0; q < 16; ++q) G[q * NFACE + t] = 0.0;
       }
-#pragma unroll
-      for (int o = 0; o < 4; ++o)
-#pragma unroll
-        for (int v = 0; v < 4; ++v) G[(o * 4 + orig_index_rt<false, 2>(v, D)) * NFACE + t] = gq[o][v];
     }
     __syncthreads();
     if (t < BN16 * BN16) {
@@ -470,22 +503,24 @@ cudaError_t adjoint_prepare() {
 }
 
 cudaError_t launch_adjoint_stage(const AdjArgs &A, int limiter, int solver, cudaStream_t s) {
-  const int nb = A.sa.nblocks;
+  auto go = [&](void (*kernel)(const AdjArgs)) {
+    return launch_dependent<AdjArgs>(kernel, A.sa.nblocks, ADJ_THREADS, ADJ_SMEM, s, A.sa.dependent, A);
+  };
   if (solver == SOLVER_HLL) {
-    if (limiter == LIM_MINMOD) adj_stage_kernel<LIM_MINMOD, SOLVER_HLL><<<nb, ADJ_THREADS, ADJ_SMEM, s>>>(A);
-    else if (limiter == LIM_VANLEER) adj_stage_kernel<LIM_VANLEER, SOLVER_HLL><<<nb, ADJ_THREADS, ADJ_SMEM, s>>>(A);
-    else return cudaErrorInvalidValue;
+    if (limiter == LIM_MINMOD) return go(&adj_stage_kernel<LIM_MINMOD, SOLVER_HLL>);
+    else if (limiter == LIM_VANLEER) return go(&adj_stage_kernel<LIM_VANLEER, SOLVER_HLL>);
   } else if (solver == SOLVER_HLLC) {
-    if (limiter == LIM_MINMOD) adj_stage_kernel<LIM_MINMOD, SOLVER_HLLC><<<nb, ADJ_THREADS, ADJ_SMEM, s>>>(A);
-    else if (limiter == LIM_VANLEER) adj_stage_kernel<LIM_VANLEER, SOLVER_HLLC><<<nb, ADJ_THREADS, ADJ_SMEM, s>>>(A);
-    else return cudaErrorInvalidValue;
-  } else {
-    return cudaErrorInvalidValue;
+    if (limiter == LIM_MINMOD) return go(&adj_stage_kernel<LIM_MINMOD, SOLVER_HLLC>);
+    else if (limiter == LIM_VANLEER) return go(&adj_stage_kernel<LIM_VANLEER, SOLVER_HLLC>);
   }
-  return cudaGetLastError();
+  return cudaErrorInvalidValue;
 }
 
-__global__ void set_scalar_kernel(double *p, double v) { *p = v; }
+__global__ void set_scalar_kernel(double *p, double v) {
+  pdl_wait();
+  pdl_trigger();
+  *p = v;
+}
 
 cudaError_t launch_set_scalar(double *p, double v, cudaStream_t s) {
   set_scalar_kernel<<<1, 1, 0, s>>>(p, v);

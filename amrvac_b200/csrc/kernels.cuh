@@ -430,6 +430,11 @@ struct Launch {
   static constexpr int VMAIN = HAS_DENSE ? VAR_DENSE : 0;
   static constexpr int SMALL_TILES = 2 * 148;
   static constexpr int NTILE = (BN / tile_edge(BN)) * (BN / tile_edge(BN));
+  // Up to one tile per SM there is no other work to hide a tile's latency, and
+  // a block edge of 16 takes a thread per face (576 threads: one round of
+  // faces instead of three; 64^2 HLLC 24.9 -> 21.7 us a step).  At two tiles per
+  // SM half of them (288) measured no gain over 256 (256^2 31.8 -> 32.2).
+  static constexpr bool HAS_WIDE = HAS_DENSE && BN == 16;
   static constexpr bool HAS_HANCOCK = (SOLVER == SOLVER_TVDLF || SOLVER == SOLVER_TVDMU) && sizeof(TF) == 8;
   static cudaError_t prepare() {
     cudaError_t e = cudaFuncSetAttribute(fv_stage_kernel<TF, MHD, NDIR, GLM, NDIM, SOLVER, LIM, BS, BN>,
@@ -437,6 +442,11 @@ struct Launch {
     if constexpr (HAS_DENSE) {
       if (e == cudaSuccess)
         e = cudaFuncSetAttribute(fv_stage_kernel<TF, MHD, NDIR, GLM, NDIM, SOLVER, LIM, BS, BN, VAR_DENSE>,
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM);
+    }
+    if constexpr (HAS_WIDE) {
+      if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(fv_stage_kernel<TF, MHD, NDIR, GLM, NDIM, SOLVER, LIM, BS, BN, VAR_WIDE>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM);
     }
     if constexpr (HAS_HANCOCK) {
@@ -448,6 +458,12 @@ struct Launch {
   }
   static cudaError_t stage(const StageArgs &A, int nctas, cudaStream_t s) {
     if constexpr (HAS_DENSE) {
+      if constexpr (HAS_WIDE) {
+        if (A.nblocks <= SMALL_TILES / 2)
+          return launch_dependent<StageArgs>(
+              &fv_stage_kernel<TF, MHD, NDIR, GLM, NDIM, SOLVER, LIM, BS, BN, VAR_WIDE>, nctas,
+              StageOcc<TF, MHD, NDIM, LIM, BN, VAR_WIDE>::THREADS, SMEM, s, A.dependent, A);
+      }
       if (A.nblocks * NTILE > SMALL_TILES) {
         return launch_dependent<StageArgs>(&fv_stage_kernel<TF, MHD, NDIR, GLM, NDIM, SOLVER, LIM, BS, BN, VAR_DENSE>,
                                            nctas, THREADS, SMEM, s, A.dependent, A);

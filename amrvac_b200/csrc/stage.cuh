@@ -30,6 +30,8 @@
 
 #include <cuda_runtime.h>
 
+#include <type_traits>
+
 #include "physics.cuh"
 #include "riemann.cuh"
 
@@ -674,7 +676,9 @@ __device__ __forceinline__ uint32_t hancock_dir(const double *smem, const int *b
 // capped for, and the staging mode (asynchronous bulk copies of the next
 // conserved plane, FP64 only).  stage_variant(VAR, fp64) gives them.
 // VAR_DENSE: the FP64 2-D hydrodynamics kernel at twice the CTAs per SM.
-constexpr int VAR_DENSE = 8;
+// VAR_WIDE: the same with a thread per face (544).
+constexpr int VAR_DENSE = 8, VAR_WIDE = 9;
+__host__ __device__ constexpr bool tuned_var(int var) { return var > 0 && var < VAR_DENSE; }
 struct StageVariant {
   int threads, minb;
   bool async;
@@ -701,11 +705,12 @@ template <class TF, bool MHD, int NDIM, int LIM, int BN, int VAR = 0>
 struct StageOcc {
   static constexpr bool FP64 = sizeof(TF) == 8;
   static constexpr int THREADS =
-      VAR > 0 && VAR != VAR_DENSE ? stage_variant(VAR, FP64).threads : (BN == BN16 ? STAGE_THREADS : stage_threads(BN));
+      VAR == VAR_WIDE ? 576 : tuned_var(VAR) ? stage_variant(VAR, FP64).threads : (BN == BN16 ? STAGE_THREADS : stage_threads(BN));
   static constexpr int BASE = stage_base(FP64, MHD, NDIM, HaloW<LIM>::value);
   static constexpr int MINB0 = BASE * 256 / THREADS < 1 ? 1 : (BASE * 256 / THREADS > 16 ? 16 : BASE * 256 / THREADS);
-  static constexpr int MINB = VAR == VAR_DENSE ? 2 * MINB0 : (VAR > 0 ? stage_variant(VAR, FP64).minb : MINB0);
-  static constexpr bool ASYNC = VAR > 0 && VAR != VAR_DENSE && stage_variant(VAR, FP64).async;
+  static constexpr int MINB = VAR == VAR_DENSE ? 2 * MINB0 : VAR == VAR_WIDE ? 1
+                              : tuned_var(VAR) ? stage_variant(VAR, FP64).minb : MINB0;
+  static constexpr bool ASYNC = tuned_var(VAR) && stage_variant(VAR, FP64).async;
 };
 
 // Asynchronous plane staging: one thread copies a block's conserved plane
@@ -913,8 +918,10 @@ __global__ void __launch_bounds__(StageOcc<TF, MHD, NDIM, LIM, BN, VAR>::THREADS
     constexpr int NHX = TB * H2, NHY = H2 * TB, NHC = H2 * H2;
     const int nhalo = update ? (need_corners ? NHX + NHY + NHC : NHX + NHY) : 0;
     // (small tiles have fewer threads than halo cells: a thread may take two)
+    // (with a thread per face the threads behind the cells' take the halo)
+    constexpr int H0 = THREADS >= TB * TB + NHX + NHY ? TB * TB : 0;
 #pragma unroll 1
-    for (int h = t; h < nhalo; h += THREADS) {
+    for (int h = t - H0; h >= 0 && h < nhalo; h += THREADS - H0) {
       int i, j, dst;
       if (h < NHX) {
         j = h / H2;
@@ -1148,14 +1155,25 @@ __global__ void __launch_bounds__(StageOcc<TF, MHD, NDIM, LIM, BN, VAR>::THREADS
             wRp[v] = q[2] - 0.25 * (q[3] - q[1]) * venk_phi(q[1], q[2], q[3], eps2);
           }
         } else {
+          // with the limiter left to run time, the usual ones are compiled in
+          // all the same and chosen once per face: a switch in every slope
+          // cost 3-D MHD HLL + cada3 23 % of its time, 2.5-D MHD HLLD + vanleer
+          // 14 %, 2-D HD HLL + minmod 15 %, 3-D HD HLLC + vanleer 7 % (FP64)
+          auto states = [&](auto limc) {
+            constexpr int L = decltype(limc)::value;
 #pragma unroll
-          for (int v = 0; v < NW; ++v) {
-            TF q[4];
-#pragma unroll
-            for (int o = 0; o < 4; ++o) q[o] = smem[base[o] + var_off(v, rot)];
-            face_states<TF, LIM, FASTF, cada3_short<TF, NDIM, LIM>, !FASTF>(P.limiter, q[0], q[1], q[2], q[3], rd, wLp[v], wRp[v],
-                                                                    special);
-          }
+            for (int v = 0; v < NW; ++v) {
+              const int vo = var_off(v, rot);
+              face_states<TF, L, FASTF, cada3_short<TF, NDIM, LIM>, !FASTF || LIM == 0>(
+                  P.limiter, smem[base[0] + vo], smem[base[1] + vo], smem[base[2] + vo], smem[base[3] + vo], rd, wLp[v],
+                  wRp[v], special);
+            }
+          };
+          if constexpr (LIM != 0) states(std::integral_constant<int, LIM>());
+          else if (P.limiter == LIM_VANLEER) states(std::integral_constant<int, LIM_VANLEER>());
+          else if (P.limiter == LIM_MINMOD) states(std::integral_constant<int, LIM_MINMOD>());
+          else if (P.limiter == LIM_CADA3) states(std::integral_constant<int, LIM_CADA3>());
+          else states(std::integral_constant<int, 0>());
         }
         // mixed form with fix_small_values: a state near a floor goes to the
         // FP64 recomputation (its flux is marked non-finite)

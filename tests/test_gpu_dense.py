@@ -1,6 +1,7 @@
-"""The two builds of the FP64 2-D hydrodynamics stage kernel (two CTAs per SM
-up to 296 tiles, four above) on both sides of that line, at block edges 16 and
-32 (four tiles per block), against the oracle: one full step, cell by cell
+"""The builds of the FP64 2-D hydrodynamics stage kernel (a thread per face up
+to 148 tiles at block edge 16, two CTAs per SM up to 296 tiles, four above) on
+both sides of those lines, at block edges 16 and 32 (four tiles per block),
+against the oracle: one full step, cell by cell
 (tests/_parity.py; bar 1e-12), with the persistent distribution and with one
 tile per CTA.
 """
@@ -15,10 +16,10 @@ pytestmark = pytest.mark.gpu
 RTOL = 1e-12
 
 
-@pytest.mark.parametrize("bn,nb", [(16, (17, 17)), (16, (37, 8)), (16, (11, 27)), (32, (2, 37)), (32, (5, 15))])
+@pytest.mark.parametrize("bn,nb", [(16, (1, 1)), (16, (37, 4)), (16, (1, 149)), (16, (17, 17)), (16, (37, 8)), (16, (11, 27)), (32, (2, 37)), (32, (5, 15))])
 @pytest.mark.parametrize("kw", [dict(flux_scheme="hllc", limiter="vanleer"), dict(flux_scheme="hll", limiter="minmod"),
                                 dict(flux_scheme="tvdlf", limiter="koren", time_stepper="twostep")])
-def test_both_builds_match_oracle(oracle_lib, bn, nb, kw):
+def test_every_build_matches_oracle(oracle_lib, bn, nb, kw):
     import torch
     if not torch.cuda.is_available():
         pytest.skip("no CUDA device")

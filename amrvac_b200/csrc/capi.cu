@@ -77,6 +77,7 @@ struct amrvac_ctx {
   double *d_dx = nullptr;
   double *d_scal = nullptr;              // see setdt_finalize_kernel
   unsigned long long *d_red = nullptr;   // getdt reduction accumulators, then the getdt kernel's CTA ticket
+  double *h_red = nullptr, *h_red_dev = nullptr;  // getdt's result in mapped host memory (lazily), and its device address
   uint32_t *d_status = nullptr;
   uint32_t *d_block_status = nullptr;
   double *d_stage = nullptr;             // upload/download staging
@@ -293,13 +294,14 @@ int launch_stage(amrvac_ctx *c, int reg_ct, int reg_new, int reg_base, double a,
 static bool valid_zchunk(int bn, int zchunk) { return zchunk == 0 || (zchunk >= 2 && bn % zchunk == 0); }
 
 // tail: 0 the reduction alone, 1 with setdt (dt, cmax_global) in the same
-// kernel, 2 also moving the time on; not with 'average', whose flagged blocks
-// are reduced by a second kernel.
+// kernel, 2 also moving the time on, 3 the two maxima to the host instead;
+// 1 to 3 not with 'average', whose flagged blocks a second kernel reduces.
 int launch_getdt(amrvac_ctx *c, int reg, int tail = 0) {
   GetdtArgs G;
   G.scal = tail ? c->d_scal : nullptr;
   G.ticket = reinterpret_cast<unsigned *>(c->d_red + 2);
   G.advance = tail == 2;
+  G.host = tail == 3 ? c->h_red_dev : nullptr;
   G.u = c->pool[reg];
   G.dxb = c->d_dx;
   G.nblocks = c->nblocks;
@@ -791,6 +793,7 @@ int amrvac_gpu_destroy(amrvac_ctx *c) {
   cudaFree(c->d_dx);
   cudaFree(c->d_scal);
   cudaFree(c->d_red);
+  cudaFreeHost(c->h_red);
   cudaFree(c->d_status);
   cudaFree(c->d_block_status);
   for (int r = 0; r < 3; ++r) cudaFree(c->d_adj[r]);
@@ -1442,20 +1445,35 @@ int amrvac_gpu_download(amrvac_ctx *c, int reg, int first, int n, double *w) {
 int amrvac_gpu_getdt(amrvac_ctx *c, int reg, double *dt, double *cmax_global) {
   if (int r = check_ctx(c, true)) return r;
   if (reg < 0 || reg > 2) return fail(AMRVAC_E_ARG, "bad register");
-  if (int r = launch_getdt(c, reg)) return r;
-  unsigned long long red[2];
-  CK(cudaMemcpyAsync(red, c->d_red, sizeof(red), cudaMemcpyDeviceToHost, c->stream));
-  CK(cudaMemsetAsync(c->d_red, 0, sizeof(red), c->stream));
-  CK(cudaStreamSynchronize(c->stream));
   double x, cm;
-  std::memcpy(&x, &red[0], sizeof(double));
-  std::memcpy(&cm, &red[1], sizeof(double));
+  if (!c->sv_on) {
+    // one launch and one wait: the kernel itself writes the result to the
+    // host and cmax_global to the device scalar (three copies and a second
+    // wait around it: a 64^2 host-driven step 82.7 us, with this and advect1's
+    // scalar 68.7)
+    if (!c->h_red) {
+      CK(cudaHostAlloc(&c->h_red, 2 * sizeof(double), cudaHostAllocMapped));
+      CK(cudaHostGetDevicePointer(&c->h_red_dev, c->h_red, 0));
+    }
+    if (int r = launch_getdt(c, reg, 3)) return r;
+    CK(cudaStreamSynchronize(c->stream));
+    x = c->h_red[0];
+    cm = c->h_red[1];
+  } else {
+    if (int r = launch_getdt(c, reg)) return r;
+    unsigned long long red[2];
+    CK(cudaMemcpyAsync(red, c->d_red, sizeof(red), cudaMemcpyDeviceToHost, c->stream));
+    CK(cudaMemsetAsync(c->d_red, 0, sizeof(red), c->stream));
+    CK(cudaStreamSynchronize(c->stream));
+    std::memcpy(&x, &red[0], sizeof(double));
+    std::memcpy(&cm, &red[1], sizeof(double));
+    CK(cudaMemcpyAsync(c->d_scal + 1, &cm, sizeof(double), cudaMemcpyHostToDevice, c->stream));
+    CK(cudaStreamSynchronize(c->stream));
+  }
   double d = 1.0e99;
   if (x > 1.0e-12) d = std::min(d, c->cfg.courantpar / x);
   if (dt) *dt = d;
   if (cmax_global) *cmax_global = cm;
-  CK(cudaMemcpyAsync(c->d_scal + 1, &cm, sizeof(double), cudaMemcpyHostToDevice, c->stream));
-  CK(cudaStreamSynchronize(c->stream));
   return d < c->cfg.dtmin ? (int)AMRVAC_ST_DT_TOO_SMALL : 0;
 }
 
@@ -1474,7 +1492,12 @@ int amrvac_gpu_advect1(amrvac_ctx *c, int reg_ct, int reg_new, int reg_base, dou
   if (reg_ct == reg_new) return fail(AMRVAC_E_ARG, "reg_ct and reg_new must differ");
   if (a_base == 0.0 && b_in != 1.0) return fail(AMRVAC_E_ARG, "a_base == 0 requires b_in == 1");
   if (int r = check_a2max(c)) return r;
-  CK(cudaMemcpyAsync(c->d_scal + 0, &dt, sizeof(double), cudaMemcpyHostToDevice, c->stream));
+  // dt goes in by a kernel's argument, and the stage follows as a dependent
+  // launch (a copy from the host's stack costs more than both launches)
+  CK(launch_set_scalar(c->d_scal + 0, dt, c->stream));
+  ++c->launches;
+  ChainScope chain(c);
+  c->chained = true;
   int r = launch_stage(c, reg_ct, reg_new, reg_base, a_base, b_in, dtfactor);
   CK(cudaStreamSynchronize(c->stream));
   return r;

@@ -62,6 +62,9 @@ struct GetdtArgs {
   double *scal;
   unsigned *ticket;
   int advance;
+  // amrvac_gpu_getdt: the last CTA writes the two maxima to the host's memory
+  // (mapped), sets scal's cmax_global and clears the words for the next call
+  double *host;
   bool dependent;  // launch: the predecessor on the stream allows a dependent launch
 };
 
@@ -177,10 +180,21 @@ __global__ void __launch_bounds__(256, 4) getdt_kernel(const GetdtArgs A) {
     if (atomicAdd(A.ticket, 1u) == gridDim.x - 1) {
       __threadfence();
       *A.ticket = 0u;
-      setdt_finalize(A.red, A.scal, A.status);
-      if (A.advance) {
-        A.scal[2] = A.scal[2] + A.scal[0];
-        A.scal[9] = A.scal[9] + 1.0;
+      if (A.host) {
+        volatile unsigned long long *red = A.red;
+        const double x = __longlong_as_double((long long)red[0]), cm = __longlong_as_double((long long)red[1]);
+        red[0] = 0ull;
+        red[1] = 0ull;
+        A.scal[1] = cm;
+        A.host[0] = x;
+        A.host[1] = cm;
+        __threadfence_system();
+      } else {
+        setdt_finalize(A.red, A.scal, A.status);
+        if (A.advance) {
+          A.scal[2] = A.scal[2] + A.scal[0];
+          A.scal[9] = A.scal[9] + 1.0;
+        }
       }
     }
   }

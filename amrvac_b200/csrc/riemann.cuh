@@ -12,8 +12,9 @@
 
 namespace amrvac {
 
+// An FP64 product that no later addition may be fused with.
 __device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
-__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ float mul_rn(float a, float b) { return a * b; }
 
 template <bool MHD, int NDIM, bool GLM>
 struct FluxTypes {
@@ -523,20 +524,22 @@ __device__ __forceinline__ void riemann_hlld(const T *wLC, const T *wRC, const T
   if constexpr (FT::bn_special) F[B] = f[B];
 }
 
-// Where HLLD starts from the primitive states: in 3-D and in FP32.  2.5-D
-// FP64 runs keep the reference's order of operations, because weakly
-// magnetised flows there (the field loop) carry a last-bit difference through
-// cada3's small slope-ratio denominators to 1e-8 within twenty steps, and
-// their results are compared with earlier ones to 1e-9.
-template <class T, int NDIM>
-constexpr bool hlld_from_primitives = NDIM == 3 || sizeof(T) == 4;
+// Where HLLD starts from the primitive states: in 3-D FP64, and in FP32 with a
+// limiter that is continuous in the data.  2.5-D FP64 runs keep the reference's
+// order of operations, because weakly magnetised flows there (the field loop)
+// carry a last-bit difference through cada3's small slope-ratio denominators to
+// 1e-8 within twenty steps; and cada3 itself jumps where tmpeta passes 1, so
+// that in FP32 every rounding difference moves a few cells to the other side
+// (1e-4 of the state on coarse grids).  Results there are compared with
+// earlier ones more closely than that.
+template <class T, int NDIM, int LIM>
+constexpr bool hlld_from_primitives = sizeof(T) == 8 ? NDIM == 3 : (LIM == LIM_VANLEER || LIM == LIM_MINMOD);
 
 // The same solver from the primitive face states alone (rotated, after
 // mhd_modify_wLR, so with GLM both sides hold the same normal field, which is
 // then Bx itself): the conserved state is formed for the face's side only and
 // common factors are taken out, a quarter fewer operations than riemann_hlld
-// (3-D MHD 128^3 FP64 0.64 -> 0.59 ms per stage, mixed 0.42 -> 0.39) at
-// rounding differences.  hlld_from_primitives says where it is used.
+// (3-D MHD 128^3 FP64 0.64 -> 0.59 ms per stage) at rounding differences.  hlld_from_primitives says where it is used.
 template <class T, int NDIR, bool GLM, int NDIM, int FAST = 0>
 __device__ __forceinline__ void riemann_hlld_prim(const T *wLp, const T *wRp, T sR, T sL, T cg, T inv_gamma_1, T *F) {
   using V = Vars<true, NDIR, GLM>;

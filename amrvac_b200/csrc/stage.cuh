@@ -254,7 +254,8 @@ __device__ __forceinline__ uint32_t load_prim(const StageArgs &A, int b, int i, 
 // (src/mod_finite_volume.t:1217-1222, 200-245).  wLp/wRp are modified.
 // HLLD and the HD HLLC form the physical flux themselves, of the side of the
 // contact that the face lies in.
-template <class T, bool MHD, int NDIR, bool GLM, int NDIM, int SOLVER, int BS, int FAST = 0>
+// LIM: the limiter the states come from, if it is fixed (hlld_from_primitives).
+template <class T, bool MHD, int NDIR, bool GLM, int NDIM, int SOLVER, int BS, int FAST = 0, int LIM = 0>
 __device__ __forceinline__ uint32_t face_from_states(T *wLp, T *wRp, const PhysParams &P, T cg, T *F,
                                                      bool small_check = true) {
   constexpr int D = 0;  // states arrive rotated: the face normal is component 0
@@ -266,7 +267,7 @@ __device__ __forceinline__ uint32_t face_from_states(T *wLp, T *wRp, const PhysP
     bool fr = small_values<T, MHD, NDIR, GLM>(wRp, true, P);
     if ((fl || fr) && P.small_values_method != 1) st |= ST_SMALL_VALUE;
   }
-  constexpr bool PRIM = SOLVER == SOLVER_HLLD && hlld_from_primitives<T, NDIM>;
+  constexpr bool PRIM = SOLVER == SOLVER_HLLD && hlld_from_primitives<T, NDIM, LIM>;
   T wLC[NW], wRC[NW];
   if constexpr (!PRIM) {
 #pragma unroll
@@ -445,9 +446,9 @@ __device__ __forceinline__ double venk_phi(double wm, double w0, double wp, doub
 }
 
 // Where cada3's short form (face_states with R2) is used: with the limiter
-// fixed to it, in 3-D and in FP32, as hlld_from_primitives (riemann.cuh).
+// fixed to it, in 3-D FP64, as hlld_from_primitives (riemann.cuh).
 template <class TF, int NDIM, int LIM>
-constexpr bool cada3_short = LIM == LIM_CADA3 && (NDIM == 3 || sizeof(TF) == 4);
+constexpr bool cada3_short = LIM == LIM_CADA3 && NDIM == 3 && sizeof(TF) == 8;
 
 // Halo width of the staged tile: two cells for the slope limiters, three for
 // the fifth-order reconstructions (face stencil i-2 .. i+3).  LIM_WENO5 as a
@@ -596,7 +597,7 @@ __device__ __noinline__ FaceFlux64<Vars<MHD, NDIR, GLM>::NW> face_retry_state(co
   for (int v = 0; v < NW; ++v) {
     const int ov = orig_index_rt<MHD, NDIR>(v, D);
     bool special = false;
-    face_states<double, LIM, false, cada3_short<float, NDIM, LIM>>(A->P.limiter, q[0][ov], q[1][ov], q[2][ov], q[3][ov], rd,
+    face_states<double, LIM, 0, cada3_short<float, NDIM, LIM>>(A->P.limiter, q[0][ov], q[1][ov], q[2][ov], q[3][ov], rd,
                                                                    wLp[v], wRp[v], special);
   }
   FaceFlux64<NW> r;
@@ -823,6 +824,8 @@ __global__ void __launch_bounds__(StageOcc<TF, MHD, NDIM, LIM, BN, VAR>::THREADS
   constexpr bool ASYNC = StageOcc<TF, MHD, NDIM, LIM, BN, VAR>::ASYNC && FP64 && NDIM == 3 && NT == 1 && HW == 2 &&
                          SOLVER != SOLVER_HANCOCK;
   __shared__ __align__(8) unsigned long long s_mbar;
+  __shared__ double s_dx[3], s_idx[3], s_dxinv[3], s_rdel[3], s_damp;
+  __shared__ double s_wlam[3];
   uint32_t mphase = 0;
   if constexpr (ASYNC) {
     if (t == 0) mbar_init(smem_addr(&s_mbar));
@@ -839,19 +842,33 @@ __global__ void __launch_bounds__(StageOcc<TF, MHD, NDIM, LIM, BN, VAR>::THREADS
   g += k1 - k0;
   uint32_t stb = 0;  // status of this block's update
   const int amr_mask = A.amr_face ? A.amr_face[b] : 0;
-  double dx[3], dxinv[3], rdel[3];
-  [[maybe_unused]] double wlam[3];  // WENO-Z+: dx^(2/3) per direction
-#pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    dx[d] = d < NDIM ? A.dxb[b * 3 + d] : 1.0;
-    dxinv[d] = -qdt / dx[d];
-    const double r = P.cada3_radius * dx[d];
-    // cada3: 1 / (cada3_radius dx)^2, or its inverse for the short form; schmid: (a2max + cadepsilon) dx^2 with
-    // a2max = schmid_rad (schmid2) or a2max_global of this step (schmid1)
-    const double a2m = P.schmid_global ? A.dt_dev[10 + d] : P.schmid_rad[d];
-    rdel[d] = (LIM == LIM_SCHMID || (LIM == 0 && P.limiter == LIM_SCHMID))
-                  ? (a2m + 1.0e-14) * (dx[d] * dx[d]) : (cada3_short<TF, NDIM, LIM> ? r * r : 1.0 / (r * r));
-    if constexpr (LIM == LIM_WENO5) wlam[d] = pow(dx[d], 2.0 / 3.0);
+  // The block's constants in shared memory, formed by one thread each: kept
+  // per thread they took 18 registers, and their divisions (and the GLM
+  // source's exponential in every cell) a tenth of the 2-D kernels'
+  // instructions.  Read behind the first barrier below; the previous column's
+  // reads end before its last one.
+  if (t < 3) {
+    const double dx = t < NDIM ? A.dxb[b * 3 + t] : 1.0;
+    s_dx[t] = dx;
+    s_idx[t] = 1.0 / dx;
+    s_dxinv[t] = -qdt / dx;
+    const double r = P.cada3_radius * dx;
+    // cada3: 1 / (cada3_radius dx)^2, or its inverse for the short form; schmid:
+    // (a2max + cadepsilon) dx^2 with a2max = schmid_rad (schmid2) or
+    // a2max_global of this step (schmid1)
+    const double a2m = P.schmid_global ? A.dt_dev[10 + t] : P.schmid_rad[t];
+    s_rdel[t] = (LIM == LIM_SCHMID || (LIM == 0 && P.limiter == LIM_SCHMID))
+                    ? (a2m + 1.0e-14) * (dx * dx) : (cada3_short<TF, NDIM, LIM> ? r * r : 1.0 / (r * r));
+    if constexpr (LIM == LIM_WENO5) s_wlam[t] = pow(dx, 2.0 / 3.0);  // WENO-Z+
+  }
+  // addsource2 with qdt (idimmax - idimmin + 1) / ndim
+  const double qsrc = qdt * double(dsel < 0 ? NDIM : 1) / double(NDIM);
+  if constexpr (MHD && GLM) {
+    if (t == 32) {  // psi's damping factor (add_source_glm)
+      double mindx = A.dxb[b * 3];
+      for (int d = 1; d < NDIM; ++d) mindx = fmin(mindx, A.dxb[b * 3 + d]);
+      s_damp = exp(-(qsrc * cg * P.glm_alpha) / mindx);
+    }
   }
   double fz_prev[NDIM == 3 ? NW : 1];
 #pragma unroll
@@ -965,17 +982,17 @@ __global__ void __launch_bounds__(StageOcc<TF, MHD, NDIM, LIM, BN, VAR>::THREADS
         if (dsel < 0 || dsel == 0) {
 #pragma unroll
           for (int o = 0; o < 3; ++o) base[o] = tv.off(slot, ci + o - 1, cj);
-          stb |= hancock_dir<MHD, NDIR, GLM, LIM, 0, VS>(smem, base, rdel[0], dxinv[0], cg, P, acc);
+          stb |= hancock_dir<MHD, NDIR, GLM, LIM, 0, VS>(smem, base, s_rdel[0], s_dxinv[0], cg, P, acc);
         }
         if (dsel < 0 || dsel == 1) {
 #pragma unroll
           for (int o = 0; o < 3; ++o) base[o] = tv.off(slot, ci, cj + o - 1);
-          stb |= hancock_dir<MHD, NDIR, GLM, LIM, 1, VS>(smem, base, rdel[1], dxinv[1], cg, P, acc);
+          stb |= hancock_dir<MHD, NDIR, GLM, LIM, 1, VS>(smem, base, s_rdel[1], s_dxinv[1], cg, P, acc);
         }
         if (NDIM == 3 && (dsel < 0 || dsel == 2)) {
 #pragma unroll
           for (int o = 0; o < 3; ++o) base[o] = ring_slot<HW>(k + o - 1) * (TB * TB) + cj * TB + ci;
-          stb |= hancock_dir<MHD, NDIR, GLM, LIM, 2, VS>(smem, base, rdel[2], dxinv[2], cg, P, acc);
+          stb |= hancock_dir<MHD, NDIR, GLM, LIM, 2, VS>(smem, base, s_rdel[2], s_dxinv[2], cg, P, acc);
         }
       }
     } else {
@@ -1066,7 +1083,7 @@ __global__ void __launch_bounds__(StageOcc<TF, MHD, NDIM, LIM, BN, VAR>::THREADS
       for (int f = t; f < nface; f += THREADS) {
         int fi, fj, FD, fl;
         face_dir(f, FD, fl);
-        const TF rd = TF(FD == 0 ? rdel[0] : (FD == 1 ? rdel[1] : rdel[2]));
+        const TF rd = TF(s_rdel[FD]);
         TF wLp[NW], wRp[NW];
         bool special = false;  // near a limiter's blending band: left to the recomputation
         int base[H2], rot[NDIR];
@@ -1101,7 +1118,7 @@ __global__ void __launch_bounds__(StageOcc<TF, MHD, NDIM, LIM, BN, VAR>::THREADS
           // flagged density or pressure in either state makes every variable
           // of the face take the flat states w(i), w(i+1)
           const int var = P.limiter == LIM_WENO5 ? 1 : (P.limiter == LIM_WENOZ5 ? 2 : 3);
-          const double lam = FD == 0 ? wlam[0] : (FD == 1 ? wlam[1] : wlam[2]);
+          const double lam = s_wlam[FD];
 #pragma unroll
           for (int v = 0; v < NW; ++v) {
             double q[6];
@@ -1123,7 +1140,7 @@ __global__ void __launch_bounds__(StageOcc<TF, MHD, NDIM, LIM, BN, VAR>::THREADS
           // WENO3limiter then fix_limiter (all variables flat where density or
           // pressure is flagged in either state)
           const int var = P.limiter == LIM_WENO3 ? 1 : 2;
-          const double dxd = FD == 0 ? dx[0] : (FD == 1 ? dx[1] : dx[2]);
+          const double dxd = s_dx[FD];
           const double dx2 = dxd * dxd;
 #pragma unroll
           for (int v = 0; v < NW; ++v) {
@@ -1143,7 +1160,7 @@ __global__ void __launch_bounds__(StageOcc<TF, MHD, NDIM, LIM, BN, VAR>::THREADS
           }
         } else if constexpr (LIM == LIM_VENK) {
           static_assert(FP64, "the Venkatakrishnan limiter is FP64 only");
-          const double dxd = FD == 0 ? dx[0] : (FD == 1 ? dx[1] : dx[2]);
+          const double dxd = s_dx[FD];
           const double kd = 0.3 * dxd;
           const double eps2 = kd * kd * kd;
 #pragma unroll
@@ -1192,7 +1209,7 @@ __global__ void __launch_bounds__(StageOcc<TF, MHD, NDIM, LIM, BN, VAR>::THREADS
         TF Fr[NW];
         // the MP5 / WENO branches of reconstruct_LR have no small-value fix of
         // the states
-        stb |= face_from_states<TF, MHD, NDIR, GLM, NDIM, SOLVER, BS, FASTF>(wLp, wRp, P, TF(cg), Fr,
+        stb |= face_from_states<TF, MHD, NDIR, GLM, NDIM, SOLVER, BS, FASTF, LIM>(wLp, wRp, P, TF(cg), Fr,
                                                                               HW == 2 && LIM != LIM_WENO3 && !near);
         if constexpr (RETRY) {
           // one test on the sum: an infinite or NaN flux component makes it
@@ -1208,7 +1225,7 @@ __global__ void __launch_bounds__(StageOcc<TF, MHD, NDIM, LIM, BN, VAR>::THREADS
         }
         // FP64: the scaled flux fC = -qdt/dx * f as in the reference; mixed:
         // the FP32 flux, scaled in FP64 by the accumulating cell thread
-        const double sc = FD == 0 ? dxinv[0] : (FD == 1 ? dxinv[1] : dxinv[2]);
+        const double sc = s_dxinv[FD];
 #pragma unroll
         for (int v = 0; v < NW; ++v) {
           if constexpr (FP64) flux_ref(f, FD, fl, v) = sc * Fr[v];
@@ -1229,10 +1246,10 @@ __global__ void __launch_bounds__(StageOcc<TF, MHD, NDIM, LIM, BN, VAR>::THREADS
             bool finite = true;
             for (int v = 0; v < NW; ++v) finite = finite && isfinite(flux_ref(f, FD, fl, v));
             if (finite) continue;
-            const double sc = FD == 0 ? dxinv[0] : (FD == 1 ? dxinv[1] : dxinv[2]);
+            const double sc = s_dxinv[FD];
             int fi, fj, base[H2];
             face_at(FD, fl, fi, fj, base);
-            const double rdd = FD == 0 ? rdel[0] : (FD == 1 ? rdel[1] : rdel[2]);
+            const double rdd = s_rdel[FD];
             FaceFlux64<NW> r;
             if constexpr (FP64) {
               bool done = false;
@@ -1264,7 +1281,7 @@ __global__ void __launch_bounds__(StageOcc<TF, MHD, NDIM, LIM, BN, VAR>::THREADS
       if (cell_thread) {
         // the fluxes are stored rotated: entry v is variable orig_index<D>(v)
         if (MERGED ? dsel != 1 : D == 0) {
-          const double sc = FP64 ? 1.0 : dxinv[0];
+          const double sc = FP64 ? 1.0 : s_dxinv[0];
           const int f = cj * (TB + 1) + ci;
 #pragma unroll
           for (int v = 0; v < NW; ++v) {
@@ -1274,7 +1291,7 @@ __global__ void __launch_bounds__(StageOcc<TF, MHD, NDIM, LIM, BN, VAR>::THREADS
           }
         }
         if (MERGED ? dsel != 0 : D == 1) {
-          const double sc = FP64 ? 1.0 : dxinv[1];
+          const double sc = FP64 ? 1.0 : s_dxinv[1];
           const int f = cj * TB + ci;
           const TF *fy = MERGED ? tv.yx : tv.fb;
 #pragma unroll
@@ -1287,7 +1304,7 @@ __global__ void __launch_bounds__(StageOcc<TF, MHD, NDIM, LIM, BN, VAR>::THREADS
           }
         }
         if constexpr (NDIM == 3) if (D == 2) {
-          const double sc = FP64 ? 1.0 : dxinv[2];
+          const double sc = FP64 ? 1.0 : s_dxinv[2];
 #pragma unroll
           for (int v = 0; v < NW; ++v) {
             double &a = acc[orig_index<MHD, NDIR, 2>(v)];
@@ -1317,17 +1334,12 @@ __global__ void __launch_bounds__(StageOcc<TF, MHD, NDIM, LIM, BN, VAR>::THREADS
       // ---- unsplit divB sources (addsource2 -> mhd_add_source)
       if constexpr (MHD) {
         if (NDIM > 1) {
-          // addsource2 with qdt (idimmax - idimmin + 1) / ndim
-          const double qsrc = qdt * double(dsel < 0 ? NDIM : 1) / double(NDIM);
           if constexpr (GLM) {
             // add_source_glm (src/mhd/mod_mhd_phys.t:5472-5531)
-            double mindx = dx[0];
-#pragma unroll
-            for (int d = 1; d < NDIM; ++d) mindx = fmin(mindx, dx[d]);
             if (P.glm_alpha < 0.0) {
               acc[V::PSI] = fabs(P.glm_alpha) * A.uin[cell_offset<NDIM>(b, NW, V::PSI, bi, bj, k, BN)];
             } else {
-              acc[V::PSI] = exp(-(qsrc * cg * P.glm_alpha) / mindx) * acc[V::PSI];
+              acc[V::PSI] = s_damp * acc[V::PSI];
             }
             if (P.glm_extended) {
               auto nbv = [&](int d, int s, int v) -> double {  // wCT at cell +/- e_d
@@ -1337,13 +1349,15 @@ __global__ void __launch_bounds__(StageOcc<TF, MHD, NDIM, LIM, BN, VAR>::THREADS
               };
 #pragma unroll
               for (int d = 0; d < NDIM; ++d) {
-                const double g = ((nbv(d, 1, V::PSI) - nbv(d, -1, V::PSI)) * 0.5) / dx[d];
+                // (2.5-D FP64 divides, as the reference does: see hlld_from_primitives)
+                const double dp = (nbv(d, 1, V::PSI) - nbv(d, -1, V::PSI)) * 0.5;
+                const double g = NDIM == 3 || !FP64 ? dp * s_idx[d] : dp / s_dx[d];
                 acc[V::E] = acc[V::E] - qsrc * double(tv.at(slot, V::B0 + d, ci, cj)) * g;
               }
               double divb = 0.0;
 #pragma unroll
               for (int d = 0; d < NDIM; ++d)
-                divb = divb + 0.5 * (nbv(d, 1, V::B0 + d) - nbv(d, -1, V::B0 + d)) * (1.0 / dx[d]);
+                divb = divb + 0.5 * (nbv(d, 1, V::B0 + d) - nbv(d, -1, V::B0 + d)) * s_idx[d];
 #pragma unroll
               for (int c = 0; c < NDIR; ++c)
                 acc[V::M0 + c] = acc[V::M0 + c] - qsrc * double(tv.at(slot, V::B0 + c, ci, cj)) * divb;
@@ -1356,17 +1370,17 @@ __global__ void __launch_bounds__(StageOcc<TF, MHD, NDIM, LIM, BN, VAR>::THREADS
             if constexpr (NDIM == 2) if (!jump_layer) {
               // add_source_linde (src/mhd/mod_mhd_phys.t:5599-5665)
               auto divb_at = [&](int i, int j) -> double {
-                double d = 0.5 * (double(tv.at(slot, V::B0, i + 1, j)) - double(tv.at(slot, V::B0, i - 1, j))) * (1.0 / dx[0]);
-                d = d + 0.5 * (double(tv.at(slot, V::B0 + 1, i, j + 1)) - double(tv.at(slot, V::B0 + 1, i, j - 1))) * (1.0 / dx[1]);
+                double d = 0.5 * (double(tv.at(slot, V::B0, i + 1, j)) - double(tv.at(slot, V::B0, i - 1, j))) * s_idx[0];
+                d = d + 0.5 * (double(tv.at(slot, V::B0 + 1, i, j + 1)) - double(tv.at(slot, V::B0 + 1, i, j - 1))) * s_idx[1];
                 return d;
               };
-              const double inv2 = 1.0 / (dx[0] * dx[0]) + 1.0 / (dx[1] * dx[1]);
+              const double inv2 = 1.0 / (s_dx[0] * s_dx[0]) + 1.0 / (s_dx[1] * s_dx[1]);
 #pragma unroll
               for (int d = 0; d < 2; ++d) {
                 const double dp = d == 0 ? divb_at(ci + 1, cj) : divb_at(ci, cj + 1);
                 const double dm = d == 0 ? divb_at(ci - 1, cj) : divb_at(ci, cj - 1);
                 double g = (dp - dm) * 0.5;
-                g = g / dx[d];
+                g = g / s_dx[d];
                 g = g * P.divbdiff / inv2;
                 acc[V::B0 + d] = acc[V::B0 + d] + g;
                 acc[V::E] = acc[V::E] + double(tv.at(slot, V::B0 + d, ci, cj)) * g;

@@ -1,0 +1,71 @@
+"""The pool behind the contexts' registers: contexts made, stepped and closed by
+several threads at once give the bits a context alone gives, and closing large
+ones gives their memory back down to the pool's bound.
+"""
+import threading
+
+import numpy as np
+import pytest
+
+from tests import _problems as P
+
+pytestmark = pytest.mark.gpu
+
+KEEP = 256 << 20  # capi.cu POOL_KEEP
+
+
+def _run(n, out, key, reps):
+    from amrvac_b200 import Context, make_cfg
+    prim, geo = P.kh_2d(n=n, seed=5)
+    blocks = P.to_blocks(P.prim_to_cons(prim, "hd", 2, 1.4), 2)
+    for _ in range(reps):
+        with Context(make_cfg(physics="hd", ndim=2, gamma=1.4, flux_scheme="hllc", limiter="vanleer")) as ctx:
+            ctx.set_uniform_grid(geo["domain_nx"], geo["xprobmin"], geo["xprobmax"])
+            ctx.upload(blocks)
+            ctx.set_time(0.0, 1.0e99, 0.0)
+            ctx.run(4)
+            out.setdefault(key, []).append(ctx.download())
+
+
+def test_threads_share_the_pool():
+    import torch
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    sizes = (64, 160, 64, 160)
+    alone, got = {}, {}
+    for n in set(sizes):
+        _run(n, alone, n, 1)
+    th = [threading.Thread(target=_run, args=(n, got, (i, n), 3)) for i, n in enumerate(sizes)]
+    for t in th:
+        t.start()
+    for t in th:
+        t.join()
+    assert len(got) == len(sizes)
+    for (_, n), runs in got.items():
+        assert len(runs) == 3
+        for r in runs:
+            assert np.array_equal(r, alone[n][0])
+
+
+def test_closed_contexts_give_memory_back():
+    import torch
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from amrvac_b200 import Context, make_cfg
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    # 1024^2 HD: 32 MB per register with its headroom 42 MB, three registers, six contexts
+    ctxs = []
+    for _ in range(6):
+        c = Context(make_cfg(physics="hd", ndim=2, gamma=1.4, flux_scheme="hllc", limiter="vanleer"))
+        c.set_uniform_grid([1024, 1024], [0.0] * 2, [1.0] * 2)
+        ctxs.append(c)
+    torch.cuda.synchronize()
+    used = before - torch.cuda.mem_get_info()[0]
+    assert used > 2 * KEEP
+    for c in ctxs:
+        c.close()
+    torch.cuda.synchronize()
+    kept = before - torch.cuda.mem_get_info()[0]
+    # the bound, and the driver's granularity of a few blocks of 32 MB
+    assert kept <= KEEP + (128 << 20), (used, kept)

@@ -359,9 +359,13 @@ __global__ void __launch_bounds__(ADJ_THREADS, AMRVAC_ADJ_MINB) adj_stage_kernel
   const PhysParams &P = S.P;
   const bool phys_lo[2] = {S.nbr[b * 27 + dir_index(-1, 0, 0)] < 0, S.nbr[b * 27 + dir_index(0, -1, 0)] < 0};
   const bool phys_hi[2] = {S.nbr[b * 27 + dir_index(1, 0, 0)] < 0, S.nbr[b * 27 + dir_index(0, 1, 0)] < 0};
-  // ---- primitives with a 3-cell halo (no corners)
-  for (int p = t; p < 22 * 16 + 6 * 16; p += ADJ_THREADS) {
-    int x, y;
+  // ---- primitives with a 3-cell halo (no corners) and lambda with a 2-cell
+  // halo (zero at physical ghosts).  A thread takes up to two positions of
+  // each; the loads of all four are issued before the first is used, so that
+  // a block waits for memory once.
+  constexpr int NP = 22 * 16 + 6 * 16, NL = 20 * 16 + 4 * 16;
+  static_assert(NP <= 2 * ADJ_THREADS && NL <= 2 * ADJ_THREADS, "two positions per thread");
+  auto prim_pos = [](int p, int &x, int &y) {
     if (p < 22 * 16) {
       y = p / 22;
       x = p - y * 22 - 3;
@@ -370,14 +374,8 @@ __global__ void __launch_bounds__(ADJ_THREADS, AMRVAC_ADJ_MINB) adj_stage_kernel
       y = r < 3 ? r - 3 : r + 13;
       x = q & (BN16 - 1);
     }
-    double w[4];
-    load_prim<false, 2, false, 2>(S, b, x, y, 0, w);
-#pragma unroll
-    for (int v = 0; v < 4; ++v) wp[v * (WP * WP) + (y + 3) * WP + (x + 3)] = w[v];
-  }
-  // ---- lambda with a 2-cell halo; zero at physical ghosts
-  for (int p = t; p < 20 * 16 + 4 * 16; p += ADJ_THREADS) {
-    int x, y;
+  };
+  auto lam_pos = [](int p, int &x, int &y) {
     if (p < 20 * 16) {
       y = p / 20;
       x = p - y * 20 - 2;
@@ -386,18 +384,52 @@ __global__ void __launch_bounds__(ADJ_THREADS, AMRVAC_ADJ_MINB) adj_stage_kernel
       y = r < 2 ? r - 2 : r + 14;
       x = q & (BN16 - 1);
     }
-    const bool phys = (x < 0 && phys_lo[0]) || (x >= BN16 && phys_hi[0]) || (y < 0 && phys_lo[1]) ||
-                      (y >= BN16 && phys_hi[1]);
-    double l[4] = {0.0, 0.0, 0.0, 0.0};
-    if (!phys) {
-      int i = x, j = y, k = 0;
-      uint32_t flip;
-      const int blk = resolve_cell<2>(S, b, i, j, k, flip);
+  };
+  {
+    double w[2][4], l[2][4];
 #pragma unroll
-      for (int v = 0; v < 4; ++v) l[v] = A.lam[cell_offset<2>(blk, 4, v, i, j, 0)];
+    for (int q = 0; q < 2; ++q) {
+      const int p = t + q * ADJ_THREADS;
+      int x, y;
+      if (p < NP) {
+        prim_pos(p, x, y);
+        load_cons<false, 2, false, 2>(S, b, x, y, 0, w[q]);
+      }
     }
 #pragma unroll
-    for (int v = 0; v < 4; ++v) lm[v * (LMW * LMW) + (y + 2) * LMW + (x + 2)] = l[v];
+    for (int q = 0; q < 2; ++q) {
+      const int p = t + q * ADJ_THREADS;
+#pragma unroll
+      for (int v = 0; v < 4; ++v) l[q][v] = 0.0;
+      if (p < NL) {
+        int i, j, k = 0;
+        lam_pos(p, i, j);
+        const bool phys = (i < 0 && phys_lo[0]) || (i >= BN16 && phys_hi[0]) || (j < 0 && phys_lo[1]) ||
+                          (j >= BN16 && phys_hi[1]);
+        if (!phys) {
+          uint32_t flip;
+          const int blk = resolve_cell<2>(S, b, i, j, k, flip);
+#pragma unroll
+          for (int v = 0; v < 4; ++v) l[q][v] = A.lam[cell_offset<2>(blk, 4, v, i, j, 0)];
+        }
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const int p = t + q * ADJ_THREADS;
+      int x, y;
+      if (p < NP) {
+        prim_pos(p, x, y);
+        cons_to_prim<false, 2, false>(P, w[q]);
+#pragma unroll
+        for (int v = 0; v < 4; ++v) wp[v * (WP * WP) + (y + 3) * WP + (x + 3)] = w[q][v];
+      }
+      if (p < NL) {
+        lam_pos(p, x, y);
+#pragma unroll
+        for (int v = 0; v < 4; ++v) lm[v * (LMW * LMW) + (y + 2) * LMW + (x + 2)] = l[q][v];
+      }
+    }
   }
   __syncthreads();
   double gp[4] = {0.0, 0.0, 0.0, 0.0};  // dL/d(primitive) of this thread's cell

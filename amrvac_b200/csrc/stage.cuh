@@ -218,13 +218,13 @@ __device__ __forceinline__ size_t ghost_offset(int slot, int nw, int v, int i, i
   return (((size_t)slot * nw + v) * GZ + gk) * (size_t)(GY * G) + (size_t)gj * G + (i + 2);
 }
 
-// Load the conserved state of a (possibly out-of-block) cell and return it
-// as primitives.  Returns a status bit if the small-value check fires.
-// (Plain loads: with a dependent launch the predecessor writes the state while
-// this kernel's CTAs already exist, which read-only loads do not allow for.)
+__device__ __forceinline__ void prefetch_l2(const double *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
+// Load the conserved state of a (possibly out-of-block) cell.  (Plain loads:
+// with a dependent launch the predecessor writes the state while this
+// kernel's CTAs already exist, which read-only loads do not allow for.)
 template <bool MHD, int NDIR, bool GLM, int NDIM, int BN = BN16>
-__device__ __forceinline__ uint32_t load_prim(const StageArgs &A, int b, int i, int j, int k,
-                                              double *w) {
+__device__ __forceinline__ void load_cons(const StageArgs &A, int b, int i, int j, int k, double *w) {
   using V = Vars<MHD, NDIR, GLM>;
   uint32_t flip;
   const int blk = resolve_cell<NDIM>(A, b, i, j, k, flip, BN);
@@ -241,12 +241,24 @@ __device__ __forceinline__ uint32_t load_prim(const StageArgs &A, int b, int i, 
       w[v] = ((flip >> v) & 1u) ? -x : x;
     }
   }
+}
+
+// A loaded state as primitives.  Returns a status bit if the small-value
+// check fires.
+template <bool MHD, int NDIR, bool GLM>
+__device__ __forceinline__ uint32_t cons_to_prim(const PhysParams &P, double *w) {
   uint32_t st = 0;
-  if (A.P.fix_small_values) {
-    if (small_values<double, MHD, NDIR, GLM>(w, false, A.P) && A.P.small_values_method != 1) st |= ST_SMALL_VALUE;
+  if (P.fix_small_values) {
+    if (small_values<double, MHD, NDIR, GLM>(w, false, P) && P.small_values_method != 1) st |= ST_SMALL_VALUE;
   }
-  to_primitive<MHD, NDIR, GLM>(w, A.P);
+  to_primitive<MHD, NDIR, GLM>(w, P);
   return st;
+}
+
+template <bool MHD, int NDIR, bool GLM, int NDIM, int BN = BN16>
+__device__ __forceinline__ uint32_t load_prim(const StageArgs &A, int b, int i, int j, int k, double *w) {
+  load_cons<MHD, NDIR, GLM, NDIM, BN>(A, b, i, j, k, w);
+  return cons_to_prim<MHD, NDIR, GLM>(A.P, w);
 }
 
 // Interface flux from reconstructed primitive left/right states: small-value
@@ -921,10 +933,7 @@ __global__ void __launch_bounds__(StageOcc<TF, MHD, NDIM, LIM, BN, VAR>::THREADS
           double w[NW];
 #pragma unroll
           for (int v = 0; v < NW; ++v) w[v] = double(tv.center(s2, v, ci, cj));
-          if (P.fix_small_values) {
-            if (small_values<double, MHD, NDIR, GLM>(w, false, P) && P.small_values_method != 1) stb |= ST_SMALL_VALUE;
-          }
-          to_primitive<MHD, NDIR, GLM>(w, P);
+          stb |= cons_to_prim<MHD, NDIR, GLM>(P, w);
 #pragma unroll
           for (int v = 0; v < NW; ++v) tv.center(s2, v, ci, cj) = TF(w[v]);
         }
@@ -969,6 +978,16 @@ __global__ void __launch_bounds__(StageOcc<TF, MHD, NDIM, LIM, BN, VAR>::THREADS
         const size_t o = cell_offset<NDIM>(b, NW, v, bi, bj, k, BN);
         const double win = A.uin[o];
         acc[v] = (A.a_base == 0.0) ? win : A.a_base * A.ubase[o] + A.b_in * win;
+      }
+    }
+    // 3-D MHD: the next plane's RK base and the plane staged next from DRAM to
+    // L2, one thread per 128-byte row (128^3 FP64 3.35 -> 3.31 ms a pass of two
+    // steps; 2-D and hydrodynamics measured up to 4 % slower with it)
+    if (MHD && NDIM == 3 && update && cell_thread && (ci & 15) == 0) {
+#pragma unroll
+      for (int v = 0; v < NW; ++v) {
+        if (A.a_base != 0.0 && k + 1 < BN) prefetch_l2(A.ubase + cell_offset<NDIM>(b, NW, v, bi, bj, k + 1, BN));
+        if (k + HW + 1 < BN) prefetch_l2(A.uin + cell_offset<NDIM>(b, NW, v, bi, bj, k + HW + 1, BN));
       }
     }
     __syncthreads();

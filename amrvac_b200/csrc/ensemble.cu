@@ -16,10 +16,11 @@
 //
 // Per-instance state on the device: dt, time, time_max, dx, solver, limiter,
 // done flag, step count and the getdt reduction word.  One step is
-//   getdt (per-instance max of the maxsum courant number) -> finalize (dt per
-//   instance, dtmin check, final_dt_reduction, exit test) -> RK stages ->
-//   advance time,
-// captured into a CUDA graph of several steps.
+//   getdt (per-instance max of the maxsum courant number; its last CTA then
+//   finalizes every instance: dt, dtmin check, final_dt_reduction, exit test,
+//   time update) -> RK stages,
+// each kernel launched dependent on the one before, captured into a CUDA
+// graph of several steps.
 #include <cuda_runtime.h>
 
 #include <algorithm>

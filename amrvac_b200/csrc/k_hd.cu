@@ -20,6 +20,15 @@ bool lookup_hd(const KernelKey &k, KernelSet *out) {
     *out = Launch<false, 2, false, 2, SOLVER_HLLC, LIM_VANLEER, BS_EINFELDT>::set();
     return true;
   }
+  // the default bound speed compiled in: cmaxmean reads the conserved states, and
+  // forming them cost registers (3-D HLLC 96x80x112 0.124 -> 0.121 ms per stage,
+  // 64x48x64 0.045 -> 0.042)
+  if (k.boundspeed == BS_EINFELDT) {
+    if (k.ndim == 2 && k.solver == SOLVER_HLL) { *out = Launch<false, 2, false, 2, SOLVER_HLL, 0, BS_EINFELDT>::set(); return true; }
+    if (k.ndim == 2 && k.solver == SOLVER_HLLC) { *out = Launch<false, 2, false, 2, SOLVER_HLLC, 0, BS_EINFELDT>::set(); return true; }
+    if (k.ndim == 3 && k.solver == SOLVER_HLL) { *out = Launch<false, 3, false, 3, SOLVER_HLL, 0, BS_EINFELDT>::set(); return true; }
+    if (k.ndim == 3 && k.solver == SOLVER_HLLC) { *out = Launch<false, 3, false, 3, SOLVER_HLLC, 0, BS_EINFELDT>::set(); return true; }
+  }
 #define AMRVAC_HD(ND, S)                                        \
   if (k.ndim == ND && k.solver == S) {                          \
     *out = Launch<false, ND, false, ND, S>::set();              \

@@ -23,7 +23,9 @@
 // y-faces of the top row (288 faces: a second round of one warp), per-cell
 // accumulation, the remaining 16x16 y-faces, accumulation, then each cell
 // thread computes its own z-face k+1/2 and keeps the k-1/2 flux in
-// registers.  Variants of the same kernel: the MUSCL-Hancock predictor
+// registers.  In 2-D hydrodynamics the faces of both directions are one phase
+// (merged_faces).  A face whose flux is not finite, or whose limiter is near a
+// blending band, is recomputed by the thread that owns it.  Variants of the same kernel: the MUSCL-Hancock predictor
 // (per-cell edge fluxes, no Riemann solver) and dimensionally split sweeps
 // (one direction per launch).
 #pragma once
@@ -1200,7 +1202,8 @@ __global__ void __launch_bounds__(StageOcc<TF, MHD, NDIM, LIM, BN, VAR>::THREADS
 #pragma unroll
             for (int v = 0; v < NW; ++v) {
               const int vo = var_off(v, rot);
-              face_states<TF, L, FASTF, cada3_short<TF, NDIM, LIM>, !FASTF || LIM == 0>(
+              face_states<TF, L, FASTF, cada3_short<TF, NDIM, LIM>, !FASTF || LIM == 0,
+                          !(MHD && NDIM == 3)>(
                   P.limiter, smem[base[0] + vo], smem[base[1] + vo], smem[base[2] + vo], smem[base[3] + vo], rd, wLp[v],
                   wRp[v], special);
             }

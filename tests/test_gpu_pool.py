@@ -54,9 +54,11 @@ def test_closed_contexts_give_memory_back():
     from amrvac_b200 import Context, make_cfg
     torch.cuda.synchronize()
     before = torch.cuda.mem_get_info()[0]
-    # 1024^2 HD: 32 MB per register with its headroom 42 MB, three registers, six contexts
+    # 1024^2 HD: 32 MB per register, 42 MB with its headroom, three registers,
+    # twelve contexts: 1.5 GB, of which the pool may hold KEEP already (what
+    # earlier contexts left), so at least 1.2 GB > 2 KEEP are new
     ctxs = []
-    for _ in range(6):
+    for _ in range(12):
         c = Context(make_cfg(physics="hd", ndim=2, gamma=1.4, flux_scheme="hllc", limiter="vanleer"))
         c.set_uniform_grid([1024, 1024], [0.0] * 2, [1.0] * 2)
         ctxs.append(c)

@@ -555,10 +555,8 @@ __device__ __forceinline__ bool near_one(float, float) { return false; }
 // slope_impl, except with R2 (limiter fixed to cada3): then it is
 // (cada3_radius dx)^2 and tmpeta <= 1 is tested as a^2 + b^2 <= rdel without
 // the product.  With the limiter fixed to cada3 and BLEND false the blending
-// band is left out: a face near it gets `special` and is recomputed.  HALF:
-// vanleer's short form (2-D HLLC 2048^2 3.59 -> 3.50 ms, but 1 % slower in the
-// 3-D MHD kernel, whose registers it shifts: the four-level blast 9.27 -> 9.36).
-template <class T, int LIM, int FAST = 0, bool R2 = false, bool BLEND = true, bool HALF = true>
+// band is left out: a face near it gets `special` and is recomputed.
+template <class T, int LIM, int FAST = 0, bool R2 = false, bool BLEND = true>
 __device__ __forceinline__ void face_states(int lim_rt, T q0, T q1, T q2, T q3, T rdel, T &wL, T &wR, bool &special) {
   constexpr T eps = T(1.4901161193847656e-08);  // sqrt(epsilon(1d0)) = 2**-26
   const int lim = LIM ? LIM : lim_rt;
@@ -600,9 +598,10 @@ __device__ __forceinline__ void face_states(int lim_rt, T q0, T q1, T q2, T q3, 
       }
       ldw = pl * d1;  // phi * a (left), phi * b (right): both d1
       rdw = pr * d1;
-    } else if (LIM == LIM_VANLEER && HALF) {
+    } else if (LIM == LIM_VANLEER) {
       // half the slope, max(a b, 0) / (a + b + qsmall): the reference's factors
-      // 2 and 1/2 cancel exactly, so the bits are those of the longer form
+      // 2 and 1/2 cancel exactly, so the bits are those of the longer form (2-D
+      // HLLC 2048^2 3.59 -> 3.50 ms, the four-level blast 9.39 -> 9.31)
       constexpr T qsmall = T(1.0e-12);
       wL = q1 + div_f<FAST>(max_(d0 * d1, T(0.0)), d1 + d0 + qsmall);
       wR = q2 - div_f<FAST>(max_(d1 * d2, T(0.0)), d2 + d1 + qsmall);

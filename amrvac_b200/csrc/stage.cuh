@@ -1202,8 +1202,7 @@ __global__ void __launch_bounds__(StageOcc<TF, MHD, NDIM, LIM, BN, VAR>::THREADS
 #pragma unroll
             for (int v = 0; v < NW; ++v) {
               const int vo = var_off(v, rot);
-              face_states<TF, L, FASTF, cada3_short<TF, NDIM, LIM>, !FASTF || LIM == 0,
-                          !(MHD && NDIM == 3)>(
+              face_states<TF, L, FASTF, cada3_short<TF, NDIM, LIM>, !FASTF || LIM == 0>(
                   P.limiter, smem[base[0] + vo], smem[base[1] + vo], smem[base[2] + vo], smem[base[3] + vo], rd, wLp[v],
                   wRp[v], special);
             }

@@ -69,6 +69,7 @@ struct amrvac_ctx {
   BcSpec bc;
   SrlMaps maps;
   cudaStream_t stream = nullptr;
+  int device = 0;        // the device that was current when the context was made
   int nblocks = 0;
   int bn = 16;           // block edge (block_nx)
   size_t per_block = 0;  // doubles per block per variable (bn^ndim)
@@ -173,12 +174,23 @@ static cudaError_t pool_alloc(double **p, size_t bytes, cudaStream_t s) {
 static void pool_free(double *p, cudaStream_t s) {
   if (p) cudaFreeAsync(p, s);
 }
-// Waits for the device as a cudaFree does, before registers go back to the
-// pool: work that the caller queued on other streams may still read them
+// The context's device current for a scope.
+struct DeviceScope {
+  int prev = -1;
+  explicit DeviceScope(int dev) {
+    int cur = dev;
+    if (cudaGetDevice(&cur) == cudaSuccess && cur != dev && cudaSetDevice(dev) == cudaSuccess) prev = cur;
+  }
+  ~DeviceScope() {
+    if (prev >= 0) cudaSetDevice(prev);
+  }
+};
+// Waits for everything on the context's device, before registers are given
+// back: work that the caller queued on other streams may still read them
 // through amrvac_gpu_register_ptr.
-static void wait_as_free() {
-  void *q = nullptr;
-  if (cudaMalloc(&q, 256) == cudaSuccess) cudaFree(q);
+static cudaError_t wait_device(const amrvac_ctx *c) {
+  DeviceScope on(c->device);
+  return cudaDeviceSynchronize();
 }
 
 // Grow-only device buffer: reallocates (without keeping the contents) only
@@ -798,9 +810,9 @@ int amrvac_gpu_create(const amrvac_cfg *cfg, amrvac_ctx **out) {
   }
   c->zchunk = valid_zchunk(bn, k.zchunk) ? k.zchunk : 0;
   {
-    int dev = 0, nsm = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    int nsm = 148;
+    cudaGetDevice(&c->device);
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device);
     c->wave_ctas = nsm * c->ks.ctas_per_sm();
     for (int v = 0; v < c->ks.nvar; ++v) c->wave_v[v] = nsm * c->ks.ctas_v[v]();
   }
@@ -846,12 +858,16 @@ int amrvac_gpu_create(const amrvac_cfg *cfg, amrvac_ctx **out) {
 
 int amrvac_gpu_destroy(amrvac_ctx *c) {
   if (!c) return AMRVAC_E_ARG;
-  if (c->stream) cudaStreamSynchronize(c->stream);
+  // registers that may still be read are not given back: after a failed wait
+  // they are left to the end of the process
+  const cudaError_t waited = wait_device(c);
   if (c->graph) cudaGraphExecDestroy(c->graph);
-  cudaFree(c->d_scal);  // first: it waits for the device (wait_as_free)
-  for (int r = 0; r < 4; ++r) pool_free(c->pool[r], c->stream);
-  for (int r = 0; r < 3; ++r) pool_free(c->d_adj[r], c->stream);
-  pool_free(c->sv_snap, c->stream);
+  if (waited == cudaSuccess) {
+    for (int r = 0; r < 4; ++r) pool_free(c->pool[r], c->stream);
+    for (int r = 0; r < 3; ++r) pool_free(c->d_adj[r], c->stream);
+    pool_free(c->sv_snap, c->stream);
+  }
+  cudaFree(c->d_scal);
   cudaFree(c->d_nbr);
   cudaFree(c->d_dx);
   cudaFree(c->d_red);
@@ -869,7 +885,7 @@ int amrvac_gpu_destroy(amrvac_ctx *c) {
   cudaFree(c->amr_ints);
   if (c->stream) cudaStreamDestroy(c->stream);
   delete c;
-  return 0;
+  return waited == cudaSuccess ? 0 : cuda_fail(waited, "amrvac_gpu_destroy");
 }
 
 static int set_blocks_impl(amrvac_ctx *c, int nblocks, const double *dx, const int *neighbor, bool level_jumps,
@@ -943,7 +959,7 @@ static int set_blocks_impl(amrvac_ctx *c, int nblocks, const double *dx, const i
   } else if (adopt_reg0) {
     // regrid into a new, larger buffer: the other registers follow its size
     const size_t cap = (size_t)nblocks + nblocks / 4 + 1;
-    wait_as_free();
+    CK(wait_device(c));
     for (int r = 0; r < 4; ++r) { pool_free(c->pool[r], c->stream); c->pool[r] = nullptr; }
     c->pool_cap = 0;
     c->pool[0] = adopt_reg0;
@@ -952,7 +968,7 @@ static int set_blocks_impl(amrvac_ctx *c, int nblocks, const double *dx, const i
     c->pool_cap = cap;
   } else {
     if ((size_t)nblocks > c->pool_cap || !c->pool[0]) {
-      if (c->pool[0]) wait_as_free();
+      if (c->pool[0]) CK(wait_device(c));
       for (int r = 0; r < 4; ++r) { pool_free(c->pool[r], c->stream); c->pool[r] = nullptr; }
       c->pool_cap = 0;
       const size_t cap = (size_t)nblocks + nblocks / 4 + 1;

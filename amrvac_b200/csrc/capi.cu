@@ -27,7 +27,10 @@ int fail(int code, const std::string &msg) {
   return code;
 }
 
+// (The runtime's last error is cleared with the report, so that the next
+// launch checked by cudaGetLastError does not report it again.)
 int cuda_fail(cudaError_t e, const char *where) {
+  cudaGetLastError();
   g_err = std::string(where) + ": " + cudaGetErrorString(e);
   return AMRVAC_E_CUDA;
 }
@@ -589,7 +592,10 @@ int launch_step(amrvac_ctx *c) {
 
 namespace amrvac {
 // Sets this thread's last-error text for entry points defined in other units.
-int record_error(int code, const std::string &msg) { return fail(code, msg); }
+int record_error(int code, const std::string &msg) {
+  if (code == AMRVAC_E_CUDA) cudaGetLastError();
+  return fail(code, msg);
+}
 }  // namespace amrvac
 
 extern "C" {

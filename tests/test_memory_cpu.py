@@ -57,3 +57,17 @@ def test_context_closed_from_another_device(fake):
     assert fake.L.amrvac_gpu_destroy(h) == 0
     assert "cudaDeviceSynchronize 0 = 0" in fake.log()
     assert [l for l in fake.log() if l.startswith("cudaSetDevice")][-1].split()[1] == "1"
+
+
+def test_a_failed_allocation_is_reported_once(fake):
+    """The runtime's last error goes with the call that reports it: a later
+    kernel launch does not report it again."""
+    import ctypes
+    import numpy as np
+    h = fake.create(**HD2)
+    assert fake.grid(h, [64, 64]) == 0
+    w = np.zeros((16, 4, 1, 20, 20))
+    fake.fail("cudaMalloc")
+    assert fake.L.amrvac_gpu_upload(h, 0, 0, 16, w.ctypes.data_as(ctypes.POINTER(ctypes.c_double))) < 0
+    assert "out of memory" in fake.error()
+    assert fake.L.amrvac_gpu_step_dt(h, 1e-3) == 0, fake.error()

@@ -6,7 +6,6 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
-#include <mutex>
 #include <string>
 #include <vector>
 
@@ -14,6 +13,7 @@
 #include "adjoint.cuh"
 #include "amr.cuh"
 #include "aux.cuh"
+#include "devmem.cuh"
 #include "kernels.cuh"
 
 using namespace amrvac;
@@ -126,57 +126,6 @@ struct amrvac_ctx {
   size_t amr_gbuf_cap = 0, amr_pflux_cap = 0, amr_bxmin_cap = 0, amr_ints_cap = 0;
 };
 
-// The registers and the adjoint's work registers come from a memory pool of the
-// library's own, one per device: a program that makes and closes contexts
-// (adjoint.solve makes two per gradient) otherwise pays for mapping and
-// unmapping their memory each time (512^2, 40 steps: 6 of 18.5 ms, and far
-// more when the frees of one call meet the work of the next).  The pool keeps
-// at most POOL_KEEP bytes that nothing uses (the driver gives the rest back at
-// the next synchronisation), and gives those back when an allocation fails.
-// Allocations and frees are ordered on the context's stream, whichever thread
-// makes them.
-constexpr unsigned long long POOL_KEEP = 256ull << 20;
-static cudaError_t device_pool(cudaMemPool_t *out) {
-  static std::mutex m;
-  static cudaMemPool_t pools[64] = {};
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
-  if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
-  std::lock_guard<std::mutex> lock(m);
-  if (!pools[dev]) {
-    cudaMemPoolProps props;
-    std::memset(&props, 0, sizeof(props));
-    props.allocType = cudaMemAllocationTypePinned;
-    props.handleTypes = cudaMemHandleTypeNone;
-    props.location.type = cudaMemLocationTypeDevice;
-    props.location.id = dev;
-    cudaMemPool_t q;
-    if ((e = cudaMemPoolCreate(&q, &props)) != cudaSuccess) return e;
-    unsigned long long keep = POOL_KEEP;
-    if ((e = cudaMemPoolSetAttribute(q, cudaMemPoolAttrReleaseThreshold, &keep)) != cudaSuccess) return e;
-    pools[dev] = q;
-  }
-  *out = pools[dev];
-  return cudaSuccess;
-}
-static cudaError_t pool_alloc(double **p, size_t bytes, cudaStream_t s) {
-  *p = nullptr;
-  cudaMemPool_t q;
-  cudaError_t e = device_pool(&q);
-  if (e != cudaSuccess) return e;
-  e = cudaMallocFromPoolAsync(reinterpret_cast<void **>(p), bytes, q, s);
-  if (e == cudaErrorMemoryAllocation) {
-    cudaGetLastError();
-    cudaMemPoolTrimTo(q, 0);
-    e = cudaMallocFromPoolAsync(reinterpret_cast<void **>(p), bytes, q, s);
-  }
-  if (e != cudaSuccess) *p = nullptr;
-  return e;
-}
-static void pool_free(double *p, cudaStream_t s) {
-  if (p) cudaFreeAsync(p, s);
-}
 // The context's device current for a scope.
 struct DeviceScope {
   int prev = -1;
@@ -869,9 +818,9 @@ int amrvac_gpu_destroy(amrvac_ctx *c) {
   const cudaError_t waited = wait_device(c);
   if (c->graph) cudaGraphExecDestroy(c->graph);
   if (waited == cudaSuccess) {
-    for (int r = 0; r < 4; ++r) pool_free(c->pool[r], c->stream);
-    for (int r = 0; r < 3; ++r) pool_free(c->d_adj[r], c->stream);
-    pool_free(c->sv_snap, c->stream);
+    for (int r = 0; r < 4; ++r) register_free(c->pool[r]);
+    for (int r = 0; r < 3; ++r) register_free(c->d_adj[r]);
+    register_free(c->sv_snap);
   }
   cudaFree(c->d_scal);
   cudaFree(c->d_nbr);
@@ -966,24 +915,24 @@ static int set_blocks_impl(amrvac_ctx *c, int nblocks, const double *dx, const i
     // regrid into a new, larger buffer: the other registers follow its size
     const size_t cap = (size_t)nblocks + nblocks / 4 + 1;
     CK(wait_device(c));
-    for (int r = 0; r < 4; ++r) { pool_free(c->pool[r], c->stream); c->pool[r] = nullptr; }
+    for (int r = 0; r < 4; ++r) { register_free(c->pool[r]); c->pool[r] = nullptr; }
     c->pool_cap = 0;
     c->pool[0] = adopt_reg0;
     for (int r = 1; r < c->nreg; ++r)
-      CK(pool_alloc(&c->pool[r], sizeof(double) * c->per_block * c->nw * cap, c->stream));
+      CK(register_alloc(&c->pool[r], sizeof(double) * c->per_block * c->nw * cap));
     c->pool_cap = cap;
   } else {
     if ((size_t)nblocks > c->pool_cap || !c->pool[0]) {
       if (c->pool[0]) CK(wait_device(c));
-      for (int r = 0; r < 4; ++r) { pool_free(c->pool[r], c->stream); c->pool[r] = nullptr; }
+      for (int r = 0; r < 4; ++r) { register_free(c->pool[r]); c->pool[r] = nullptr; }
       c->pool_cap = 0;
       const size_t cap = (size_t)nblocks + nblocks / 4 + 1;
       for (int r = 0; r < c->nreg; ++r)
-        CK(pool_alloc(&c->pool[r], sizeof(double) * c->per_block * c->nw * cap, c->stream));
+        CK(register_alloc(&c->pool[r], sizeof(double) * c->per_block * c->nw * cap));
       c->pool_cap = cap;
       if (c->sv_on) {
-        pool_free(c->sv_snap, c->stream);
-        CK(pool_alloc(&c->sv_snap, sizeof(double) * c->per_block * c->nw * cap, c->stream));
+        register_free(c->sv_snap);
+        CK(register_alloc(&c->sv_snap, sizeof(double) * c->per_block * c->nw * cap));
       }
     }
     for (int r = 0; r < c->nreg; ++r) CK(cudaMemsetAsync(c->pool[r], 0, bytes, c->stream));
@@ -1004,7 +953,7 @@ static int set_blocks_impl(amrvac_ctx *c, int nblocks, const double *dx, const i
   CK(cudaMemsetAsync(c->d_block_status, 0, sizeof(uint32_t) * nblocks, c->stream));
   CK(cudaStreamSynchronize(c->stream));
   c->h_dx = dxb;
-  for (int r = 0; r < 3; ++r) { pool_free(c->d_adj[r], c->stream); c->d_adj[r] = nullptr; }
+  for (int r = 0; r < 3; ++r) { register_free(c->d_adj[r]); c->d_adj[r] = nullptr; }
   c->adj_prepared = false;
   delete c->amr; c->amr = nullptr;
   return 0;
@@ -1291,7 +1240,7 @@ static int amr_grid_impl(amrvac_ctx *c, int nleaf, const int *leaf, const int *n
     int *d_op = nullptr;
     cudaError_t e = cudaSuccess;
     if ((size_t)nb <= c->pool_cap) newreg = c->pool[1];  // scratch register: swapped in afterwards
-    else e = pool_alloc(&newreg, sizeof(double) * c->per_block * c->nw * ((size_t)nb + nb / 4 + 1), c->stream);
+    else e = register_alloc(&newreg, sizeof(double) * c->per_block * c->nw * ((size_t)nb + nb / 4 + 1));
     if (e == cudaSuccess) e = cudaMalloc(&d_op, sizeof(int) * 9 * (size_t)nb);
     if (e == cudaSuccess)
       e = cudaMemcpyAsync(d_op, ops, sizeof(int) * 9 * (size_t)nb, cudaMemcpyHostToDevice, c->stream);
@@ -1308,12 +1257,13 @@ static int amr_grid_impl(amrvac_ctx *c, int nleaf, const int *leaf, const int *n
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     cudaFree(d_op);
     if (e != cudaSuccess) {
-      if (newreg != c->pool[1]) pool_free(newreg, c->stream);
+      cudaStreamSynchronize(c->stream);  // the remap may still run
+      if (newreg != c->pool[1]) register_free(newreg);
       return cuda_fail(e, "amr_regrid");
     }
   }
   if (int r = set_blocks_impl(c, nb, dx.data(), nbr.data(), true, newreg)) {
-    if (newreg && c->pool[0] != newreg && c->pool[1] != newreg) pool_free(newreg, c->stream);
+    if (newreg && c->pool[0] != newreg && c->pool[1] != newreg) register_free(newreg);
     return r;
   }
   // device copies
@@ -2038,7 +1988,7 @@ static int adjoint_step_impl(amrvac_ctx *c, const double *u0, const double *u1, 
   }
   const size_t bytes = sizeof(double) * c->per_block * c->nw * c->nblocks;
   for (int r = 0; r < 3; ++r)
-    if (!c->d_adj[r]) CK(pool_alloc(&c->d_adj[r], bytes, c->stream));
+    if (!c->d_adj[r]) CK(register_alloc(&c->d_adj[r], bytes));
   double *S1 = c->d_adj[0], *S2 = c->d_adj[1], *S3 = c->d_adj[2];
   // stage inputs: the caller's buffers, or registers 0..2 recomputed below
   const double *W[3] = {u0 ? u0 : c->pool[0], u1 ? u1 : c->pool[1], u2 ? u2 : c->pool[2]};

@@ -1,0 +1,23 @@
+// Device memory of contexts and ensembles.
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include <cstddef>
+
+namespace amrvac {
+
+// The large registers of contexts (block registers, the adjoint's, the copy of
+// 'average').  Plain cudaMalloc memory, of which the library keeps up to
+// REGISTER_KEEP bytes that no context uses: a program that makes and closes
+// contexts (adjoint.solve makes two per gradient) otherwise pays for mapping
+// and unmapping the same sizes each time.
+//
+// register_free expects that the caller has waited for all work on the register:
+// it is idle, so any context on any stream may have it next.  One larger than
+// the bound goes back to the driver at once, as do the oldest above it.
+constexpr size_t REGISTER_KEEP = (size_t)256 << 20;
+cudaError_t register_alloc(double **p, size_t bytes);
+void register_free(double *p);
+
+}  // namespace amrvac

@@ -14,7 +14,6 @@
 #include <map>
 #include <mutex>
 #include <string>
-#include <vector>
 
 namespace {
 
@@ -55,15 +54,6 @@ cudaError_t done(const char *fn, const char *args, cudaError_t e) {
   logf("%s %s = %d", fn, args, (int)e);
   if (e != cudaSuccess) last = e;
   return e;
-}
-std::vector<void *> pending;  // freed on a stream, not yet seen by the host
-void seen() {
-  for (void *p : pending) {
-    used -= live[p].bytes;
-    live.erase(p);
-    std::free(p);
-  }
-  pending.clear();
 }
 cudaError_t plain(const char *fn, const char *args = "") {
   std::lock_guard<std::mutex> g(mtx);
@@ -174,7 +164,6 @@ cudaError_t cudaDeviceGetAttribute(int *v, cudaDeviceAttr a, int) {
 cudaError_t cudaDeviceSynchronize() {
   char a[16];
   std::snprintf(a, sizeof a, "%d", cur_dev);
-  seen();
   return plain("cudaDeviceSynchronize", a);
 }
 cudaError_t cudaMalloc(void **p, size_t n) { return alloc("cudaMalloc", p, n, true); }
@@ -209,10 +198,7 @@ cudaError_t cudaStreamCreateWithFlags(cudaStream_t *s, unsigned) {
   return plain("cudaStreamCreateWithFlags");
 }
 cudaError_t cudaStreamDestroy(cudaStream_t) { return plain("cudaStreamDestroy"); }
-cudaError_t cudaStreamSynchronize(cudaStream_t) {
-  seen();
-  return plain("cudaStreamSynchronize");
-}
+cudaError_t cudaStreamSynchronize(cudaStream_t) { return plain("cudaStreamSynchronize"); }
 cudaError_t cudaStreamBeginCapture(cudaStream_t, cudaStreamCaptureMode) { return plain("cudaStreamBeginCapture"); }
 cudaError_t cudaStreamEndCapture(cudaStream_t, cudaGraph_t *g) {
   *g = (cudaGraph_t)1;
@@ -247,21 +233,6 @@ static cudaError_t launch(dim3 g, dim3 b) {
 cudaError_t cudaLaunchKernel(const void *, dim3 g, dim3 b, void **, size_t, cudaStream_t) { return launch(g, b); }
 cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t *c, const void *, void **) {
   return launch(c->gridDim, c->blockDim);
-}
-
-// ---- stream-ordered pools: freed memory counts until the host has waited
-cudaError_t cudaMemPoolCreate(cudaMemPool_t *q, const cudaMemPoolProps *) {
-  *q = (cudaMemPool_t)1;
-  return plain("cudaMemPoolCreate");
-}
-cudaError_t cudaMemPoolSetAttribute(cudaMemPool_t, cudaMemPoolAttr, void *) { return plain("cudaMemPoolSetAttribute"); }
-cudaError_t cudaMemPoolTrimTo(cudaMemPool_t, size_t) { return plain("cudaMemPoolTrimTo"); }
-cudaError_t cudaMallocFromPoolAsync(void **p, size_t n, cudaMemPool_t, cudaStream_t) {
-  return alloc("cudaMallocFromPoolAsync", p, n, true);
-}
-cudaError_t cudaFreeAsync(void *p, cudaStream_t) {
-  pending.push_back(p);
-  return plain("cudaFreeAsync");
 }
 
 }  // extern "C"

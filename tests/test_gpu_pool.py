@@ -1,6 +1,6 @@
-"""The pool behind the contexts' registers: contexts made, stepped and closed by
-several threads at once give the bits a context alone gives, and closing large
-ones gives their memory back down to the pool's bound.
+"""The contexts' registers, some of which are kept for the next context: contexts
+made, stepped and closed by several threads at once give the bits a context
+alone gives, and closing large ones gives their memory back down to the bound.
 """
 import threading
 
@@ -11,7 +11,7 @@ from tests import _problems as P
 
 pytestmark = pytest.mark.gpu
 
-KEEP = 256 << 20  # capi.cu POOL_KEEP
+KEEP = 256 << 20  # devmem.cuh REGISTER_KEEP
 
 
 def _run(n, out, key, reps):
@@ -55,7 +55,7 @@ def test_closed_contexts_give_memory_back():
     torch.cuda.synchronize()
     before = torch.cuda.mem_get_info()[0]
     # 1024^2 HD: 32 MB per register, 42 MB with its headroom, three registers,
-    # twelve contexts: 1.5 GB, of which the pool may hold KEEP already (what
+    # twelve contexts: 1.5 GB, of which the library may hold KEEP already (what
     # earlier contexts left), so at least 1.2 GB > 2 KEEP are new
     ctxs = []
     for _ in range(12):
@@ -71,3 +71,18 @@ def test_closed_contexts_give_memory_back():
     kept = before - torch.cuda.mem_get_info()[0]
     # the bound, and the driver's granularity of a few blocks of 32 MB
     assert kept <= KEEP + (128 << 20), (used, kept)
+
+
+def test_memory_is_back_when_close_returns():
+    """No wait of the caller's after the close."""
+    import torch
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from amrvac_b200 import Context, make_cfg
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    c = Context(make_cfg(physics="hd", ndim=2, gamma=1.4, flux_scheme="hllc", limiter="vanleer"))
+    c.set_uniform_grid([4096, 4096], [0.0] * 2, [1.0] * 2)  # three registers of 671 MB
+    c.run(1)
+    c.close()
+    assert before - torch.cuda.mem_get_info()[0] <= KEEP + (128 << 20)

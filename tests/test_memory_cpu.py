@@ -28,13 +28,13 @@ def test_registers_are_given_back_behind_a_wait_for_the_device(fake):
     fake.grid(h, [128, 128])
     log = fake.log()
     wait = log.index("cudaDeviceSynchronize 0 = 0")
-    assert wait < _first(log, "cudaFree", "cudaFreeAsync", "cudaMalloc", "cudaMallocFromPoolAsync"), log
+    assert wait < _first(log, "cudaFree", "cudaMalloc"), log
     fake.L.fake_reset()
     assert fake.grid(h, [128, 128]) == 0
     fake.clear()
     assert fake.L.amrvac_gpu_destroy(h) == 0
     log = fake.log()
-    assert log.index("cudaDeviceSynchronize 0 = 0") < _first(log, "cudaFree", "cudaFreeAsync"), log
+    assert log.index("cudaDeviceSynchronize 0 = 0") < _first(log, "cudaFree"), log
 
 
 def test_a_failed_wait_is_reported(fake):
@@ -43,7 +43,7 @@ def test_a_failed_wait_is_reported(fake):
     fake.clear()
     fake.fail("cudaDeviceSynchronize", err=700)
     assert fake.grid(h, [128, 128]) < 0
-    assert _first(fake.log(), "cudaFree", "cudaFreeAsync") == len(fake.log())  # nothing was given back
+    assert _first(fake.log(), "cudaFree") == len(fake.log())  # nothing was given back
     fake.fail("cudaDeviceSynchronize", err=700)
     assert fake.L.amrvac_gpu_destroy(h) < 0
 
@@ -71,3 +71,44 @@ def test_a_failed_allocation_is_reported_once(fake):
     assert fake.L.amrvac_gpu_upload(h, 0, 0, 16, w.ctypes.data_as(ctypes.POINTER(ctypes.c_double))) < 0
     assert "out of memory" in fake.error()
     assert fake.L.amrvac_gpu_step_dt(h, 1e-3) == 0, fake.error()
+
+
+KEEP = 256 << 20  # devmem.cuh REGISTER_KEEP
+
+
+def test_grown_registers_fit_where_the_old_ones_were(fake):
+    """set_blocks on a device that holds the new registers only once the old
+    ones are gone."""
+    h = fake.create(**HD2)
+    assert fake.grid(h, [1600, 1600]) == 0  # 3 x 102 MB
+    fake.L.fake_capacity(fake.L.fake_used() + (260 << 20))
+    assert fake.grid(h, [2048, 2048]) == 0, fake.error()  # 3 x 168 MB
+    assert fake.L.amrvac_gpu_destroy(h) == 0
+
+
+def test_closed_context_keeps_no_more_than_the_bound(fake):
+    """Without any wait of the caller's after the close."""
+    for n in (2048, 1024, 512, 2048, 4096):  # one register: 168, 42, 10, 168, 671 MB
+        h = fake.create(**HD2)
+        assert fake.grid(h, [n, n]) == 0
+        used = fake.L.fake_used()
+        assert fake.L.amrvac_gpu_destroy(h) == 0
+        log = [l for l in fake.log() if l.startswith("cudaDeviceSynchronize") or l.startswith("cudaStreamSynchronize")]
+        assert log and fake.L.fake_used() <= min(KEEP, used)
+
+
+def test_registers_are_used_again(fake):
+    h = fake.create(**HD2)
+    assert fake.grid(h, [512, 512]) == 0
+    assert fake.L.amrvac_gpu_destroy(h) == 0
+    h = fake.create(**HD2)
+    fake.clear()
+    assert fake.grid(h, [512, 512]) == 0
+    assert not [l for l in fake.log() if l.startswith("cudaMalloc") and int(l.split()[1]) > 1 << 20]
+    # a much smaller grid does not sit on a large register
+    small = fake.create(**HD2)
+    assert fake.L.amrvac_gpu_destroy(h) == 0
+    fake.clear()
+    assert fake.grid(small, [256, 256]) == 0
+    assert [l for l in fake.log() if l.startswith("cudaMalloc") and int(l.split()[1]) > 1 << 20]
+    assert fake.L.amrvac_gpu_destroy(small) == 0

@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 
 #include "aux.cuh"
+#include "devmem.cuh"
 #include "kernels.cuh"
 
 namespace amrvac {
@@ -149,7 +150,7 @@ __global__ void wait_probe_kernel(int spins, uint32_t *status) {
 
 cudaError_t run_wait_probe(int spins, uint32_t *flags) {
   uint32_t *d = nullptr;
-  cudaError_t e = cudaMalloc(&d, sizeof(uint32_t));
+  cudaError_t e = device_alloc(&d, sizeof(uint32_t));
   if (e != cudaSuccess) return e;
   if ((e = cudaMemset(d, 0, sizeof(uint32_t))) == cudaSuccess) {
     wait_probe_kernel<<<1, 32>>>(spins, d);
@@ -165,7 +166,7 @@ cudaError_t measure_fp64_peak(double *tflops) {
   if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
   if ((e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
   double *out;
-  if ((e = cudaMalloc(&out, sizeof(double))) != cudaSuccess) return e;
+  if ((e = device_alloc(&out, sizeof(double))) != cudaSuccess) return e;
   cudaEvent_t a, b;
   cudaEventCreate(&a);
   cudaEventCreate(&b);

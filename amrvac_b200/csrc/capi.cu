@@ -154,7 +154,7 @@ static cudaError_t ensure_capacity(T **p, size_t *cap, size_t need) {
   *p = nullptr;
   *cap = 0;
   const size_t n = need + need / 4 + 1;
-  const cudaError_t e = cudaMalloc(p, sizeof(T) * n);
+  const cudaError_t e = device_alloc(p, sizeof(T) * n);
   if (e == cudaSuccess) *cap = n;
   return e;
 }
@@ -782,11 +782,11 @@ int amrvac_gpu_create(const amrvac_cfg *cfg, amrvac_ctx **out) {
   // flag, slowsteps, steps since set_time, a2max_global(1:3) (schmid1)
   const double sc[13] = {0.0, 0.0, 0.0, 1.0e99, 0.0, k.dtmin, k.courantpar, 0.0, double(k.slowsteps), 0.0,
                          0.0, 0.0, 0.0};
-  if ((e = cudaMalloc(&c->d_scal, sizeof(sc))) != cudaSuccess ||
+  if ((e = device_alloc(&c->d_scal, sizeof(sc))) != cudaSuccess ||
       (e = cudaMemcpy(c->d_scal, sc, sizeof(sc), cudaMemcpyHostToDevice)) != cudaSuccess ||
-      (e = cudaMalloc(&c->d_red, 3 * sizeof(unsigned long long))) != cudaSuccess ||
+      (e = device_alloc(&c->d_red, 3 * sizeof(unsigned long long))) != cudaSuccess ||
       (e = cudaMemset(c->d_red, 0, 3 * sizeof(unsigned long long))) != cudaSuccess ||
-      (e = cudaMalloc(&c->d_status, sizeof(uint32_t))) != cudaSuccess ||
+      (e = device_alloc(&c->d_status, sizeof(uint32_t))) != cudaSuccess ||
       (e = cudaMemset(c->d_status, 0, sizeof(uint32_t))) != cudaSuccess) {
     amrvac_gpu_destroy(c);
     return cuda_fail(e, "context allocation");
@@ -802,7 +802,7 @@ int amrvac_gpu_create(const amrvac_cfg *cfg, amrvac_ctx **out) {
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
     const size_t fit = ((size_t)256 << 20) / (sizeof(double) * c->sv_per_cta);
     c->sv_ctas = (int)std::max<size_t>(1, std::min<size_t>(fit, (size_t)nsm));
-    if ((e = cudaMalloc(&c->sv_scratch, sizeof(double) * c->sv_per_cta * c->sv_ctas)) != cudaSuccess) {
+    if ((e = device_alloc(&c->sv_scratch, sizeof(double) * c->sv_per_cta * c->sv_ctas)) != cudaSuccess) {
       amrvac_gpu_destroy(c);
       return cuda_fail(e, "small-value scratch allocation");
     }
@@ -943,9 +943,9 @@ static int set_blocks_impl(amrvac_ctx *c, int nblocks, const double *dx, const i
     c->d_nbr = nullptr; c->d_dx = nullptr; c->d_block_status = nullptr;
     c->nbr_cap = 0;
     const size_t cap = (size_t)nblocks + nblocks / 4 + 1;
-    CK(cudaMalloc(&c->d_nbr, sizeof(int) * 27 * cap));
-    CK(cudaMalloc(&c->d_dx, sizeof(double) * 3 * cap));
-    CK(cudaMalloc(&c->d_block_status, sizeof(uint32_t) * cap));
+    CK(device_alloc(&c->d_nbr, sizeof(int) * 27 * cap));
+    CK(device_alloc(&c->d_dx, sizeof(double) * 3 * cap));
+    CK(device_alloc(&c->d_block_status, sizeof(uint32_t) * cap));
     c->nbr_cap = cap;
   }
   CK(cudaMemcpyAsync(c->d_nbr, nbr.data(), sizeof(int) * nbr.size(), cudaMemcpyHostToDevice, c->stream));
@@ -1241,7 +1241,7 @@ static int amr_grid_impl(amrvac_ctx *c, int nleaf, const int *leaf, const int *n
     cudaError_t e = cudaSuccess;
     if ((size_t)nb <= c->pool_cap) newreg = c->pool[1];  // scratch register: swapped in afterwards
     else e = register_alloc(&newreg, sizeof(double) * c->per_block * c->nw * ((size_t)nb + nb / 4 + 1));
-    if (e == cudaSuccess) e = cudaMalloc(&d_op, sizeof(int) * 9 * (size_t)nb);
+    if (e == cudaSuccess) e = device_alloc(&d_op, sizeof(int) * 9 * (size_t)nb);
     if (e == cudaSuccess)
       e = cudaMemcpyAsync(d_op, ops, sizeof(int) * 9 * (size_t)nb, cudaMemcpyHostToDevice, c->stream);
     if (e == cudaSuccess) {
@@ -1425,7 +1425,7 @@ static int ensure_stage(amrvac_ctx *c, size_t doubles) {
   cudaFree(c->d_stage);
   c->d_stage = nullptr;
   c->stage_doubles = 0;
-  CK(cudaMalloc(&c->d_stage, sizeof(double) * doubles));
+  CK(device_alloc(&c->d_stage, sizeof(double) * doubles));
   c->stage_doubles = doubles;
   return 0;
 }
@@ -1809,7 +1809,7 @@ static int run_points(amrvac_ctx *c, int n, int idim, const double *a, const dou
   const size_t sz = (size_t)n * c->nw;
   double *dev = nullptr;
   const size_t total = sz * 4 + (size_t)n * out_per + (size_t)n;
-  CK(cudaMalloc(&dev, sizeof(double) * total));
+  CK(device_alloc(&dev, sizeof(double) * total));
   double *da = dev, *db = dev + sz, *dc = dev + 2 * sz, *dd = dev + 3 * sz, *dout = dev + 4 * sz,
          *dout2 = dout + (size_t)n * out_per;
   auto up = [&](double *dst, const double *src) -> cudaError_t {
@@ -1862,7 +1862,7 @@ int amrvac_gpu_div_points(int n, const double *x, const double *y, double *q, do
   if (n <= 0 || !x || !y || !q || !r || !seed) return fail(AMRVAC_E_ARG, "div_points: bad arguments");
   const size_t b = sizeof(double) * (size_t)n;
   double *d = nullptr;
-  CK(cudaMalloc(&d, 5 * b));
+  CK(device_alloc(&d, 5 * b));
   cudaError_t e = cudaMemcpy(d, x, b, cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemcpy(d + n, y, b, cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = launch_div_points(n, d, d + n, d + 2 * (size_t)n, d + 3 * (size_t)n, d + 4 * (size_t)n, 0);
@@ -2081,8 +2081,8 @@ int amrvac_gpu_lohner(amrvac_ctx *c, int reg, const double *weight, const int *l
     c->d_amr_err = nullptr;
     c->amr_int_cap = 0;
     const size_t cap = (size_t)c->nblocks + c->nblocks / 4 + 1;
-    CK(cudaMalloc(&c->d_amr_int, sizeof(int) * 2 * cap));
-    CK(cudaMalloc(&c->d_amr_err, sizeof(double) * cap));
+    CK(device_alloc(&c->d_amr_int, sizeof(int) * 2 * cap));
+    CK(device_alloc(&c->d_amr_err, sizeof(double) * cap));
     c->amr_int_cap = cap;
   }
   CK(cudaMemcpyAsync(c->d_amr_int, lev.data(), sizeof(int) * c->nblocks, cudaMemcpyHostToDevice, c->stream));

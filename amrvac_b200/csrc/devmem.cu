@@ -25,6 +25,21 @@ struct Registers {
     cudaFree(it->p);
     kept.erase(it);
   }
+  // cudaMalloc; with the device short of memory the registers kept there go
+  // first (the lock is held)
+  cudaError_t alloc(void **p, size_t bytes, int dev) {
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation && !kept.empty()) {
+      cudaGetLastError();
+      for (auto it = kept.begin(); it != kept.end();) {
+        auto cur = it++;
+        if (cur->dev == dev) drop(cur);
+      }
+      e = cudaMalloc(p, bytes);
+    }
+    if (e != cudaSuccess) *p = nullptr;
+    return e;
+  }
 };
 // (never destroyed: the driver may be gone before static objects are)
 Registers &registers() {
@@ -35,8 +50,7 @@ Registers &registers() {
 }  // namespace
 
 // The smallest kept register that holds `bytes` with at most a quarter to
-// spare (a register is a block count with 25 % headroom), else a new one; with
-// the device short of memory the kept ones of that device go first.
+// spare (a register is a block count with 25 % headroom), else a new one.
 cudaError_t register_alloc(double **p, size_t bytes) {
   *p = nullptr;
   int dev = 0;
@@ -56,18 +70,19 @@ cudaError_t register_alloc(double **p, size_t bytes) {
     R.kept.erase(best);
     return cudaSuccess;
   }
-  e = cudaMalloc(p, bytes);
-  if (e == cudaErrorMemoryAllocation && !R.kept.empty()) {
-    cudaGetLastError();
-    for (auto it = R.kept.begin(); it != R.kept.end();) {
-      auto cur = it++;
-      if (cur->dev == dev) R.drop(cur);
-    }
-    e = cudaMalloc(p, bytes);
-  }
+  e = R.alloc(reinterpret_cast<void **>(p), bytes, dev);
   if (e == cudaSuccess) R.used[*p] = Reg{*p, bytes, dev};
-  else *p = nullptr;
   return e;
+}
+
+cudaError_t device_alloc(void **p, size_t bytes) {
+  *p = nullptr;
+  int dev = 0;
+  const cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  Registers &R = registers();
+  std::lock_guard<std::mutex> lock(R.m);
+  return R.alloc(p, bytes, dev);
 }
 
 void register_free(double *p) {

@@ -20,4 +20,12 @@ constexpr size_t REGISTER_KEEP = (size_t)256 << 20;
 cudaError_t register_alloc(double **p, size_t bytes);
 void register_free(double *p);
 
+// cudaMalloc for everything else of the library's: with the device short of
+// memory the registers kept on it are given back and it is tried again.
+cudaError_t device_alloc(void **p, size_t bytes);
+template <class T>
+cudaError_t device_alloc(T **p, size_t bytes) {
+  return device_alloc(reinterpret_cast<void **>(p), bytes);
+}
+
 }  // namespace amrvac

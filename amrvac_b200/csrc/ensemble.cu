@@ -33,6 +33,7 @@
 
 #include "../../include/amrvac_gpu.h"
 #include "aux.cuh"
+#include "devmem.cuh"
 #include "kernels.cuh"
 
 namespace amrvac {
@@ -730,7 +731,7 @@ int ens_ensure_stage(amrvac_ens *e, size_t doubles) {
   cudaFree(e->d_stage);
   e->d_stage = nullptr;
   e->stage_doubles = 0;
-  ECK(cudaMalloc(&e->d_stage, sizeof(double) * doubles));
+  ECK(device_alloc(&e->d_stage, sizeof(double) * doubles));
   e->stage_doubles = doubles;
   return 0;
 }
@@ -889,10 +890,10 @@ int amrvac_ens_create(const amrvac_cfg *cfg, int ninst, const amrvac_ens_instanc
   // ---- device memory
   cudaError_t ce;
 #define EALLOC(ptr, bytes)                                           \
-  if ((ce = cudaMalloc(&(ptr), (bytes))) != cudaSuccess) {           \
+  if ((ce = device_alloc(&(ptr), (bytes))) != cudaSuccess) {         \
     free_all(e);                                                     \
     delete e;                                                        \
-    return ecuda(ce, "cudaMalloc");                                  \
+    return ecuda(ce, "device_alloc");                                \
   }
   if ((ce = cudaStreamCreateWithFlags(&e->stream, cudaStreamNonBlocking)) != cudaSuccess) {
     delete e;

@@ -67,7 +67,7 @@ def test_a_failed_allocation_is_reported_once(fake):
     h = fake.create(**HD2)
     assert fake.grid(h, [64, 64]) == 0
     w = np.zeros((16, 4, 1, 20, 20))
-    fake.fail("cudaMalloc")
+    fake.fail("cudaMalloc", times=2)
     assert fake.L.amrvac_gpu_upload(h, 0, 0, 16, w.ctypes.data_as(ctypes.POINTER(ctypes.c_double))) < 0
     assert "out of memory" in fake.error()
     assert fake.L.amrvac_gpu_step_dt(h, 1e-3) == 0, fake.error()
@@ -112,3 +112,37 @@ def test_registers_are_used_again(fake):
     assert fake.grid(small, [256, 256]) == 0
     assert [l for l in fake.log() if l.startswith("cudaMalloc") and int(l.split()[1]) > 1 << 20]
     assert fake.L.amrvac_gpu_destroy(small) == 0
+
+
+def test_kept_registers_make_room_for_other_memory(fake):
+    """A device that is full but for what the library keeps unused: staging
+    buffers, small per-block arrays and ensembles still fit."""
+    import ctypes
+    import numpy as np
+    from amrvac_b200 import _lib, make_cfg
+    dp = ctypes.POINTER(ctypes.c_double)
+
+    def keep():
+        h = fake.create(**HD2)
+        assert fake.grid(h, [1024, 1024]) == 0
+        assert fake.L.amrvac_gpu_destroy(h) == 0
+
+    h = fake.create(**HD2)
+    assert fake.grid(h, [64, 64]) == 0
+    keep()
+    fake.L.fake_capacity(fake.L.fake_used())
+    w = np.zeros((16, 4, 1, 20, 20))
+    assert fake.L.amrvac_gpu_upload(h, 0, 0, 16, w.ctypes.data_as(dp)) == 0, fake.error()
+    fake.L.fake_capacity(1 << 40)
+    keep()
+    fake.L.fake_capacity(fake.L.fake_used())
+    inst = (_lib.AmrvacEnsInstance * 1)()
+    inst[0].ndim, inst[0].time_max = 2, 1.0
+    for d in range(2):
+        inst[0].domain_nx[d], inst[0].xprobmax[d] = 64, 1.0
+    inst[0].flux_scheme, inst[0].limiter = _lib.FS["hllc"], _lib.LIMITER["vanleer"]
+    cfg = make_cfg(physics="hd", ndim=2, gamma=1.4, typeboundary=["cont"] * 4)
+    e = ctypes.c_void_p()
+    assert fake.L.amrvac_ens_create(ctypes.byref(cfg), 1, inst, ctypes.byref(e)) == 0, fake.error()
+    assert fake.L.amrvac_ens_destroy(e) == 0
+    assert fake.L.amrvac_gpu_destroy(h) == 0

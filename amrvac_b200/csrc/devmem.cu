@@ -1,6 +1,9 @@
 // Device memory of contexts and ensembles (devmem.cuh).
 #include "devmem.cuh"
 
+#include <cuda.h>
+
+#include <iterator>
 #include <list>
 #include <mutex>
 #include <unordered_map>
@@ -9,10 +12,48 @@ namespace amrvac {
 
 namespace {
 
+// The driver's identity of an allocation: its context, and an id that no other
+// allocation of the process ever has.  A kept register whose identity is not
+// what it was went with its context (cudaDeviceReset) and is only forgotten;
+// the address may be another's by now.
+struct Identity {
+  CUcontext ctx = nullptr;
+  unsigned long long id = 0;
+  bool operator==(const Identity &o) const { return ctx == o.ctx && id == o.id; }
+};
+template <class F>
+F driver_function(const char *name) {
+  void *f = nullptr;
+  cudaDriverEntryPointQueryResult q;
+  if (cudaGetDriverEntryPointByVersion(name, &f, 12000, cudaEnableDefault, &q) != cudaSuccess ||
+      q != cudaDriverEntryPointSuccess)
+    f = nullptr;
+  return reinterpret_cast<F>(f);
+}
+bool identity(void *p, Identity *out) {
+  using Get = CUresult (*)(void *, CUpointer_attribute, CUdeviceptr);
+  static const Get get = driver_function<Get>("cuPointerGetAttribute");
+  const CUdeviceptr d = reinterpret_cast<CUdeviceptr>(p);
+  return get && get(&out->ctx, CU_POINTER_ATTRIBUTE_CONTEXT, d) == CUDA_SUCCESS &&
+         get(&out->id, CU_POINTER_ATTRIBUTE_BUFFER_ID, d) == CUDA_SUCCESS;
+}
+CUcontext current_context() {
+  using Get = CUresult (*)(CUcontext *);
+  static const Get get = driver_function<Get>("cuCtxGetCurrent");
+  CUcontext c = nullptr;
+  cudaFree(nullptr);  // a thread's first call makes the device's context current
+  return get && get(&c) == CUDA_SUCCESS ? c : nullptr;
+}
+
 struct Reg {
   double *p;
   size_t bytes;
   int dev;
+  Identity is;
+  bool there() const {
+    Identity now;
+    return identity(p, &now) && now == is;
+  }
 };
 struct Registers {
   std::mutex m;
@@ -22,7 +63,7 @@ struct Registers {
 
   void drop(std::list<Reg>::iterator it) {
     kept_bytes -= it->bytes;
-    cudaFree(it->p);
+    if (it->there()) cudaFree(it->p);
     kept.erase(it);
   }
   // cudaMalloc; with the device short of memory the registers kept there go
@@ -58,20 +99,28 @@ cudaError_t register_alloc(double **p, size_t bytes) {
   if (e != cudaSuccess) return e;
   Registers &R = registers();
   std::lock_guard<std::mutex> lock(R.m);
-  auto best = R.kept.end();
-  for (auto it = R.kept.begin(); it != R.kept.end(); ++it)
-    if (it->dev == dev && it->bytes >= bytes && it->bytes <= bytes + bytes / 4 &&
-        (best == R.kept.end() || it->bytes < best->bytes))
-      best = it;
-  if (best != R.kept.end()) {
-    *p = best->p;
-    R.used[best->p] = *best;
-    R.kept_bytes -= best->bytes;
+  const CUcontext ctx = R.kept.empty() ? nullptr : current_context();
+  for (;;) {
+    auto best = R.kept.end();
+    for (auto it = R.kept.begin(); it != R.kept.end(); ++it)
+      if (it->is.ctx == ctx && it->bytes >= bytes && it->bytes <= bytes + bytes / 4 &&
+          (best == R.kept.end() || it->bytes < best->bytes))
+        best = it;
+    if (best == R.kept.end()) break;
+    const Reg r = *best;
+    R.kept_bytes -= r.bytes;
     R.kept.erase(best);
+    if (!r.there()) continue;
+    R.used[r.p] = r;
+    *p = r.p;
     return cudaSuccess;
   }
   e = R.alloc(reinterpret_cast<void **>(p), bytes, dev);
-  if (e == cudaSuccess) R.used[*p] = Reg{*p, bytes, dev};
+  if (e == cudaSuccess) {
+    Reg r{*p, bytes, dev, {}};
+    if (!identity(*p, &r.is)) r.is.ctx = nullptr;  // not told apart: not kept
+    R.used[*p] = r;
+  }
   return e;
 }
 
@@ -91,9 +140,15 @@ void register_free(double *p) {
   std::lock_guard<std::mutex> lock(R.m);
   const auto it = R.used.find(p);
   if (it == R.used.end()) return;
-  R.kept.push_front(it->second);
-  R.kept_bytes += it->second.bytes;
+  const Reg r = it->second;
   R.used.erase(it);
+  if (!r.is.ctx) {
+    cudaFree(p);
+    return;
+  }
+  if (!r.there()) return;
+  R.kept.push_front(r);
+  R.kept_bytes += r.bytes;
   // the oldest go first; one above the bound by itself takes no other with it
   if (R.kept.front().bytes > REGISTER_KEEP) R.drop(R.kept.begin());
   while (R.kept_bytes > REGISTER_KEEP) R.drop(std::prev(R.kept.end()));

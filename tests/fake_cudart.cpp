@@ -4,6 +4,7 @@
 // libcudart (tests/_fakecuda.py).
 //
 // Log lines: "<function> <arguments> = <error>".
+#include <cuda.h>
 #include <cuda_runtime_api.h>
 
 #include <algorithm>
@@ -23,6 +24,7 @@ struct Fail {
 struct Block {
   size_t bytes;
   int dev;
+  unsigned long long id;
 };
 std::mutex mtx;
 std::string logbuf;
@@ -30,7 +32,7 @@ std::map<std::string, Fail> fails;
 std::map<void *, Block> live;
 size_t capacity = (size_t)1 << 40, used = 0;
 int cur_dev = 0, nsm = 148;
-unsigned long long context_id = 1;
+unsigned long long allocations = 0;
 thread_local cudaError_t last = cudaSuccess;
 
 void logf(const char *fmt, ...) {
@@ -65,7 +67,7 @@ cudaError_t alloc(const char *fn, void **p, size_t n, bool device) {
   if (e == cudaSuccess && device && used + n > capacity) e = cudaErrorMemoryAllocation;
   if (e == cudaSuccess) {
     *p = std::calloc(n ? n : 1, 1);
-    live[*p] = Block{device ? n : 0, cur_dev};
+    live[*p] = Block{device ? n : 0, cur_dev, ++allocations};
     if (device) used += n;
   }
   char a[64];
@@ -116,10 +118,9 @@ size_t fake_used() { return used; }
 void fake_capacity(size_t n) { capacity = n; }
 void fake_sms(int n) { nsm = n; }
 int fake_last() { return (int)last; }
-// the memory of a device that was reset: everything on it is gone
+// what a device held goes with its context
 void fake_device_reset() {
   std::lock_guard<std::mutex> g(mtx);
-  ++context_id;
   live.clear();
   used = 0;
 }
@@ -233,6 +234,23 @@ static cudaError_t launch(dim3 g, dim3 b) {
 cudaError_t cudaLaunchKernel(const void *, dim3 g, dim3 b, void **, size_t, cudaStream_t) { return launch(g, b); }
 cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t *c, const void *, void **) {
   return launch(c->gridDim, c->blockDim);
+}
+
+// ---- driver functions, asked for by name
+static CUresult context(CUcontext *c) { *c = (CUcontext)(size_t)(1 + cur_dev); return CUDA_SUCCESS; }
+static CUresult attribute(void *out, CUpointer_attribute a, CUdeviceptr p) {
+  std::lock_guard<std::mutex> g(mtx);
+  const auto it = live.find((void *)p);
+  if (it == live.end()) return CUDA_ERROR_INVALID_VALUE;
+  if (a == CU_POINTER_ATTRIBUTE_CONTEXT) *(CUcontext *)out = (CUcontext)(size_t)(1 + it->second.dev);
+  else *(unsigned long long *)out = it->second.id;
+  return CUDA_SUCCESS;
+}
+cudaError_t cudaGetDriverEntryPointByVersion(const char *name, void **f, unsigned, unsigned long long,
+                                             cudaDriverEntryPointQueryResult *q) {
+  *f = !std::strcmp(name, "cuCtxGetCurrent") ? (void *)&context : (void *)&attribute;
+  *q = cudaDriverEntryPointSuccess;
+  return cudaSuccess;
 }
 
 }  // extern "C"

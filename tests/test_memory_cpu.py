@@ -146,3 +146,25 @@ def test_kept_registers_make_room_for_other_memory(fake):
     assert fake.L.amrvac_ens_create(ctypes.byref(cfg), 1, inst, ctypes.byref(e)) == 0, fake.error()
     assert fake.L.amrvac_ens_destroy(e) == 0
     assert fake.L.amrvac_gpu_destroy(h) == 0
+
+
+def test_registers_lost_with_their_device_context_are_not_used_again(fake):
+    """cudaDeviceReset between two contexts takes the kept registers away."""
+    h = fake.create(**HD2)
+    assert fake.grid(h, [512, 512]) == 0
+    assert fake.L.amrvac_gpu_destroy(h) == 0
+    fake.L.fake_device_reset()
+    h = fake.create(**HD2)
+    fake.clear()
+    assert fake.grid(h, [512, 512]) == 0
+    assert len([l for l in fake.log() if l.startswith("cudaMalloc") and int(l.split()[1]) > 1 << 20]) == 3
+    fake.clear()
+    fake.L.fake_device_reset()
+    fake.L.amrvac_gpu_destroy(h)
+    # nothing of that size is freed or kept: the addresses may be others' now
+    assert not [l for l in fake.log() if l.startswith("cudaFree ") and l.endswith("= 0") and int(l.split()[1]) > 1 << 20]
+    h = fake.create(**HD2)
+    fake.clear()
+    assert fake.grid(h, [512, 512]) == 0
+    assert len([l for l in fake.log() if l.startswith("cudaMalloc") and int(l.split()[1]) > 1 << 20]) == 3
+    assert fake.L.amrvac_gpu_destroy(h) == 0

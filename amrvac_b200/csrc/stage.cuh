@@ -1241,7 +1241,7 @@ __global__ void __launch_bounds__(StageOcc<TF, MHD, NDIM, LIM, BN, VAR>::THREADS
           const bool finite = !near && !special && isfinite(fsum);
           if (!finite) {
             retry = true;
-            Fr[0] = TF(NAN);
+            Fr[0] = special ? TF(INFINITY) : TF(NAN);  // infinite: near the blending band alone
           }
         }
         // FP64: the scaled flux fC = -qdt/dx * f as in the reference; mixed:
@@ -1258,15 +1258,14 @@ __global__ void __launch_bounds__(StageOcc<TF, MHD, NDIM, LIM, BN, VAR>::THREADS
         // fix-up pass: the thread's own faces whose flux is not finite or
         // whose limiter is near its blending band (an FP32 face of the mixed
         // form, or an FP64 face that met a special operand in the unguarded
-        // arithmetic), recomputed in FP64: in the fast arithmetic with the
-        // blend first, then with the guarded forms
+        // arithmetic), recomputed in FP64 with the guarded forms; a face near
+        // the blending band alone in the fast arithmetic first
         if (retry) {
           for (int f = t; f < nface; f += THREADS) {
             int FD, fl;
             face_dir(f, FD, fl);
-            bool finite = true;
-            for (int v = 0; v < NW; ++v) finite = finite && isfinite(flux_ref(f, FD, fl, v));
-            if (finite) continue;
+            const TF mark = flux_ref(f, FD, fl, 0);
+            if (isfinite(mark)) continue;
             const double sc = s_dxinv[FD];
             int fi, fj, base[H2];
             face_at(FD, fl, fi, fj, base);
@@ -1274,7 +1273,7 @@ __global__ void __launch_bounds__(StageOcc<TF, MHD, NDIM, LIM, BN, VAR>::THREADS
             FaceFlux64<NW> r;
             if constexpr (FP64) {
               bool done = false;
-              if constexpr (LIM == LIM_CADA3) {
+              if constexpr (LIM == LIM_CADA3) if (!isnan(mark)) {
                 r = face_retry_fp64<TF, MHD, NDIR, GLM, NDIM, SOLVER, LIM, BS, VS, true>(smem, FD, base[0], base[1],
                                                                                          base[2], base[3], rdd, cg, P);
                 done = true;

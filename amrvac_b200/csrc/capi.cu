@@ -81,6 +81,7 @@ struct amrvac_ctx {
   int *d_nbr = nullptr;
   double *d_dx = nullptr;
   double *d_scal = nullptr;              // see setdt_finalize_kernel
+  void *d_wait = nullptr;                // for wait_device
   unsigned long long *d_red = nullptr;   // getdt reduction accumulators, then the getdt kernel's CTA ticket
   double *h_red = nullptr, *h_red_dev = nullptr;  // getdt's result in mapped host memory (lazily), and its device address
   uint32_t *d_status = nullptr;
@@ -126,6 +127,7 @@ struct amrvac_ctx {
   size_t amr_gbuf_cap = 0, amr_pflux_cap = 0, amr_bxmin_cap = 0, amr_ints_cap = 0;
 };
 
+constexpr size_t WAIT_BYTES = 256;
 // The context's device current for a scope.
 struct DeviceScope {
   int prev = -1;
@@ -139,10 +141,17 @@ struct DeviceScope {
 };
 // Waits for everything on the context's device, before registers are given
 // back: work that the caller queued on other streams may still read them
-// through amrvac_gpu_register_ptr.
-static cudaError_t wait_device(const amrvac_ctx *c) {
+// through amrvac_gpu_register_ptr.  By cudaFree of an allocation held for it,
+// which synchronises across all streams and, unlike cudaDeviceSynchronize, is
+// valid while another thread captures a stream (amrvac_gpu_run's first call).
+// set_blocks makes the next one; where that failed it is made here.
+static cudaError_t wait_device(amrvac_ctx *c) {
   DeviceScope on(c->device);
-  return cudaDeviceSynchronize();
+  if (!c->d_wait)
+    if (cudaError_t e = device_alloc(&c->d_wait, WAIT_BYTES)) return e;
+  void *const p = c->d_wait;
+  c->d_wait = nullptr;
+  return cudaFree(p);
 }
 
 // Grow-only device buffer: reallocates (without keeping the contents) only
@@ -787,7 +796,8 @@ int amrvac_gpu_create(const amrvac_cfg *cfg, amrvac_ctx **out) {
       (e = device_alloc(&c->d_red, 3 * sizeof(unsigned long long))) != cudaSuccess ||
       (e = cudaMemset(c->d_red, 0, 3 * sizeof(unsigned long long))) != cudaSuccess ||
       (e = device_alloc(&c->d_status, sizeof(uint32_t))) != cudaSuccess ||
-      (e = cudaMemset(c->d_status, 0, sizeof(uint32_t))) != cudaSuccess) {
+      (e = cudaMemset(c->d_status, 0, sizeof(uint32_t))) != cudaSuccess ||
+      (e = device_alloc(&c->d_wait, WAIT_BYTES)) != cudaSuccess) {
     amrvac_gpu_destroy(c);
     return cuda_fail(e, "context allocation");
   }
@@ -953,6 +963,7 @@ static int set_blocks_impl(amrvac_ctx *c, int nblocks, const double *dx, const i
   CK(cudaMemsetAsync(c->d_block_status, 0, sizeof(uint32_t) * nblocks, c->stream));
   CK(cudaStreamSynchronize(c->stream));
   c->h_dx = dxb;
+  if (!c->d_wait) CK(device_alloc(&c->d_wait, WAIT_BYTES));
   for (int r = 0; r < 3; ++r) { register_free(c->d_adj[r]); c->d_adj[r] = nullptr; }
   c->adj_prepared = false;
   delete c->amr; c->amr = nullptr;

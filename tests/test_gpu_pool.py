@@ -86,3 +86,21 @@ def test_memory_is_back_when_close_returns():
     c.run(1)
     c.close()
     assert before - torch.cuda.mem_get_info()[0] <= KEEP + (128 << 20)
+
+
+def test_close_waits_for_other_streams():
+    """A stream of the caller's may still read a register (register_ptr)."""
+    import torch
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from amrvac_b200 import Context, make_cfg
+    c = Context(make_cfg(physics="hd", ndim=2, gamma=1.4, flux_scheme="hllc", limiter="vanleer"))
+    c.set_uniform_grid([64, 64], [0.0] * 2, [1.0] * 2)
+    for act in (lambda: c.set_uniform_grid([128, 128], [0.0] * 2, [1.0] * 2), c.close):
+        s, done = torch.cuda.Stream(), torch.cuda.Event()
+        with torch.cuda.stream(s):
+            torch.cuda._sleep(100_000_000)  # about 50 ms
+            done.record()
+        assert not done.query()
+        act()
+        assert done.query()

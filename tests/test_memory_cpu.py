@@ -13,50 +13,68 @@ def fake():
     return Fake()
 
 
+WAIT = "cudaFree 256 = 0"  # wait_device's allocation: cudaFree waits for all streams of the device
+
+
 def _first(log, *names):
-    return next((i for i, l in enumerate(log) if l.split()[0] in names), len(log))
+    """Index of the first call of one of the names on memory, the wait's apart."""
+    return next((i for i, l in enumerate(log) if l.split()[0] in names and l.split()[1] not in ("0", "256")), len(log))
 
 
 def test_registers_are_given_back_behind_a_wait_for_the_device(fake):
     """Work queued on other streams may still read a register (register_ptr):
     the whole device is waited for, also when it is full, before a register is
-    freed, and a failed wait is reported."""
+    freed or used again."""
     h = fake.create(**HD2)
     assert fake.grid(h, [64, 64]) == 0
-    fake.clear()
-    fake.fail("cudaMalloc")  # a full device: the growth below fails further on
-    fake.grid(h, [128, 128])
-    log = fake.log()
-    wait = log.index("cudaDeviceSynchronize 0 = 0")
-    assert wait < _first(log, "cudaFree", "cudaMalloc"), log
-    fake.L.fake_reset()
-    assert fake.grid(h, [128, 128]) == 0
+    for n in (128, 256, 512):
+        fake.clear()
+        fake.fail("cudaMalloc", times=2)  # a full device: the growth fails further on
+        assert fake.grid(h, [n, n]) < 0
+        log = fake.log()
+        assert log.index(WAIT) < _first(log, "cudaFree", "cudaMalloc"), log
+        fake.L.fake_reset()
+        assert fake.grid(h, [n, n]) == 0
     fake.clear()
     assert fake.L.amrvac_gpu_destroy(h) == 0
     log = fake.log()
-    assert log.index("cudaDeviceSynchronize 0 = 0") < _first(log, "cudaFree"), log
+    assert log.index(WAIT) < _first(log, "cudaFree"), log
 
 
 def test_a_failed_wait_is_reported(fake):
     h = fake.create(**HD2)
     assert fake.grid(h, [64, 64]) == 0
-    fake.clear()
-    fake.fail("cudaDeviceSynchronize", err=700)
-    assert fake.grid(h, [128, 128]) < 0
-    assert _first(fake.log(), "cudaFree") == len(fake.log())  # nothing was given back
-    fake.fail("cudaDeviceSynchronize", err=700)
+    reg = next(l.split()[1] for l in fake.log() if l.startswith("cudaMalloc") and int(l.split()[1]) > 100000)
+    for fn, err in (("cudaFree", 700), ("cudaMalloc", 2)):  # the wait itself, and nothing to wait with
+        fake.clear()
+        fake.fail(fn, times=9, err=err)
+        assert fake.grid(h, [128, 128]) < 0
+        assert f"cudaFree {reg} = 0" not in fake.log()  # nothing was given back
+        fake.L.fake_reset()
+    fake.fail("cudaFree", err=700)
     assert fake.L.amrvac_gpu_destroy(h) < 0
+    assert f"cudaFree {reg} = 0" not in fake.log()
+
+
+def test_the_wait_is_valid_while_another_thread_captures(fake):
+    """cudaDeviceSynchronize is an invalid call while any stream of the device
+    is being captured."""
+    h = fake.create(**HD2)
+    assert fake.grid(h, [64, 64]) == 0 and fake.grid(h, [512, 512]) == 0
+    assert fake.L.amrvac_gpu_destroy(h) == 0
+    assert not [l for l in fake.log() if l.startswith("cudaDeviceSynchronize")]
 
 
 def test_context_closed_from_another_device(fake):
-    """Its own device is waited for, and the caller's stays current."""
+    """What it allocates to wait is its own device's, and the caller's stays
+    current."""
     h = fake.create(**HD2)
     assert fake.grid(h, [64, 64]) == 0
     fake.L.cudaSetDevice(1)
     fake.clear()
     assert fake.L.amrvac_gpu_destroy(h) == 0
-    assert "cudaDeviceSynchronize 0 = 0" in fake.log()
-    assert [l for l in fake.log() if l.startswith("cudaSetDevice")][-1].split()[1] == "1"
+    devs = [l.split()[1] for l in fake.log() if l.startswith("cudaSetDevice")]
+    assert devs == ["0", "1"] and WAIT in fake.log()
 
 
 def test_a_failed_allocation_is_reported_once(fake):
@@ -93,8 +111,7 @@ def test_closed_context_keeps_no_more_than_the_bound(fake):
         assert fake.grid(h, [n, n]) == 0
         used = fake.L.fake_used()
         assert fake.L.amrvac_gpu_destroy(h) == 0
-        log = [l for l in fake.log() if l.startswith("cudaDeviceSynchronize") or l.startswith("cudaStreamSynchronize")]
-        assert log and fake.L.fake_used() <= min(KEEP, used)
+        assert fake.L.fake_used() <= min(KEEP, used)
 
 
 def test_registers_are_used_again(fake):

@@ -566,8 +566,8 @@ __device__ __forceinline__ void riemann_hlld_prim(const T *wLp, const T *wRp, T 
   // well.  As NaN it sent every face of a direction to the recomputation (64^3,
   // B along x, a step: cada3 FP64 612 -> 253 us, vanleer mixed 458 -> 202; with an
   // oblique field 251 -> 253 and 203 -> 202).
-  qR = qR != T(0.0) ? rcp_f<FAST>(qR) : qR;
-  qL = qL != T(0.0) ? rcp_f<FAST>(qL) : qL;
+  qR = rcp0_f<FAST>(qR);
+  qL = rcp0_f<FAST>(qL);
   const T kR = Bx * (sm - wRp[M]) * qR, kL = Bx * (sm - wLp[M]) * qL;
   const T pR = (suR * dvR - Bx2) * qR, pL = (suL * dvL - Bx2) * qL;
   const T sqR = sqrt_f<FAST>(rR), sqL = sqrt_f<FAST>(rL);

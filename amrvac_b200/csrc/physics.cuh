@@ -429,9 +429,9 @@ __device__ __forceinline__ uint32_t cbounds(const T *wLC, const T *wRC, const T 
   return st;
 }
 
-// Minimum and maximum of finite numbers.  In FP64 one compare and a select:
-// fmin / fmax also order NaN operands, which takes two or three instructions
-// more (a NaN here reaches the flux through the state that held it).
+// Minimum and maximum by one compare and a select in FP64 (fmin / fmax also
+// order NaN operands, which takes two or three instructions more).  With a NaN
+// operand the result is the second one: the callers place them accordingly.
 __device__ __forceinline__ double min_(double a, double b) { return a < b ? a : b; }
 __device__ __forceinline__ double max_(double a, double b) { return a > b ? a : b; }
 __device__ __forceinline__ float min_(float a, float b) { return fminf(a, b); }
@@ -451,8 +451,12 @@ __device__ __forceinline__ T slope_impl(int lim, T a, T b, T rdelinv) {
   constexpr T third = T(1.0) / T(3.0);
   switch (lim) {
     case LIM_MINMOD: {
+      // fmin / fmax ignore a NaN difference.  Where this runs once per face (FAST),
+      // one compare and a select does for the difference beyond the face (b of
+      // the left state, a of the right): the other one belongs to both states.
       const T t = fsign(T(1.0), a);
-      return t * max_(T(0.0), min_(fabs(a), t * b));
+      if constexpr (FAST) return t * max_(LEFT ? min_(t * b, fabs(a)) : min_(fabs(a), t * b), T(0.0));
+      else return t * fmax(T(0.0), fmin(fabs(a), t * b));
     }
     case LIM_VANLEER:
       return div_f<FAST>(T(2.0) * max_(b * a, T(0.0)), a + b + qsmall);
@@ -588,8 +592,9 @@ __device__ __forceinline__ void face_states(int lim_rt, T q0, T q1, T q2, T q3, 
     } else {
       const T Al = cada_asymptotic(tl), Ar = cada_asymptotic(tr);
       const T el = R2 ? sl : sl * rdel, er = R2 ? sr : sr * rdel, one = R2 ? rdel : T(1.0);
-      pl = el <= one ? Al : cada_limited(tl, Al, T(0.5), T(1.6));
-      pr = er <= one ? Ar : cada_limited(tr, Ar, T(0.5), T(1.6));
+      // (a NaN difference takes the asymptotic form, which is NaN with it)
+      pl = el > one ? cada_limited(tl, Al, T(0.5), T(1.6)) : Al;
+      pr = er > one ? cada_limited(tr, Ar, T(0.5), T(1.6)) : Ar;
       special = special || near_one(el, one) || near_one(er, one);
     }
     const T ldw = pl * d1, rdw = pr * d1;  // phi * a (left), phi * b (right): both d1

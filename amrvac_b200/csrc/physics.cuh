@@ -138,7 +138,7 @@ __device__ __forceinline__ double div_nr(double x, double y) { return x / y; }
 __device__ __forceinline__ double sqrt_nr(double x) {
   double y;
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  y = fmin(y, 0x1.0p511);
+  y = y > 0x1.0p511 ? 0x1.0p511 : y;  // (fmin would cap a NaN, too)
   double s = x * y, h = 0.5 * y;
   const double r = fma(-s, h, 0.5);
   s = fma(s, r, s);

@@ -1,4 +1,5 @@
-"""Operands that are not numbers: how far a NaN cell reaches in one stage.  The
+"""Operands that are not numbers: how far a NaN cell, and one of negative
+pressure, reaches in one stage.  The
 limiters that ignore a NaN difference (minmod) reach one cell, those that carry
 it two; the compiled-in limiters as the run-time ones and as the oracle.
 """
@@ -76,3 +77,15 @@ def test_nan_in_hlld(ndim, precision):
     bad = {lim: _bad("mhd", ndim, np.nan, limiter=lim, **kw) for lim in ("cada3", "vanleer", "minmod")}
     assert np.array_equal(bad["cada3"], bad["vanleer"])
     assert bad["minmod"].sum() < bad["vanleer"].sum()
+
+
+@pytest.mark.parametrize("physics,ndim,fs,limiter", [
+    ("hd", 2, "hllc", "vanleer"), ("hd", 2, "hll", "minmod"), ("hd", 2, "tvdlf", "minmod"), ("hd", 3, "hllc", "vanleer")])
+def test_negative_pressure_is_not_passed_over(oracle_lib, physics, ndim, fs, limiter):
+    """The signal speeds' root of a negative number is NaN, as in the oracle;
+    an infinity of either sign would choose one side's flux."""
+    _cuda()
+    kw = dict(flux_scheme=fs, limiter=limiter)
+    bad = _bad_oracle(oracle_lib, physics, ndim, -5.0, **kw)
+    assert bad.any()
+    assert np.array_equal(_bad(physics, ndim, -5.0, **kw), bad)

@@ -99,7 +99,8 @@ struct amrvac_ctx {
   int zchunk = 0;          // 0: persistent plane ranges; 16/8/4: one z-chunk per CTA
   int sweep = -1;          // dimensional splitting: the current sweep of the step (-1: unsplit)
   bool fixed_dir = false;  // sweep is a direction (amrvac_gpu_advect1_dim), not a sweep index
-  int wave_ctas = 1;       // resident stage CTAs on the device (one wave)
+  int nsm = 148;           // SMs of the device
+  int wave_hancock = 1;    // resident CTAs of the Hancock predictor on the device (one wave)
   int var = 0;             // stage-kernel variant (KernelSet::stage_v; chosen by the autotuner)
   // small_values_method 'average': whole-block recomputation of the flagged
   // blocks (smallavg.cu), its scratch, and a pre-stage copy of a register
@@ -223,6 +224,7 @@ StageArgs stage_args(amrvac_ctx *c, int reg_ct, int reg_new, int reg_base, doubl
   A.nbr = c->d_nbr;
   A.dxb = c->d_dx;
   A.nblocks = c->nblocks;
+  A.nsm = c->nsm;
   A.zchunk = c->zchunk;
   for (int s = 0; s < 6; ++s) {
     A.bc_kind[s] = c->bc.kind[s];
@@ -269,7 +271,7 @@ int launch_stage(amrvac_ctx *c, int reg_ct, int reg_new, int reg_base, double a,
   const long planes = (long)c->nblocks * ntile * (c->cfg.ndim == 3 ? bn : 1);
   int nctas;
   if (c->zchunk > 0) nctas = c->nblocks * ntile * (c->cfg.ndim == 3 ? bn / c->zchunk : 1);
-  else nctas = (int)std::min<long>(planes, hancock ? c->wave_ctas : c->wave_v[c->var]);
+  else nctas = (int)std::min<long>(planes, hancock ? c->wave_hancock : c->wave_v[c->var]);
   const bool restore = !hancock && c->P.fix_small_values && c->P.small_values_method == 0;
   if (restore || c->sv_on) {
     CK(cudaMemsetAsync(c->d_block_status, 0, sizeof(uint32_t) * c->nblocks, c->stream));
@@ -332,6 +334,7 @@ static bool valid_zchunk(int bn, int zchunk) { return zchunk == 0 || (zchunk >= 
 int launch_getdt(amrvac_ctx *c, int reg, int tail = 0) {
   GetdtArgs G;
   G.scal = tail ? c->d_scal : nullptr;
+  G.nsm = c->nsm;
   G.ticket = reinterpret_cast<unsigned *>(c->d_red + 2);
   G.advance = tail == 2;
   G.host = tail == 3 ? c->h_red_dev : nullptr;
@@ -774,11 +777,10 @@ int amrvac_gpu_create(const amrvac_cfg *cfg, amrvac_ctx **out) {
   }
   c->zchunk = valid_zchunk(bn, k.zchunk) ? k.zchunk : 0;
   {
-    int nsm = 148;
     cudaGetDevice(&c->device);
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device);
-    c->wave_ctas = nsm * c->ks.ctas_per_sm();
-    for (int v = 0; v < c->ks.nvar; ++v) c->wave_v[v] = nsm * c->ks.ctas_v[v]();
+    cudaDeviceGetAttribute(&c->nsm, cudaDevAttrMultiProcessorCount, c->device);
+    c->wave_hancock = c->nsm * c->ks.hancock_ctas_per_sm();
+    for (int v = 0; v < c->ks.nvar; ++v) c->wave_v[v] = c->nsm * c->ks.ctas_v[v]();
   }
   c->per_block = 1;
   for (int d = 0; d < k.ndim; ++d) c->per_block *= bn;
@@ -807,11 +809,8 @@ int amrvac_gpu_create(const amrvac_cfg *cfg, amrvac_ctx **out) {
     size_t gc = 1;
     for (int d = 0; d < k.ndim; ++d) gc *= (size_t)(bn + 4);
     c->sv_per_cta = 5 * (size_t)nw * gc + (2 * gc + 7) / 8;
-    int nsm = 148, dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
     const size_t fit = ((size_t)256 << 20) / (sizeof(double) * c->sv_per_cta);
-    c->sv_ctas = (int)std::max<size_t>(1, std::min<size_t>(fit, (size_t)nsm));
+    c->sv_ctas = (int)std::max<size_t>(1, std::min<size_t>(fit, (size_t)c->nsm));
     if ((e = device_alloc(&c->sv_scratch, sizeof(double) * c->sv_per_cta * c->sv_ctas)) != cudaSuccess) {
       amrvac_gpu_destroy(c);
       return cuda_fail(e, "small-value scratch allocation");

@@ -66,6 +66,7 @@ struct GetdtArgs {
   // (mapped), sets scal's cmax_global and clears the words for the next call
   double *host;
   bool dependent;  // launch: the predecessor on the stream allows a dependent launch
+  int nsm;         // launch: SMs of the device
 };
 
 __device__ __forceinline__ double warp_max(double v) {
@@ -371,7 +372,7 @@ __global__ void __launch_bounds__(256) linde3d_kernel(const StageArgs A) {
 // ---------------------------------------------------------------- dispatch
 struct KernelSet {
   cudaError_t (*prepare)() = nullptr;
-  int (*ctas_per_sm)() = nullptr;
+  int (*hancock_ctas_per_sm)() = nullptr;
   cudaError_t (*stage)(const StageArgs &, int nctas, cudaStream_t) = nullptr;
   // MUSCL-Hancock predictor of twostep Predictor_Corrector (tvdlf sets only)
   cudaError_t (*hancock)(const StageArgs &, int nctas, cudaStream_t) = nullptr;
@@ -434,21 +435,31 @@ struct Launch {
   using V = Vars<MHD, NDIR, GLM>;
   static constexpr int THREADS = StageOcc<TF, MHD, NDIM, LIM, BN>::THREADS;
   static constexpr size_t SMEM = Tile<TF, V::NW, NDIM, HaloW<LIM>::value, tile_edge(BN)>::BYTES;
-  // typepred1 = fs_hancock for tvdlf and tvdmu (src/io/mod_input_output.t:787-797)
   // The 2-D hydrodynamics tile is small (30 KB) and its kernel waits for its
   // block's loads and barriers: four CTAs per SM (64 registers) instead of two
-  // hide them, 2048^2 HLLC + vanleer FP64 0.37 -> 0.31 ms per stage.  A grid
-  // that the two-CTA kernel holds in one wave has no second CTA to hide
-  // behind, and runs the kernel without spills (64^2: 28 against 26 us a step).
+  // hide them, 2048^2 HLLC + vanleer FP64 0.37 -> 0.31 ms per stage.  So they do
+  // for the other solvers and limiters (1024^2, us a step: HLL + cada3 292 -> 252,
+  // Roe 293 -> 265, TVDLF 223 -> 193, HLL + WENO3 560 -> 424, HLL + Venkatakrishnan
+  // 639 -> 521).  A grid that the two-CTA kernel holds in one wave has no second
+  // CTA to hide behind, and runs the kernel that spills least (64^2: 28 -> 26 us a
+  // step; 272^2 in blocks of 8, 1156 tiles at eight CTAs per SM: 53 -> 35).
   static constexpr bool HAS_DENSE = !MHD && NDIM == 2 && sizeof(TF) == 8 && HaloW<LIM>::value == 2;
   static constexpr int VMAIN = HAS_DENSE ? VAR_DENSE : 0;
-  static constexpr int SMALL_TILES = 2 * 148;
   static constexpr int NTILE = (BN / tile_edge(BN)) * (BN / tile_edge(BN));
   // Up to one tile per SM there is no other work to hide a tile's latency, and
   // a block edge of 16 takes a thread per face (576 threads: one round of
   // faces instead of three; 64^2 HLLC 24.9 -> 21.7 us a step).  At two tiles per
   // SM half of them (288) measured no gain over 256 (256^2 31.8 -> 32.2).
   static constexpr bool HAS_WIDE = HAS_DENSE && BN == 16;
+  // the build that runs nblocks blocks on nsm SMs
+  static int build(int nblocks, int nsm) {
+    if (HAS_WIDE && nblocks <= nsm) return VAR_WIDE;
+    return HAS_DENSE && nblocks * NTILE > StageOcc<TF, MHD, NDIM, LIM, BN>::MINB * nsm ? VAR_DENSE : 0;
+  }
+  // typepred1 = fs_hancock for tvdlf and tvdmu (src/io/mod_input_output.t:787-797),
+  // in a wave of its own: it is less dense than the stage's and, at small block
+  // edges, has more CTAs per SM than two (512^2 in blocks of 8, tvdlf: 72 us a
+  // step; with 296 CTAs, two per SM, 131)
   static constexpr bool HAS_HANCOCK = (SOLVER == SOLVER_TVDLF || SOLVER == SOLVER_TVDMU) && sizeof(TF) == 8;
   static cudaError_t prepare() {
     cudaError_t e = cudaFuncSetAttribute(fv_stage_kernel<TF, MHD, NDIR, GLM, NDIM, SOLVER, LIM, BS, BN>,
@@ -471,17 +482,17 @@ struct Launch {
     return e;
   }
   static cudaError_t stage(const StageArgs &A, int nctas, cudaStream_t s) {
+    [[maybe_unused]] const int var = build(A.nblocks, A.nsm);
+    if constexpr (HAS_WIDE) {
+      if (var == VAR_WIDE)
+        return launch_dependent<StageArgs>(
+            &fv_stage_kernel<TF, MHD, NDIR, GLM, NDIM, SOLVER, LIM, BS, BN, VAR_WIDE>, nctas,
+            StageOcc<TF, MHD, NDIM, LIM, BN, VAR_WIDE>::THREADS, SMEM, s, A.dependent, A);
+    }
     if constexpr (HAS_DENSE) {
-      if constexpr (HAS_WIDE) {
-        if (A.nblocks <= SMALL_TILES / 2)
-          return launch_dependent<StageArgs>(
-              &fv_stage_kernel<TF, MHD, NDIR, GLM, NDIM, SOLVER, LIM, BS, BN, VAR_WIDE>, nctas,
-              StageOcc<TF, MHD, NDIM, LIM, BN, VAR_WIDE>::THREADS, SMEM, s, A.dependent, A);
-      }
-      if (A.nblocks * NTILE > SMALL_TILES) {
+      if (var == VAR_DENSE)
         return launch_dependent<StageArgs>(&fv_stage_kernel<TF, MHD, NDIR, GLM, NDIM, SOLVER, LIM, BS, BN, VAR_DENSE>,
                                            nctas, THREADS, SMEM, s, A.dependent, A);
-      }
     }
     return launch_dependent<StageArgs>(&fv_stage_kernel<TF, MHD, NDIR, GLM, NDIM, SOLVER, LIM, BS, BN>, nctas, THREADS,
                                        SMEM, s, A.dependent, A);
@@ -500,26 +511,30 @@ struct Launch {
   }
   static cudaError_t hancock(const StageArgs &A, int nctas, cudaStream_t s) {
     if constexpr (HAS_HANCOCK) {
-      // nctas is one wave of the main kernel, which is denser than this one
-      if (HAS_DENSE && A.zchunk == 0 && nctas > SMALL_TILES) nctas = SMALL_TILES;
       return launch_dependent<StageArgs>(&fv_stage_kernel<TF, MHD, NDIR, GLM, NDIM, SOLVER_HANCOCK, LIM, BS, BN>, nctas,
                                          THREADS, SMEM, s, A.dependent, A);
     } else {
       return cudaErrorNotSupported;
     }
   }
-  static int ctas_per_sm() {
+  template <int SOL, int VAR>
+  static int resident() {
     int n = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-            &n, fv_stage_kernel<TF, MHD, NDIR, GLM, NDIM, SOLVER, LIM, BS, BN, VMAIN>, THREADS, SMEM) != cudaSuccess)
+            &n, fv_stage_kernel<TF, MHD, NDIR, GLM, NDIM, SOL, LIM, BS, BN, VAR>, THREADS, SMEM) != cudaSuccess)
       return 1;
     return n > 0 ? n : 1;
+  }
+  static int ctas_per_sm() { return resident<SOLVER, VMAIN>(); }
+  static int hancock_ctas_per_sm() {
+    if constexpr (HAS_HANCOCK) return resident<SOLVER_HANCOCK, 0>();
+    else return 1;
   }
   static cudaError_t getdt(const GetdtArgs &A, cudaStream_t s) {
     int ncell = 1;
     for (int d = 0; d < NDIM; ++d) ncell *= A.bn;
     const long items = (long)A.nblocks * (A.type_courant == 1 ? (ncell + GETDT_CHUNK - 1) / GETDT_CHUNK : 1);
-    const int nctas = (int)(items < 4 * 148 ? items : 4 * 148);
+    const int nctas = (int)(items < 4 * A.nsm ? items : 4 * A.nsm);
     return launch_dependent<GetdtArgs>(&getdt_kernel<MHD, NDIR, GLM, NDIM>, nctas, 256, 0, s, A.dependent, A);
   }
   template <int D>
@@ -558,7 +573,7 @@ struct Launch {
   static KernelSet set() {
     KernelSet k;
     k.prepare = &prepare;
-    k.ctas_per_sm = &ctas_per_sm;
+    k.hancock_ctas_per_sm = &hancock_ctas_per_sm;
     k.stage = &stage;
     if (HAS_HANCOCK) k.hancock = &hancock;
     if (MHD && NDIM == 3 && !GLM) k.linde3d = &linde3d;

@@ -138,6 +138,7 @@ struct StageArgs {
   int split_xy;             // 1: typedimsplit 'xy' (same order every step)
   int bn;                   // block edge, for the kernels that take it at run time
   int dependent;            // launch: the predecessor on the stream allows a dependent launch
+  int nsm;                  // launch: SMs of the device
 };
 
 // Direction of a dimensionally split sweep (src/mod_advance.t:23-45):

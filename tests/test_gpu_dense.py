@@ -1,7 +1,8 @@
 """The builds of the FP64 2-D hydrodynamics stage kernel (a thread per face up
 to 148 tiles at block edge 16, two CTAs per SM up to 296 tiles, four above) on
-both sides of those lines, at block edges 16 and 32 (four tiles per block),
-against the oracle: one full step, cell by cell
+both sides of those lines, at block edges 16 and 32 (four tiles per block), and
+at 8, 10 and 12 (lines at 1184, 592 and 444 tiles: eight, four and three CTAs
+per SM), against the oracle: one full step, cell by cell
 (tests/_parity.py; bar 1e-12), with the persistent distribution and with one
 tile per CTA.
 """
@@ -16,7 +17,8 @@ pytestmark = pytest.mark.gpu
 RTOL = 1e-12
 
 
-@pytest.mark.parametrize("bn,nb", [(16, (1, 1)), (16, (37, 4)), (16, (1, 149)), (16, (17, 17)), (16, (37, 8)), (16, (11, 27)), (32, (2, 37)), (32, (5, 15))])
+@pytest.mark.parametrize("bn,nb", [(16, (1, 1)), (16, (37, 4)), (16, (1, 149)), (16, (17, 17)), (16, (37, 8)), (16, (11, 27)), (32, (2, 37)), (32, (5, 15)),
+                                   (8, (34, 34)), (8, (35, 34)), (10, (37, 16)), (10, (37, 17)), (12, (37, 12)), (12, (37, 13))])
 @pytest.mark.parametrize("kw", [dict(flux_scheme="hllc", limiter="vanleer"), dict(flux_scheme="hll", limiter="minmod"),
                                 dict(flux_scheme="tvdlf", limiter="koren", time_stepper="twostep")])
 def test_every_build_matches_oracle(oracle_lib, bn, nb, kw):

@@ -83,7 +83,7 @@ struct amrvac_ctx {
   double *d_scal = nullptr;              // see setdt_finalize_kernel
   void *d_wait = nullptr;                // for wait_device
   unsigned long long *d_red = nullptr;   // getdt reduction accumulators, then the getdt kernel's CTA ticket
-  double *h_red = nullptr, *h_red_dev = nullptr;  // getdt's result in mapped host memory (lazily), and its device address
+  double *h_red = nullptr, *h_red_dev = nullptr;  // getdt's result in mapped host memory (not 'average'), and its device address
   uint32_t *d_status = nullptr;
   uint32_t *d_block_status = nullptr;
   double *d_stage = nullptr;             // upload/download staging
@@ -799,7 +799,8 @@ int amrvac_gpu_create(const amrvac_cfg *cfg, amrvac_ctx **out) {
       (e = cudaMemset(c->d_red, 0, 3 * sizeof(unsigned long long))) != cudaSuccess ||
       (e = device_alloc(&c->d_status, sizeof(uint32_t))) != cudaSuccess ||
       (e = cudaMemset(c->d_status, 0, sizeof(uint32_t))) != cudaSuccess ||
-      (e = device_alloc(&c->d_wait, WAIT_BYTES)) != cudaSuccess) {
+      (e = device_alloc(&c->d_wait, WAIT_BYTES)) != cudaSuccess ||
+      (!c->sv_on && (e = host_words_alloc(&c->h_red, &c->h_red_dev)) != cudaSuccess)) {
     amrvac_gpu_destroy(c);
     return cuda_fail(e, "context allocation");
   }
@@ -835,7 +836,7 @@ int amrvac_gpu_destroy(amrvac_ctx *c) {
   cudaFree(c->d_nbr);
   cudaFree(c->d_dx);
   cudaFree(c->d_red);
-  cudaFreeHost(c->h_red);
+  if (waited == cudaSuccess) host_words_free(c->h_red);
   cudaFree(c->d_status);
   cudaFree(c->d_block_status);
   cudaFree(c->d_amr_int);
@@ -1496,10 +1497,6 @@ int amrvac_gpu_getdt(amrvac_ctx *c, int reg, double *dt, double *cmax_global) {
     // host and cmax_global to the device scalar (three copies and a second
     // wait around it: a 64^2 host-driven step 82.7 us, with this and advect1's
     // scalar 68.7)
-    if (!c->h_red) {
-      CK(cudaHostAlloc(&c->h_red, 2 * sizeof(double), cudaHostAllocMapped));
-      CK(cudaHostGetDevicePointer(&c->h_red_dev, c->h_red, 0));
-    }
     if (int r = launch_getdt(c, reg, 3)) return r;
     CK(cudaStreamSynchronize(c->stream));
     x = c->h_red[0];

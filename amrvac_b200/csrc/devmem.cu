@@ -7,6 +7,7 @@
 #include <list>
 #include <mutex>
 #include <unordered_map>
+#include <vector>
 
 namespace amrvac {
 
@@ -152,6 +153,64 @@ void register_free(double *p) {
   // the oldest go first; one above the bound by itself takes no other with it
   if (R.kept.front().bytes > REGISTER_KEEP) R.drop(R.kept.begin());
   while (R.kept_bytes > REGISTER_KEEP) R.drop(std::prev(R.kept.end()));
+}
+
+namespace {
+
+struct HostPage {
+  static constexpr int SLOTS = 256;
+  double *p;
+  Identity is;  // none: not told apart
+  std::vector<int> free;
+  bool there() const {
+    Identity now;
+    return !is.ctx || (identity(p, &now) && now == is);
+  }
+};
+struct HostPages {
+  std::mutex m;
+  std::list<HostPage> pages;
+};
+HostPages &host_pages() {
+  static HostPages *h = new HostPages;
+  return *h;
+}
+
+}  // namespace
+
+cudaError_t host_words_alloc(double **host, double **dev) {
+  HostPages &H = host_pages();
+  std::lock_guard<std::mutex> lock(H.m);
+  for (auto it = H.pages.begin(); it != H.pages.end();) {
+    auto cur = it++;
+    if (!cur->there()) H.pages.erase(cur);  // went with its context
+  }
+  auto page = H.pages.begin();
+  while (page != H.pages.end() && page->free.empty()) ++page;
+  if (page == H.pages.end()) {
+    HostPage n;
+    const cudaError_t e = cudaHostAlloc(reinterpret_cast<void **>(&n.p), sizeof(double) * 2 * HostPage::SLOTS,
+                                        cudaHostAllocMapped | cudaHostAllocPortable);
+    if (e != cudaSuccess) return e;
+    if (!identity(n.p, &n.is)) n.is = Identity();
+    for (int q = HostPage::SLOTS; q-- > 0;) n.free.push_back(q);
+    H.pages.push_front(n);
+    page = H.pages.begin();
+  }
+  double *const p = page->p + 2 * page->free.back();
+  const cudaError_t e = cudaHostGetDevicePointer(reinterpret_cast<void **>(dev), p, 0);
+  if (e != cudaSuccess) return e;
+  page->free.pop_back();
+  *host = p;
+  return cudaSuccess;
+}
+
+void host_words_free(double *host) {
+  if (!host) return;
+  HostPages &H = host_pages();
+  std::lock_guard<std::mutex> lock(H.m);
+  for (HostPage &g : H.pages)
+    if (host >= g.p && host < g.p + 2 * HostPage::SLOTS) g.free.push_back((int)(host - g.p) / 2);
 }
 
 }  // namespace amrvac

@@ -28,4 +28,10 @@ cudaError_t device_alloc(T **p, size_t bytes) {
   return device_alloc(reinterpret_cast<void **>(p), bytes);
 }
 
+// Two words of page-locked host memory that kernels write, and their address
+// on the current device.  From pages made once per process: a page of a
+// context's own cost 2.2 ms to make and 0.3 ms to free.
+cudaError_t host_words_alloc(double **host, double **dev);
+void host_words_free(double *host);
+
 }  // namespace amrvac

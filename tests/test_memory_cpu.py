@@ -185,3 +185,42 @@ def test_registers_lost_with_their_device_context_are_not_used_again(fake):
     assert fake.grid(h, [512, 512]) == 0
     assert len([l for l in fake.log() if l.startswith("cudaMalloc") and int(l.split()[1]) > 1 << 20]) == 3
     assert fake.L.amrvac_gpu_destroy(h) == 0
+
+
+def _getdt(fake, h):
+    import ctypes
+    dt, cm = ctypes.c_double(), ctypes.c_double()
+    return fake.L.amrvac_gpu_getdt(h, 0, ctypes.byref(dt), ctypes.byref(cm))
+
+
+@pytest.mark.parametrize("fn", ["cudaHostAlloc", "cudaHostGetDevicePointer"])
+def test_getdt_never_runs_without_its_result_words(fake, fn):
+    """They are made with the context, which is refused where they cannot be;
+    getdt itself allocates nothing."""
+    import ctypes
+    from amrvac_b200 import make_cfg
+    fake.L.fake_device_reset()  # no page is there yet
+    h = ctypes.c_void_p()
+    fake.fail(fn)
+    cfg = make_cfg(**HD2)
+    assert fake.L.amrvac_gpu_create(ctypes.byref(cfg), ctypes.byref(h)) < 0
+    fake.L.fake_reset()
+    h = fake.create(**HD2)
+    assert fake.grid(h, [64, 64]) == 0
+    fake.clear()
+    fake.fail(fn)
+    assert _getdt(fake, h) >= 0 and _getdt(fake, h) >= 0
+    assert {l.split()[0] for l in fake.log()} == {"launch", "cudaStreamSynchronize"}
+    assert fake.L.amrvac_gpu_destroy(h) == 0
+
+
+def test_result_words_share_pages(fake):
+    """One page for 256 contexts, kept; each context has words of its own."""
+    fake.L.fake_device_reset()
+    hs = [fake.create(**HD2) for _ in range(257)]
+    for h in hs:
+        assert fake.L.amrvac_gpu_destroy(h) == 0
+    h = fake.create(**HD2)
+    assert len([l for l in fake.log() if l.startswith("cudaHostAlloc")]) == 2
+    assert not [l for l in fake.log() if l.startswith("cudaFreeHost")]
+    assert fake.L.amrvac_gpu_destroy(h) == 0

@@ -925,6 +925,7 @@ static int set_blocks_impl(amrvac_ctx *c, int nblocks, const double *dx, const i
     // regrid into a new, larger buffer: the other registers follow its size
     const size_t cap = (size_t)nblocks + nblocks / 4 + 1;
     CK(wait_device(c));
+    c->nblocks = 0;  // a failure from here on leaves no blocks set
     for (int r = 0; r < 4; ++r) { register_free(c->pool[r]); c->pool[r] = nullptr; }
     c->pool_cap = 0;
     c->pool[0] = adopt_reg0;
@@ -934,6 +935,7 @@ static int set_blocks_impl(amrvac_ctx *c, int nblocks, const double *dx, const i
   } else {
     if ((size_t)nblocks > c->pool_cap || !c->pool[0]) {
       if (c->pool[0]) CK(wait_device(c));
+      c->nblocks = 0;
       for (int r = 0; r < 4; ++r) { register_free(c->pool[r]); c->pool[r] = nullptr; }
       c->pool_cap = 0;
       const size_t cap = (size_t)nblocks + nblocks / 4 + 1;
@@ -945,9 +947,10 @@ static int set_blocks_impl(amrvac_ctx *c, int nblocks, const double *dx, const i
         CK(register_alloc(&c->sv_snap, sizeof(double) * c->per_block * c->nw * cap));
       }
     }
+    c->nblocks = 0;
     for (int r = 0; r < c->nreg; ++r) CK(cudaMemsetAsync(c->pool[r], 0, bytes, c->stream));
   }
-  c->nblocks = nblocks;
+  c->nblocks = 0;
   if ((size_t)nblocks > c->nbr_cap || !c->d_nbr) {
     cudaFree(c->d_nbr); cudaFree(c->d_dx); cudaFree(c->d_block_status);
     c->d_nbr = nullptr; c->d_dx = nullptr; c->d_block_status = nullptr;
@@ -967,6 +970,7 @@ static int set_blocks_impl(amrvac_ctx *c, int nblocks, const double *dx, const i
   for (int r = 0; r < 3; ++r) { register_free(c->d_adj[r]); c->d_adj[r] = nullptr; }
   c->adj_prepared = false;
   delete c->amr; c->amr = nullptr;
+  c->nblocks = nblocks;
   return 0;
 }
 
@@ -1277,7 +1281,8 @@ static int amr_grid_impl(amrvac_ctx *c, int nleaf, const int *leaf, const int *n
     if (newreg && c->pool[0] != newreg && c->pool[1] != newreg) register_free(newreg);
     return r;
   }
-  // device copies
+  // device copies; a failure among them leaves no blocks set
+  c->nblocks = 0;
   AmrDev *A = new AmrDev();
   c->amr = A;
   A->h_leaf.assign(4 * (size_t)nb, 0);
@@ -1346,6 +1351,7 @@ static int amr_grid_impl(amrvac_ctx *c, int nleaf, const int *leaf, const int *n
   A->F.sweep = -1;
   A->F.scal = c->d_scal;
   CK(cudaStreamSynchronize(c->stream));
+  c->nblocks = nb;
   return 0;
 }
 

@@ -224,3 +224,19 @@ def test_result_words_share_pages(fake):
     assert len([l for l in fake.log() if l.startswith("cudaHostAlloc")]) == 2
     assert not [l for l in fake.log() if l.startswith("cudaFreeHost")]
     assert fake.L.amrvac_gpu_destroy(h) == 0
+
+
+@pytest.mark.parametrize("after", range(7))
+def test_a_failed_growth_leaves_no_blocks(fake, after):
+    """Whichever allocation fails, a step is refused instead of launched on
+    registers or tables that are not there."""
+    fake.L.fake_device_reset()  # no kept registers
+    h = fake.create(**HD2)
+    assert fake.grid(h, [64, 64]) == 0
+    fake.fail("cudaMalloc", after=after, times=99)
+    assert fake.grid(h, [128, 128]) < 0
+    fake.L.fake_reset()
+    assert fake.L.amrvac_gpu_step(h) < 0 and "no blocks set" in fake.error()
+    assert not [l for l in fake.log() if l.startswith("launch")]
+    assert fake.grid(h, [128, 128]) == 0 and fake.L.amrvac_gpu_step(h) == 0
+    assert fake.L.amrvac_gpu_destroy(h) == 0

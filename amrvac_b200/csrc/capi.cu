@@ -1702,8 +1702,10 @@ int amrvac_gpu_stage_variant(amrvac_ctx *c, int *var, int *nvar, int *threads, i
   if (int r = check_ctx(c, false)) return r;
   if (var) *var = c->var;
   if (nvar) *nvar = c->ks.nvar;
-  if (threads) *threads = c->ks.var_threads[c->var];
-  if (ctas_per_sm) *ctas_per_sm = c->ks.var_minb[c->var];
+  int t = c->ks.var_threads[c->var], m = c->ks.var_minb[c->var];
+  if (c->var == 0) c->ks.shape(c->nblocks, c->nsm, &t, &m);
+  if (threads) *threads = t;
+  if (ctas_per_sm) *ctas_per_sm = m;
   if (async) *async = c->ks.var_async[c->var];
   return 0;
 }

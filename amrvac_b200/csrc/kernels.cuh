@@ -395,6 +395,8 @@ struct KernelSet {
   int (*ctas_v[MAXVAR])() = {};
   cudaError_t (*prepare_v[MAXVAR])() = {};
   int var_threads[MAXVAR] = {}, var_minb[MAXVAR] = {}, var_async[MAXVAR] = {};
+  // threads per CTA and CTAs per SM of variant 0 on a grid (Launch::build)
+  void (*shape)(int nblocks, int nsm, int *threads, int *minb) = nullptr;
 };
 
 // One stage-kernel variant of a scheme (see stage_variant).
@@ -455,6 +457,13 @@ struct Launch {
   static int build(int nblocks, int nsm) {
     if (HAS_WIDE && nblocks <= nsm) return VAR_WIDE;
     return HAS_DENSE && nblocks * NTILE > StageOcc<TF, MHD, NDIM, LIM, BN>::MINB * nsm ? VAR_DENSE : 0;
+  }
+  static void shape(int nblocks, int nsm, int *threads, int *minb) {
+    const int var = build(nblocks, nsm);
+    *threads = var == VAR_WIDE ? StageOcc<TF, MHD, NDIM, LIM, BN, VAR_WIDE>::THREADS : THREADS;
+    *minb = var == VAR_WIDE    ? StageOcc<TF, MHD, NDIM, LIM, BN, VAR_WIDE>::MINB
+            : var == VAR_DENSE ? StageOcc<TF, MHD, NDIM, LIM, BN, VAR_DENSE>::MINB
+                               : StageOcc<TF, MHD, NDIM, LIM, BN>::MINB;
   }
   // typepred1 = fs_hancock for tvdlf and tvdmu (src/io/mod_input_output.t:787-797),
   // in a wave of its own: it is less dense than the stage's and, at small block
@@ -587,6 +596,7 @@ struct Launch {
     StageVar<MHD, NDIR, GLM, NDIM, SOLVER, LIM, BS, TF, BN, 0>::add(k, 0);
     k.stage_v[0] = &stage;
     k.ctas_v[0] = &ctas_per_sm;
+    k.shape = &shape;
     return k;
   }
 };

@@ -291,7 +291,9 @@ int amrvac_gpu_set_zchunk(amrvac_ctx *ctx, int zchunk);
  * HLLD + cada3 + Einfeldt + GLM scheme at block_nx 16 has three more —
  * threads per CTA, the CTAs per SM the registers are capped for, and (FP64)
  * asynchronous bulk-copy staging of the next conserved plane.  Select one
- * (e.g. from a cache), or read the current one with its parameters. */
+ * (e.g. from a cache), or read the current one with its parameters (for
+ * variant 0, which has several builds in 2-D hydrodynamics, those of the build
+ * that runs the current grid). */
 int amrvac_gpu_set_stage_variant(amrvac_ctx *ctx, int var);
 int amrvac_gpu_stage_variant(amrvac_ctx *ctx, int *var, int *nvar, int *threads, int *ctas_per_sm, int *async);
 /* Read back the last step's dt, cmax_global and global_time (synchronises). */

@@ -40,3 +40,18 @@ def test_builds_follow_the_devices_size(fake, sms):
     fake.L.fake_sms(sms)
     assert {t for _, t in _launches(fake, (16 * sms, 16), **kw)} == {576}
     assert {t for _, t in _launches(fake, (16 * sms + 16, 16), **kw)} == {256}
+
+
+@pytest.mark.parametrize("tiles", [1, 148, 149, 296, 297])
+def test_stage_variant_reports_what_runs(fake, tiles):
+    import ctypes
+    h = fake.create(**HD2, flux_scheme="hllc", limiter="vanleer")
+    assert fake.grid(h, [16 * tiles, 16]) == 0
+    fake.clear()
+    assert fake.L.amrvac_gpu_step(h) == 0
+    ran = {int(l.split()[3]) for l in fake.log()[1:] if l.startswith("launch")}
+    v = [ctypes.c_int() for _ in range(5)]
+    assert fake.L.amrvac_gpu_stage_variant(h, *[ctypes.byref(x) for x in v]) == 0
+    assert ran == {v[2].value}
+    assert v[3].value == (1 if tiles <= 148 else 2 if tiles <= 296 else 4)
+    assert fake.L.amrvac_gpu_destroy(h) == 0

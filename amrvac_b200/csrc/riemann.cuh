@@ -533,7 +533,7 @@ __device__ __forceinline__ void riemann_hlld(const T *wLC, const T *wRC, const T
 // (1e-4 of the state on coarse grids).  Results there are compared with
 // earlier ones more closely than that.
 template <class T, int NDIM, int LIM>
-constexpr bool hlld_from_primitives = sizeof(T) == 8 ? NDIM == 3 : (LIM == LIM_VANLEER || LIM == LIM_MINMOD);
+constexpr bool hlld_from_primitives = sizeof(T) == 8 ? NDIM == 3 : LIM == LIM_VANLEER;
 
 // The same solver from the primitive face states alone (rotated, after
 // mhd_modify_wLR, so with GLM both sides hold the same normal field, which is

@@ -89,3 +89,67 @@ def test_negative_pressure_is_not_passed_over(oracle_lib, physics, ndim, fs, lim
     bad = _bad_oracle(oracle_lib, physics, ndim, -5.0, **kw)
     assert bad.any()
     assert np.array_equal(_bad(physics, ndim, -5.0, **kw), bad)
+
+
+def _block_hd2(value=None):
+    """A 64^2 state, the energy of cell (20, 20) set to value."""
+    prim = np.array(P.random_smooth("hd", 2, 2, 64))
+    cons = P.prim_to_cons(prim, "hd", 2, 1.4)
+    if value is not None:
+        cons[3, 0, 20, 20] = value
+    return cons
+
+
+@pytest.mark.parametrize("value", [np.inf, np.nan, 0.0, 1e-310])
+@pytest.mark.parametrize("fs,limiter", [("hll", "minmod"), ("hllc", "vanleer")])
+def test_adjoint_beside_a_special_operand(fs, limiter, value):
+    """One adjoint step: cells that the state's special cell (infinite, NaN, no
+    energy, subnormal) does not reach get the gradient they get without it, bit
+    for bit; a value that is not a number is not passed over."""
+    _cuda()
+    import torch
+    from amrvac_b200.adjoint import blocks_to_domain, domain_to_blocks, solve
+    lam = torch.from_numpy(np.random.default_rng(3).standard_normal((4, 64, 64))).cuda()
+    grad = []
+    for v in (None, value):
+        u = domain_to_blocks(torch.from_numpy(_block_hd2(v)[:, 0]).cuda()).requires_grad_(True)
+        g = torch.tensor(1.4, dtype=torch.float64, device="cuda", requires_grad=True)
+        un = solve(u, g, np.array([1e-3]), (64, 64), (0.0, 0.0), (1.0, 1.0), limiter=limiter, flux_scheme=fs)
+        d = blocks_to_domain(un, 64, 64)
+        w = lam.clone()
+        w[:, 12:29, 12:29] = 0.0  # the loss does not see what the cell reaches forward
+        d = torch.where(w == 0.0, torch.zeros_like(d), d)
+        (d * w).sum().backward()
+        grad.append(blocks_to_domain(u.grad, 64, 64).cpu().numpy())
+    far = np.ones((64, 64), bool)
+    far[4:37, 4:37] = False  # six cells a step forward, as many back
+    assert np.array_equal(grad[0][:, far], grad[1][:, far])
+    assert np.isfinite(grad[0]).all()
+
+
+@pytest.mark.parametrize("value", [np.nan, 0.0, 1e-310])
+def test_ensemble_beside_a_special_operand(value):
+    """FP64 ensembles repeat a face that met a special operand with the guarded
+    forms, as the single-grid kernel does: the same bits, and the instances
+    beside it do not notice."""
+    _cuda()
+    from amrvac_b200 import Context, Ensemble, Instance, make_cfg
+    kw = dict(physics="hd", ndim=2, gamma=1.4, typeboundary=["cont"] * 4, typeboundspeed="cmaxleftright")
+    states = [P.to_blocks(_block_hd2(v), 2) for v in (None, value, None)]
+    inst = [Instance(2, (64, 64), flux_scheme="hllc", limiter="vanleer", time_max=1.0) for _ in states]
+    ens = Ensemble(make_cfg(**kw), inst)
+    for i, w in enumerate(states):
+        ens.upload(i, w)
+    ens.step()
+    out = [P.interior(ens.download(i), 2) for i in range(3)]
+    ens.close()
+    assert np.isfinite(out[0]).all() and np.array_equal(out[0], out[2])
+    with Context(make_cfg(flux_scheme="hllc", limiter="vanleer", **kw)) as c:
+        c.set_uniform_grid([64, 64], [0.0] * 2, [1.0] * 2)
+        c.upload(states[1])
+        c.set_time(0.0, 1.0, 0.0)
+        c.step()
+        ref = P.interior(c.download(), 2)
+    assert np.array_equal(np.isfinite(out[1]), np.isfinite(ref))
+    m = np.isfinite(ref)
+    assert np.abs(out[1][m] - ref[m]).max() <= 1e-12 * np.abs(ref[m]).max()

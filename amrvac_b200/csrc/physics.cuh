@@ -133,12 +133,15 @@ __device__ __forceinline__ double div_nr(double x, double y) { return x / y; }
 // (Markstein, ch. 8; Goldschmidt's form) from the hardware's approximate
 // reciprocal square root (PTX rsqrt.approx.ftz.f64): one coupled step takes
 // the seed's ~2^-20 to ~2^-40, the residual correction s + (x - s^2) h to the
-// order of 2^-80 before the final rounding.  The seed is capped at 2^511 so
-// that x = 0 gives 0 (the seed of 0 is infinite); a negative x gives NaN.
+// order of 2^-80 before the final rounding.  An infinite seed (x = 0) becomes
+// 2^511, so that x = 0 gives 0; a negative x gives NaN.
 __device__ __forceinline__ double sqrt_nr(double x) {
   double y;
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  y = y > 0x1.0p511 ? 0x1.0p511 : y;  // (fmin would cap a NaN, too)
+  // (by the high word, on the integer pipe: 2^511 is the largest finite seed, and
+  // fmin would cap a NaN, too)
+  const int hi = __double2hiint(y);
+  y = __hiloint2double(hi == 0x7ff00000 ? 0x5fe00000 : hi, __double2loint(y));
   double s = x * y, h = 0.5 * y;
   const double r = fma(-s, h, 0.5);
   s = fma(s, r, s);

@@ -692,7 +692,7 @@ __device__ __forceinline__ uint32_t hancock_dir(const double *smem, const int *b
 // capped for, and the staging mode (asynchronous bulk copies of the next
 // conserved plane, FP64 only).  stage_variant(VAR, fp64) gives them.
 // VAR_DENSE: the FP64 2-D hydrodynamics kernel at twice the CTAs per SM.
-// VAR_WIDE: the same with a thread per face (544).
+// VAR_WIDE: the same with a thread per face (544, in 18 warps).
 constexpr int VAR_DENSE = 8, VAR_WIDE = 9;
 __host__ __device__ constexpr bool tuned_var(int var) { return var > 0 && var < VAR_DENSE; }
 struct StageVariant {
@@ -708,9 +708,12 @@ __host__ __device__ constexpr StageVariant stage_variant(int var, bool fp64) {
 }
 // CTAs per SM of 256 threads: two in FP64 MHD (104.8 KB of shared memory in
 // 3-D, and registers), three in mixed MHD; 3-D hydrodynamics has room for
-// three (58 KB; 80 registers, a few spilled: 96x80x112 HLLC FP64 0.155 ->
-// 0.143 ms per stage), mixed 2-D hydrodynamics for four (64 registers, 2048^2
-// 0.255 -> 0.228).  2.5-D MHD at three spills too much (432x304 0.033 -> 0.053).
+// three (58 KB; 80 registers, 100 to 340 bytes spilled: 96x80x112 HLLC FP64
+// 0.155 -> 0.143 ms per stage; 128^3, us a step: Roe 1288 -> 977, TVDLF 753 ->
+// 664, HLL + WENO3 1917 -> 1652, HLL + Venkatakrishnan 2786 -> 2422; only blocks
+// of 10 are faster with two, 100^3 HLLC 532 -> 473), mixed 2-D hydrodynamics for
+// four (64 registers, 2048^2 0.255 -> 0.228).  2.5-D MHD at three spills too much
+// (432x304 0.033 -> 0.053).
 __host__ __device__ constexpr int stage_base(bool fp64, bool mhd, int ndim, int hw) {
   if (hw == 3) return 1;
   if (mhd) return fp64 ? AMRVAC_STAGE_MINB : AMRVAC_STAGE_MINB_MIXED;

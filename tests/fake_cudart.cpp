@@ -117,7 +117,6 @@ void fake_clear_log() { logbuf.clear(); }
 size_t fake_used() { return used; }
 void fake_capacity(size_t n) { capacity = n; }
 void fake_sms(int n) { nsm = n; }
-int fake_last() { return (int)last; }
 // what a device held goes with its context
 void fake_device_reset() {
   std::lock_guard<std::mutex> g(mtx);
